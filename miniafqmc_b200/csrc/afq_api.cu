@@ -16,6 +16,7 @@
 #include "afq_cv.h"
 #include "afq_kernels.h"
 #include "afq_mixed.h"
+#include "afq_oz.h"
 #include "zgemm_fp64.cuh"
 
 using afq::launch_csr_gather;
@@ -84,6 +85,7 @@ struct afq_handle {
   int* comb_idx = nullptr;
 
   afq::MixedState* mixed = nullptr;
+  afq::OzState* oz = nullptr;   // FP64 form: products on the int8 tensor cores
   afq::CvState* cv = nullptr;
   afq::CvConfig cv_cfg;
 
@@ -417,6 +419,14 @@ cudaError_t body_ortho(afq_handle* h) {
   return afq::launch_ortho(h->W, h->N, h->n, h->nw, h->st);
 }
 
+// FP64 exchange partial sums of m walkers: int8 tensor cores where set up, else the FP64
+// pipe (h->nblk follows the choice).
+cudaError_t fp64_exchange(afq_handle* h, const z_t* G, int m, z_t* Kpart) {
+  if (afq::oz_has_exchange(h->oz, m)) return afq::oz_exchange(h->oz, G, m, Kpart, h->nblk, h->st);
+  int nb = 0;
+  return afq::launch_exchange(h->Lh, G, h->N, h->n, h->nc, m, Kpart, &nb, h->st);
+}
+
 cudaError_t body_energy(afq_handle* h, int mode) {
   cudaError_t e;
   const int nak = (int)h->NAK;
@@ -446,10 +456,7 @@ cudaError_t body_energy(afq_handle* h, int mode) {
       if ((e = zgemm_launch<true, true>(g, 1, ep, h->st, h->f64cfg[afq_handle::F64_COUL])) !=
           cudaSuccess)
         return e;
-      int nb = 0;
-      if ((e = afq::launch_exchange(h->Lh, h->Gc, h->N, h->n, h->nc, h->nw, h->Kpart, &nb,
-                                    h->st)) != cudaSuccess)
-        return e;
+      if ((e = fp64_exchange(h, h->Gc, h->nw, h->Kpart)) != cudaSuccess) return e;
     }
     if ((e = afq::launch_energy_reduce(h->Gc, h->haj, nak, nullptr, h->cvec, h->nc, h->Kpart,
                                        h->nblk, h->nw, 1, h->Wd, h->parts, h->st)) != cudaSuccess)
@@ -488,7 +495,8 @@ cudaError_t st_ortho(afq_handle* h) {
 }
 cudaError_t st_energy(afq_handle* h, int mode) {
   int nl = mode == AFQ_ENERGY_VAKBL ? 3
-           : (h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_ENERGY) + 2 : 5);
+           : h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_ENERGY) + 2
+           : afq::oz_has_exchange(h->oz, h->nw) ? 4 + afq::oz_exchange_launches(h->oz, h->nw) : 5;
   return staged(h, AFQ_STAGE_ENERGY, nl, [&] { return body_energy(h, mode); });
 }
 
@@ -886,6 +894,7 @@ void afq_destroy(afq_handle* h) {
     cudaEventDestroy(r.b);
   }
   if (h->mixed) afq::mixed_destroy(h->mixed);
+  if (h->oz) afq::oz_destroy(h->oz);
   if (h->cv) afq::cv_destroy(h->cv);
   if (h->st) cudaStreamSynchronize(h->st);
   for (void* p : h->allocs)
@@ -998,7 +1007,15 @@ afq_status afq_set_hamiltonian(afq_handle* h, const afq_csr_z* Spvn, const afq_c
       h->nblk = nb;
     }
   }
-  if (!h->mixed) AFQ_CUDA(h, fp64_tune(h));
+  if (!h->mixed) {
+    afq::OzInit oi{N, n, nc, h->nw, h->Lh};
+    AFQ_CUDA(h, afq::oz_create(oi, &h->oz, h->st));
+    if (afq::oz_has_exchange(h->oz, h->nw)) {   // one partial sum per Cholesky vector
+      if (nc > h->nblk) AFQ_CUDA(h, dalloc(h, &h->Kpart, (size_t)h->nw * 2 * nc));
+      h->nblk = nc;
+    }
+    AFQ_CUDA(h, fp64_tune(h));
+  }
   AFQ_CUDA(h, cudaStreamSynchronize(h->st));
   h->have_ham = true;
   return AFQ_OK;
@@ -1308,8 +1325,7 @@ afq_status energy_cv(afq_handle* h, double* sums) {
   in.N = h->N;
   in.exact_exchange = [h](const z_t* gsub, int m, z_t* kp) -> cudaError_t {
     if (h->mixed) return afq::mixed_exchange(h->mixed, gsub, m, kp, h->nblk, h->st);
-    int nb = 0;
-    return afq::launch_exchange(h->Lh, gsub, h->N, h->n, h->nc, m, kp, &nb, h->st);
+    return fp64_exchange(h, gsub, m, kp);
   };
   if (h->mixed && h->cv_cfg.base)
     in.base_exchange = [h](const z_t* g, int m, z_t* kp) -> cudaError_t {
@@ -1821,9 +1837,9 @@ afq_status afq_synchronize(afq_handle* h) {
   if (!h) return AFQ_ERR_ARG;
   AFQ_CUDA(h, cudaStreamSynchronize(h->st));
   if (h->cv) AFQ_CUDA(h, afq::cv_sync(h->cv));   // the estimator's online training
-  if (h->mixed) {
+  if (h->mixed || h->oz) {
     int flags = 0;
-    AFQ_CUDA(h, afq::mixed_error(h->mixed, &flags));
+    AFQ_CUDA(h, h->mixed ? afq::mixed_error(h->mixed, &flags) : afq::oz_error(h->oz, &flags));
     if (flags) return fail(h, AFQ_ERR_CUDA, "tensor-core pipeline wait timed out (flags " +
                                                 std::to_string(flags) + ")");
   }

@@ -1,0 +1,362 @@
+// FP64 products on the int8 tensor cores (tcgen05 kind::i8) by error-free splitting.
+//
+// Every FP64 operand row is scaled by a power of two and written as kOzS signed 8-bit digits
+// (Ootomo, Ozaki and Yokota, "DGEMM on integer matrix multiplication unit", 2024; Ozaki et
+// al., "Error-free transformations of matrix multiplication", 2012):
+//   x = 2^e sum_{i=1..S} d_i 2^-(8i - 1),   d_i in [-128, 127]
+// (55 bits below the row's power of two for S = 7).  The products d_i d_j with i + j = D
+// share one weight, so D' = S accumulators per output hold all pairs with i + j <= S + 1,
+//   acc_D = sum_{i + j = D} sum_k a_i[m][k] b_j[n][k]      (exact in int32),
+// and the FP64 result is sum_D acc_D 2^(2 - 8D), times the two row scales.  The dropped
+// pairs lie below 2^-57 of (row maximum) x (column maximum).
+//
+// Layout and tile.  TMEM holds 512 columns of 32-bit accumulators, so S = 7 accumulators
+// allow a 128 x 64 output tile (448 columns).  The seven B slices of a tile sit one after
+// the other in shared memory (64 rows each), so the products of A slice i with B slices
+// 1 .. S + 1 - i are ONE matrix product of N = 64 (S + 1 - i) columns whose accumulators
+// are consecutive in TMEM, starting at accumulator i: ten tcgen05.mma per 32 bytes of K
+// instead of 28, and each A slice is read from shared memory once or twice.
+// What bounds it: operand supply.  A K slab of 64 bytes costs 7 x (128 + 64) x 64 = 86 KB
+// for 1792 tensor-pipe clocks (48 bytes per clock and SM from L2).
+//
+// One persistent CTA per SM: warp 8 copies slabs (bulk copies) into a two-stage ring, one thread of
+// warp 9 issues the MMAs, and warps 0-7 turn the accumulators into FP64 results in
+// registers (releasing TMEM to the next tile) and then run the epilogue functor while that
+// tile's MMAs proceed.  Waits are bounded as in tc_gemm.cuh.
+#pragma once
+#include "tc_gemm.cuh"
+
+namespace oz {
+
+constexpr int kS = 7;                 // 8-bit digits per operand
+constexpr int kBM = 128, kBN = 64;    // output tile
+constexpr int kSlab = 64;             // bytes (= digits) of K per ring stage
+constexpr int kStages = 2;
+constexpr uint32_t kABytes = kS * kBM * kSlab, kBBytes = kS * kBN * kSlab;
+constexpr uint32_t kStageBytes = kABytes + kBBytes;
+constexpr int kEpi = 256, kThreads = kEpi + 64;
+constexpr size_t kSmem = 1024 + kStages * kStageBytes + 8 * (2 * kStages + 3) + 16;
+// int32 accumulators: at most S pairs of digits of magnitude 128 per K entry
+constexpr int kMaxK = 16384;
+static_assert((long long)kS * 128 * 128 * kMaxK < (1LL << 31), "int32 accumulation");
+// acc_5 2^24 + acc_6 2^16 + acc_7 2^8 + acc_8 (4, 5, 6 and 7 pairs) below 2^51 for K <= 1024
+static_assert((4LL * (1 << 24) + 5 * (1 << 16) + 6 * (1 << 8) + 7) * 128 * 128 * 1024 < (1LL << 51),
+              "one integer for the four low accumulators");
+static_assert(kS * kBN <= 512 && kSmem <= 227 * 1024, "TMEM / shared memory");
+
+// Digit slices of a batch of rows, stored as the shared-memory images the MMAs read: for
+// each batch, tile of R rows (R = 128 for an A operand, 64 for a B operand) and K slab, the
+// kS slices' R x 64-byte blocks one after the other, 16-byte pieces swizzled as SWIZZLE_64B
+// (piece index ^ (row / 2) mod 4).  A ring stage of an operand is then one contiguous bulk
+// copy.  K is zero padded to whole slabs; rows past the last one hold any digits (their
+// products are never stored).  scale [batch][rows] = 2^e of each row (0 for a zero row, NaN
+// for a row with a non-finite entry, which makes every output of the row NaN).
+struct Slices {
+  int8_t* d = nullptr;
+  double* scale = nullptr;
+  int rows = 0, batch = 0, tile = 0, nslab = 0;
+  // source rows per batch, each giving one or two operand rows
+  AFQ_HD int per_batch(bool two) const { return two ? rows / 2 : rows; }
+  AFQ_HD int tiles() const { return (rows + tile - 1) / tile; }
+  AFQ_HD long long stage() const { return (long long)kS * tile * kSlab; }
+  size_t bytes() const { return (size_t)batch * tiles() * nslab * stage(); }
+};
+// Offset of digit (row r of the batch, K entry k, slice 0); the slices are tile x kSlab
+// bytes apart.
+AFQ_HD long long slice_offset(const Slices& s, int batch, int r, int k) {
+  const int rt = r / s.tile, rr = r - rt * s.tile, ks = k / kSlab, kb = k % kSlab;
+  return (((long long)batch * s.tiles() + rt) * s.nslab + ks) * s.stage() + rr * kSlab +
+         (((kb >> 4) ^ (rr >> 1)) & 3) * 16 + (kb & 15);
+}
+
+struct Job {
+  const int8_t *a, *b;
+  const double *sa, *sb;            // row scales [batch][rows]
+  int a_rows, b_rows, a_tiles, b_tiles;   // rows and row tiles per batch (0: not batched)
+  tc::TileSched sched;
+  int M, N;                         // output rows and columns per batch
+  int m_tile, n_tile;               // first row tile of A and of B of the launch
+  int nslab, slab_split;            // K slabs, and slabs per z when split along K (else 0)
+};
+
+AFQ_D void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
+          "r"(tc::smem_u32(dst)),
+      "l"(src), "r"(bytes), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+AFQ_D void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc));
+}
+// int32 accumulator, signed 8-bit A and B, both K-major
+constexpr uint32_t idesc_i8(int M, int N) {
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
+         ((uint32_t)(M >> 4) << 24);
+}
+// 8 consecutive TMEM columns of this thread's lane (no wait)
+AFQ_D void tmem_ld8(uint32_t taddr, int* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                 "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+// 32-byte store (32-byte aligned)
+AFQ_D void store4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d)
+               : "memory");
+}
+AFQ_D void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// sum_D acc_D 2^(2 - 8D), D = 2 .. 8, times 2^30: integer sums of consecutive accumulators,
+// exact below 2^51, formed on top of the bits of 1.5 x 2^52 by 32 x 32 + 64-bit multiply-adds
+// (subtracting that constant converts them without a conversion instruction).  SHORT (K of
+// at most 1024): the four low accumulators fit one sum; otherwise the last stays apart.
+// The drain is issue bound: 7 integer and 3 to 5 FP64 instructions per output.
+constexpr long long kMagicBits = 0x4338000000000000LL;   // 1.5 x 2^52
+constexpr int kShortSlabs = 1024 / kSlab;
+AFQ_D long long mad_wide(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+template <bool SHORT>
+AFQ_D double combine(const int (&a)[kS]) {
+  constexpr double kMagic = 6755399441055744.0;
+  const double hi = __longlong_as_double(mad_wide(
+                        a[2], 1, mad_wide(a[1], 1 << 8, mad_wide(a[0], 1 << 16, kMagicBits)))) -
+                    kMagic;
+  if constexpr (SHORT) {
+    const double lo = __longlong_as_double(mad_wide(
+                          a[6], 1, mad_wide(a[5], 1 << 8, mad_wide(a[4], 1 << 16,
+                                   mad_wide(a[3], 1 << 24, kMagicBits))))) -
+                      kMagic;
+    return fma(lo, 0x1p-32, hi);
+  }
+  const double mid = __longlong_as_double(mad_wide(
+                         a[5], 1, mad_wide(a[4], 1 << 8, mad_wide(a[3], 1 << 16, kMagicBits)))) -
+                     kMagic;
+  const double lo = __longlong_as_double(mad_wide(a[6], 1, kMagicBits)) - kMagic;
+  return fma(fma(lo, 0x1p-8, mid), 0x1p-24, hi);
+}
+
+// The 32 columns of this thread's lane at trow (accumulators kBN columns apart).
+template <bool SHORT>
+AFQ_D void drain(uint32_t trow, double (&v)[32]) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 8) {
+    int r[kS][8];
+#pragma unroll
+    for (int d = 0; d < kS; d++) tmem_ld8(trow + d * kBN + c, r[d]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      int a[kS];
+#pragma unroll
+      for (int d = 0; d < kS; d++) a[d] = r[d][q];
+      v[c + q] = combine<SHORT>(a);
+    }
+  }
+}
+
+// Epilogue functor: epi(z, m, n, v) with v[32] the results of row m, columns n .. n + 31 of
+// the launch (rows >= M and columns >= N included: the functor checks).
+template <class Epi>
+__global__ void __launch_bounds__(kThreads, 1)
+oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi, int* err) {
+  extern __shared__ __align__(1024) uint8_t oz_smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(oz_smem_raw) + 1023) & ~uintptr_t(1023));
+  auto stA = [&](int s) { return smem + s * kStageBytes; };
+  auto stB = [&](int s) { return smem + s * kStageBytes + kABytes; };
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
+  uint64_t* empty = full + kStages;
+  uint64_t* accf = empty + kStages;
+  uint64_t* acce = accf + 1;
+  uint64_t* fin = acce + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int WPROD = kEpi / 32, WMMA = WPROD + 1;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; s++) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    tc::mbar_init(accf, 1);
+    tc::mbar_init(acce, kEpi);
+    tc::mbar_init(fin, 1);
+    tc::fence_barrier_init();
+  }
+  if (warp == 0) {
+    tc::tmem_alloc(tmem_slot, 512);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int total = job.sched.total();
+  auto slabs = [&](int z, int& s0) {
+    s0 = job.slab_split ? z * job.slab_split : 0;
+    return job.slab_split ? min(job.slab_split, job.nslab - s0) : job.nslab;
+  };
+
+  if (warp == WPROD && lane == 0) {
+    // ---- producer: one bulk copy per operand and stage (all slices)
+    int g = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+      int z, mt, nt, s0;
+      job.sched.decode(t, z, mt, nt);
+      const int ns = slabs(z, s0);
+      const int8_t* pa =
+          job.a + ((long long)(z * job.a_tiles + job.m_tile + mt) * job.nslab + s0) * kABytes;
+      const int8_t* pb =
+          job.b + ((long long)(z * job.b_tiles + job.n_tile + nt) * job.nslab + s0) * kBBytes;
+      for (int k = 0; k < ns; k++, g++) {
+        const int s = g % kStages;
+        if (!tc::mbar_wait(&empty[s], ((g / kStages) & 1) ^ 1)) {
+          atomicOr(err, tc::ERR_TIMEOUT_PRODUCER);
+          ok = false;
+          break;
+        }
+        tc::mbar_expect_tx(&full[s], kStageBytes);
+        bulk_load(stA(s), pa + (long long)k * kABytes, kABytes, &full[s]);
+        bulk_load(stB(s), pb + (long long)k * kBBytes, kBBytes, &full[s]);
+      }
+    }
+    for (int q = max(0, g - kStages); q < g; q++)
+      tc::mbar_wait_drain(&full[q % kStages], (q / kStages) & 1);
+  } else if (warp == WMMA && lane == 0) {
+    // ---- MMA issuer
+    int g = 0, li = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total && ok; t += gridDim.x, li++) {
+      int z, mt, nt, s0;
+      job.sched.decode(t, z, mt, nt);
+      const int ns = slabs(z, s0);
+      if (!tc::mbar_wait(acce, (li & 1) ^ 1)) {
+        atomicOr(err, tc::ERR_TIMEOUT_MMA);
+        break;
+      }
+      tc::tc_fence_after();
+      for (int k = 0; k < ns; k++, g++) {
+        const int s = g % kStages;
+        if (!tc::mbar_wait(&full[s], (g / kStages) & 1)) {
+          atomicOr(err, tc::ERR_TIMEOUT_MMA);
+          ok = false;
+          break;
+        }
+        tc::tc_fence_after();
+        const uint64_t ad = tc::sdesc_k<kSlab>(tc::smem_u32(stA(s)));
+        const uint64_t bd = tc::sdesc_k<kSlab>(tc::smem_u32(stB(s)));
+#pragma unroll
+        for (int u = 0; u < kSlab / 32; u++) {
+#pragma unroll
+          for (int i = 0; i < kS; i++) {   // A slice i times B slices 0 .. S - 1 - i
+            const uint64_t ai = ad + (uint64_t)((i * kBM * kSlab) >> 4) + 2 * u;
+            const uint32_t first = (k | u | i) != 0;
+#pragma unroll
+            for (int j = 0; j < kS - i; j += 4) {
+              const int nc = (kS - i - j < 4 ? kS - i - j : 4) * kBN;
+              umma_i8(tmem + (i + j) * kBN, ai, bd + (uint64_t)((j * kBN * kSlab) >> 4) + 2 * u,
+                      idesc_i8(kBM, nc), first);
+            }
+          }
+        }
+        tc::umma_commit(&empty[s]);
+      }
+      if (!ok) break;
+      tc::umma_commit(accf);
+    }
+    tc::umma_commit(fin);
+    tc::mbar_wait_drain(fin, 0);
+  }
+  if (warp < WPROD) {
+    // ---- accumulators -> FP64 -> functor: warpgroup wg takes 32 of the 64 columns
+    const int wg = warp >> 2, wq = warp & 3;
+    const int row = wq * 32 + lane;
+    const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16) + wg * 32;
+    int li = 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, li++) {
+      int z, mt, nt;
+      job.sched.decode(t, z, mt, nt);
+      const int m = mt * kBM + row, n0 = nt * kBN + wg * 32;
+      const long long ra = (long long)z * job.a_rows + job.m_tile * kBM;
+      const long long rb = (long long)z * job.b_rows + job.n_tile * kBN;
+      const double sa = m < job.M ? job.sa[ra + m] : 0.0;
+      const double sb = n0 + lane < job.N ? job.sb[rb + n0 + lane] : 0.0;   // lane's column
+      // the warp goes on as one (the TMEM loads and shuffles below are warp-wide)
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(accf, li & 1))) {
+        if (lane == 0) atomicOr(err, tc::ERR_TIMEOUT_EPILOGUE);
+        break;
+      }
+      tc::tc_fence_after();
+      double v[32];
+      if (job.slab_split ? job.slab_split <= kShortSlabs : job.nslab <= kShortSlabs)
+        drain<true>(trow, v);
+      else
+        drain<false>(trow, v);
+      tc::tc_fence_before();
+      tc::mbar_arrive(acce);
+      const double sa30 = sa * 0x1p-30;
+#pragma unroll
+      for (int c = 0; c < 32; c++) v[c] *= sa30 * __shfl_sync(0xffffffffu, sb, c);
+      epi(z, m, n0, v);
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, 512);
+}
+
+// ------------------------------------------------------------------ host side
+// C[z][m][n] = sum_k A[z][m0 + m][k] B[z][n0 + n][k], m < M, n < N, with m0 = 128 m_tile and
+// n0 = 64 n_tile.  An operand of batch 1 is shared by all batches.  slab_split > 0: z counts
+// K ranges of slab_split slabs of an unbatched product instead of batches.
+struct Gemm {
+  const Slices *a, *b;
+  int M, N, nbatch;
+  int m_tile = 0, n_tile = 0;
+  int slab_split = 0;
+  bool m_fast = true;
+};
+
+template <class Epi>
+cudaError_t launch(const Gemm& g, const Epi& epi, int* err, cudaStream_t st) {
+  if (g.M <= 0 || g.N <= 0 || g.nbatch <= 0) return cudaSuccess;
+  if (g.a->tile != kBM || g.b->tile != kBN || g.a->nslab != g.b->nslab) return cudaErrorInvalidValue;
+  auto kern = oz_gemm_kernel<Epi>;
+  static DeviceAttr attr;
+  cudaError_t e = attr.ensure(kSmem, [kern](size_t b) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+  });
+  if (e != cudaSuccess) return e;
+  Job j;
+  j.a = g.a->d;
+  j.b = g.b->d;
+  j.sa = g.a->scale;
+  j.sb = g.b->scale;
+  const bool ab = !g.slab_split && g.a->batch > 1, bb = !g.slab_split && g.b->batch > 1;
+  j.a_rows = ab ? g.a->rows : 0;
+  j.b_rows = bb ? g.b->rows : 0;
+  j.a_tiles = ab ? g.a->tiles() : 0;
+  j.b_tiles = bb ? g.b->tiles() : 0;
+  j.sched = tc::TileSched{(g.M + kBM - 1) / kBM, (g.N + kBN - 1) / kBN, g.nbatch,
+                          g.m_fast ? 1 : 0, 0};
+  j.M = g.M;
+  j.N = g.N;
+  j.m_tile = g.m_tile;
+  j.n_tile = g.n_tile;
+  j.nslab = g.a->nslab;
+  j.slab_split = g.slab_split;
+  const int total = j.sched.total();
+  const int grid = total < tc::sm_count() ? total : tc::sm_count();
+  kern<<<grid, kThreads, kSmem, st>>>(j, epi, err);
+  return cudaGetLastError();
+}
+
+}  // namespace oz

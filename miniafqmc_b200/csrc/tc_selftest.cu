@@ -6,6 +6,7 @@
 
 #include "../../include/afqmc_b200.h"
 #include "afq_mixed.h"
+#include "afq_oz.h"
 #include "tc_gemm.cuh"
 
 namespace {
@@ -155,6 +156,7 @@ extern "C" afq_status afq_set_tc_wait_limit(int device, long long clocks) {
   // every module holding tensor-core kernels keeps its own copy of the bound
   cudaError_t e = tc::set_wait_clocks(clocks);
   if (e == cudaSuccess) e = afq::mixed_set_wait_clocks(clocks);
+  if (e == cudaSuccess) e = afq::oz_set_wait_clocks(clocks);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   cudaSetDevice(prev);
   return e == cudaSuccess ? AFQ_OK : AFQ_ERR_CUDA;
