@@ -340,6 +340,8 @@ cudaError_t body_dm(afq_handle* h, int want_gc, int save_old) {
 
 cudaError_t body_vbias(afq_handle* h) {
   if (h->mixed) return afq::mixed_vbias(h->mixed, h->Gc, h->vbias, h->st);
+  if (afq::oz_has_gsite(h->oz, afq::OZ_VBIAS))
+    return afq::oz_gsite(h->oz, afq::OZ_VBIAS, h->Gc, h->vbias, h->st);
   if (h->spT_dense) {
     ZGemmDesc g{h->nc, h->nw, (int)h->NAK, h->spT_dense, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
     EpiStore e{h->vbias, h->nw, 0, zmk(0, 0), 0};
@@ -370,6 +372,7 @@ cudaError_t dense_vhs(afq_handle* h, int cfg) {
 
 cudaError_t body_vhs(afq_handle* h) {
   if (h->mixed) return afq::mixed_vhs(h->mixed, h->X, h->vHS, h->st);
+  if (afq::oz_has_vhs(h->oz)) return afq::oz_vhs(h->oz, h->X, h->vHS, h->st);
   if (h->sp_dense || h->sp_dense_r) return dense_vhs(h, h->vhsd_cfg);
   return afq::launch_csr_walker(h->sp_ri, h->sp_ci, h->sp_v, h->sp_rv, h->X, h->N * h->N, h->nw,
                                 h->vHS, (long long)h->N * h->N, h->st,
@@ -379,6 +382,8 @@ cudaError_t body_vhs(afq_handle* h) {
 cudaError_t body_propagate(afq_handle* h) {
   h->dm_cache = false;
   if (h->mixed) return afq::mixed_propagate(h->mixed, h->W, h->vHS, h->st);
+  if (afq::oz_has_propagate(h->oz))
+    return afq::oz_propagate(h->oz, h->W, h->vHS, h->S, h->T1, h->st);
   const int N = h->N, n2 = 2 * h->n, nw = h->nw;
   const long long sWN = (long long)N * n2, sV = (long long)N * N;
   const int zc = h->f64cfg[afq_handle::F64_PROP];
@@ -419,6 +424,15 @@ cudaError_t body_ortho(afq_handle* h) {
   return afq::launch_ortho(h->W, h->N, h->n, h->nw, h->st);
 }
 
+// The Coulomb vector of every walker, cvec [nchol][nw] (FP64 form).
+cudaError_t fp64_coulomb(afq_handle* h, int cfg) {
+  if (afq::oz_has_gsite(h->oz, afq::OZ_COULOMB))
+    return afq::oz_gsite(h->oz, afq::OZ_COULOMB, h->Gc, h->cvec, h->st);
+  ZGemmDesc g{h->nc, h->nw, (int)h->NAK, h->Lh, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
+  EpiStore ep{h->cvec, h->nw, 0, zmk(0, 0), 0};
+  return zgemm_launch<true, true>(g, 1, ep, h->st, cfg);
+}
+
 // FP64 exchange partial sums of m walkers: int8 tensor cores where set up, else the FP64
 // pipe (h->nblk follows the choice).
 cudaError_t fp64_exchange(afq_handle* h, const z_t* G, int m, z_t* Kpart) {
@@ -431,7 +445,10 @@ cudaError_t body_energy(afq_handle* h, int mode) {
   cudaError_t e;
   const int nak = (int)h->NAK;
   if (mode == AFQ_ENERGY_VAKBL) {
-    if (h->vk_dense) {
+    if (afq::oz_has_gsite(h->oz, afq::OZ_VAKBL)) {
+      if ((e = afq::oz_gsite(h->oz, afq::OZ_VAKBL, h->Gc, h->Gcloc, h->st)) != cudaSuccess)
+        return e;
+    } else if (h->vk_dense) {
       ZGemmDesc g{nak, h->nw, nak, h->vk_dense, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
       EpiStore ep{h->Gcloc, h->nw, 0, zmk(0, 0), 0};
       if ((e = zgemm_launch<true, true>(g, 1, ep, h->st, h->f64cfg[afq_handle::F64_VAKBL])) !=
@@ -451,11 +468,7 @@ cudaError_t body_energy(afq_handle* h, int mode) {
           cudaSuccess)
         return e;
     } else {
-      ZGemmDesc g{h->nc, h->nw, nak, h->Lh, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
-      EpiStore ep{h->cvec, h->nw, 0, zmk(0, 0), 0};
-      if ((e = zgemm_launch<true, true>(g, 1, ep, h->st, h->f64cfg[afq_handle::F64_COUL])) !=
-          cudaSuccess)
-        return e;
+      if ((e = fp64_coulomb(h, h->f64cfg[afq_handle::F64_COUL])) != cudaSuccess) return e;
       if ((e = fp64_exchange(h, h->Gc, h->nw, h->Kpart)) != cudaSuccess) return e;
     }
     if ((e = afq::launch_energy_reduce(h->Gc, h->haj, nak, nullptr, h->cvec, h->nc, h->Kpart,
@@ -472,18 +485,20 @@ cudaError_t st_dm(afq_handle* h, int want_gc, int save_old) {
   return staged(h, stage, nl, [&] { return body_dm(h, want_gc, save_old); });
 }
 cudaError_t st_vbias(afq_handle* h) {
-  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VBIAS) : 1;
+  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VBIAS)
+           : afq::oz_has_gsite(h->oz, afq::OZ_VBIAS) ? afq::oz_gsite_launches(h->oz, afq::OZ_VBIAS) : 1;
   return staged(h, AFQ_STAGE_VBIAS, nl, [&] { return body_vbias(h); });
 }
 cudaError_t st_sigma(afq_handle* h, int use_xraw) {
   return staged(h, AFQ_STAGE_SIGMA, 1, [&] { return body_sigma(h, use_xraw); });
 }
 cudaError_t st_vhs(afq_handle* h) {
-  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VHS) : 1;
+  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VHS) : afq::oz_has_vhs(h->oz) ? 2 : 1;
   return staged(h, AFQ_STAGE_VHS, nl, [&] { return body_vhs(h); });
 }
 cudaError_t st_propagate(afq_handle* h) {
-  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_PROPAGATE) : h->d.taylor_order + 2;
+  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_PROPAGATE)
+           : afq::oz_has_propagate(h->oz) ? afq::oz_propagate_launches(h->oz) : h->d.taylor_order + 2;
   return staged(h, AFQ_STAGE_PROPAGATE, nl, [&] { return body_propagate(h); });
 }
 cudaError_t st_weights(afq_handle* h, int update_eshift) {
@@ -494,9 +509,11 @@ cudaError_t st_ortho(afq_handle* h) {
                 [&] { return body_ortho(h); });
 }
 cudaError_t st_energy(afq_handle* h, int mode) {
-  int nl = mode == AFQ_ENERGY_VAKBL ? 3
-           : h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_ENERGY) + 2
-           : afq::oz_has_exchange(h->oz, h->nw) ? 4 + afq::oz_exchange_launches(h->oz, h->nw) : 5;
+  const int site = mode == AFQ_ENERGY_VAKBL ? afq::OZ_VAKBL : afq::OZ_COULOMB;
+  int nl = 2 + (afq::oz_has_gsite(h->oz, site) ? afq::oz_gsite_launches(h->oz, site) : 1);
+  if (mode != AFQ_ENERGY_VAKBL)
+    nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_ENERGY) + 2
+                  : nl + (afq::oz_has_exchange(h->oz, h->nw) ? afq::oz_exchange_launches(h->oz, h->nw) : 1);
   return staged(h, AFQ_STAGE_ENERGY, nl, [&] { return body_energy(h, mode); });
 }
 
@@ -1008,7 +1025,8 @@ afq_status afq_set_hamiltonian(afq_handle* h, const afq_csr_z* Spvn, const afq_c
     }
   }
   if (!h->mixed) {
-    afq::OzInit oi{N, n, nc, h->nw, h->Lh};
+    afq::OzInit oi{N, n, nc, h->nw, h->d.taylor_order, h->Lh, h->spT_dense, h->vk_dense,
+                   h->sp_dense, h->sp_dense_r, (long long)Spvn->rowIndex[N * N], h->P};
     AFQ_CUDA(h, afq::oz_create(oi, &h->oz, h->st));
     if (afq::oz_has_exchange(h->oz, h->nw)) {   // one partial sum per Cholesky vector
       if (nc > h->nblk) AFQ_CUDA(h, dalloc(h, &h->Kpart, (size_t)h->nw * 2 * nc));
@@ -1336,10 +1354,7 @@ afq_status energy_cv(afq_handle* h, double* sums) {
     if (h->mixed) {
       r = afq::mixed_coulomb(h->mixed, h->Gc, h->cvec, h->st);
     } else {
-      const int nak = (int)h->NAK;
-      ZGemmDesc g{h->nc, h->nw, nak, h->Lh, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
-      EpiStore ep{h->cvec, h->nw, 0, zmk(0, 0), 0};
-      r = zgemm_launch<true, true>(g, 1, ep, h->st);
+      r = fp64_coulomb(h, 0);
     }
     if (r != cudaSuccess) return r;
     return afq::cv_energy(h->cv, in, sums, h->st);

@@ -9,14 +9,33 @@ namespace afq {
 struct OzState;
 
 struct OzInit {
-  int N, n, nchol, nw;
-  const z_t* Lh;   // [nchol][2][n][N] half-rotated factors (null: no exchange)
+  int N, n, nchol, nw, order;
+  const z_t* Lh;         // [nchol][2][n][N] half-rotated factors (null: no Cholesky energy)
+  const z_t* SpvnT;      // dense [nchol][2nN] (null: vbias stays on the CSR path)
+  const z_t* Vakbl;      // dense [2nN][2nN] or null
+  const z_t* Spvn;       // dense [N^2][nchol] of complex values, or null
+  const double* Spvn_r;  // dense [N^2][nchol] of real values, or null
+  long long spvn_nnz;
+  const z_t* P;          // Propg1 [N][N]
 };
 
 // Slices the static operands of the products that take this path (rules in oz.cu) and
 // allocates their workspaces; *out stays null when none does or memory is short.
 cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st);
 void oz_destroy(OzState* o);
+// Products of G [nw][2nN] with a static operand, out [rows][nw]: vbias (SpvnT), the Coulomb
+// vector (Lh), Vakbl G.
+enum OzSite { OZ_VBIAS, OZ_COULOMB, OZ_VAKBL, OZ_NG };
+bool oz_has_gsite(const OzState* o, int site);
+int oz_gsite_launches(const OzState* o, int site);
+cudaError_t oz_gsite(OzState* o, int site, const z_t* Gc, z_t* out, cudaStream_t st);
+// vHS [nw][N][N] from X [nchol][nw].
+bool oz_has_vhs(const OzState* o);
+cudaError_t oz_vhs(OzState* o, const z_t* X, z_t* vHS, cudaStream_t st);
+// W [nw][N][2n] <- P (sum_k (i vHS)^k / k!) P W; S, T scratch [nw][2n][N].
+bool oz_has_propagate(const OzState* o);
+int oz_propagate_launches(const OzState* o);
+cudaError_t oz_propagate(OzState* o, z_t* W, const z_t* vHS, z_t* S, z_t* T, cudaStream_t st);
 bool oz_has_exchange(const OzState* o, int nwalk);
 int oz_exchange_launches(const OzState* o, int nwalk);
 // Exchange partial sums of nwalk walkers, one per Cholesky vector: Kpart[nwalk][2][nblk] with

@@ -1,5 +1,6 @@
 // FP64 contraction stages on the int8 tensor cores: operand splitting, the products of
 // oz_gemm.cuh and the kernels around them.
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <vector>
 
@@ -23,6 +24,23 @@ struct OzState {
   double* T = nullptr;
   int ex_w = 0, ex_c = 0;   // walkers and Cholesky vectors per chunk
   bool exchange = false;
+  // products with G: static operand rows, G rows (w, re | im) shared by the sites, partial
+  // products of the K splits
+  struct GSite {
+    bool on = false;
+    Slices a;
+    int rows = 0, splits = 1, slab_split = 0;
+  } gs[OZ_NG];
+  bool greal = false;
+  Slices gb;
+  double* part = nullptr;
+  long long part_ld = 0;
+  // vHS: Spvn rows ik, X rows (w, re | im)
+  bool vhs = false, sreal = false;
+  Slices sp, xb;
+  // propagation: Propg1, vHS and the walker columns (j, re | im) for either
+  bool prop = false, preal = false;
+  Slices pa, va, pb, tb;
 };
 
 namespace {
@@ -60,7 +78,8 @@ struct RowSrc {
 // How complex source rows become operand rows: kReal: one row of real parts; kPairs: one
 // row of (re, im) pairs (a complex A operand); kSplitRe: rows 2r = re, 2r + 1 = im (B of a
 // real A); kSplitCx: rows 2r = (re, -im) pairs, 2r + 1 = (im, re) pairs (B of a complex A).
-enum { kReal, kPairs, kSplitRe, kSplitCx };
+// kDouble: rows of real doubles (RowSrc strides in doubles).
+enum { kReal, kPairs, kSplitRe, kSplitCx, kDouble };
 
 struct RowScale {
   double s1, s2, scale;   // q = rn(x s1 s2) = rn(x 2^(55 - e)), scale = 2^e
@@ -102,57 +121,26 @@ AFQ_D unsigned long long absbits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
 }
 
-// One warp (WIDE = false) or one CTA (WIDE) per source row: the row's maximum, then its
-// digits, four K entries per thread and step.  Memory bound: 16 bytes read per complex
-// entry and up to 14 (28 for kSplitCx) written; the second read of the row hits L1 / L2.
-template <int MODE, bool WIDE>
-__global__ void __launch_bounds__(256)
-slice_kernel(RowSrc src, int nrows, int K, Slices s) {
-  __shared__ unsigned long long red[2][8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = WIDE ? blockIdx.x : blockIdx.x * 8 + warp;
-  if (r >= nrows) return;   // whole warps (WIDE: never)
-  const int t = WIDE ? threadIdx.x : lane, nt = WIDE ? 256 : 32;
-  const z_t* p = src.row(r);
-  unsigned long long m0 = 0, m1 = 0;   // of the real and of the imaginary parts
-  for (int k = t; k < K; k += nt) {
-    const z_t v = p[k];
-    m0 = max(m0, absbits(v.x));
-    m1 = max(m1, absbits(v.y));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-  }
-  if constexpr (WIDE) {
-    if (lane == 0) {
-      red[0][warp] = m0;
-      red[1][warp] = m1;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      m0 = max(m0, red[0][i]);
-      m1 = max(m1, red[1][i]);
-    }
-  }
-  if constexpr (MODE == kPairs || MODE == kSplitCx) m0 = m1 = max(m0, m1);
-  const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
-  constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
-  const int rb = r / s.per_batch(TWO), r0 = (r - rb * s.per_batch(TWO)) * (TWO ? 2 : 1);
-  if (t == 0) {
-    double* sc = s.scale + (long long)rb * s.rows + r0;
-    sc[0] = s0.scale;
-    if constexpr (TWO) sc[1] = s1.scale;
-  }
+// Digits of a source row from entry k0 on (K entries; KD digits stored, past the row's end
+// zeros), thread t of nt, four digits per step.
+template <int MODE>
+AFQ_D void slice_row(const z_t* __restrict__ p, int K, const Slices& s, int rb, int r0,
+                     const RowScale& s0, const RowScale& s1, int kd0, int kd1, int t, int nt) {
   const z_t zero = zmk(0, 0);
+  const double* pd = reinterpret_cast<const double*>(p);
   unsigned q[kS];
-  const int Kp = s.nslab * oz::kSlab, plane = s.tile * oz::kSlab;
-  for (int k = 4 * t; k < Kp; k += 4 * nt) {
+  const int plane = s.tile * oz::kSlab;
+  for (int k = kd0 + 4 * t; k < kd1; k += 4 * nt) {
     int8_t* o = s.d + oz::slice_offset(s, rb, r0, k);
     // rows 2r and 2r + 1 share a row pair of the swizzle: the second is 64 bytes on
-    if constexpr (MODE == kReal || MODE == kSplitRe) {
+    if constexpr (MODE == kDouble) {
+      double x[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) x[e] = k + e < K ? pd[k + e] : 0.0;
+      digits4(x, s0, q);
+#pragma unroll
+      for (int i = 0; i < kS; i++) *reinterpret_cast<unsigned*>(o + i * plane) = q[i];
+    } else if constexpr (MODE == kReal || MODE == kSplitRe) {
       double x[4], y[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) {
@@ -183,16 +171,203 @@ slice_kernel(RowSrc src, int nrows, int K, Slices s) {
     }
   }
 }
+// Largest magnitudes (as bits) of the real (m0) and imaginary (m1) parts of entries
+// [k0, k1), thread t of nt.
+template <int MODE>
+AFQ_D void row_max(const z_t* __restrict__ p, int k0, int k1, int t, int nt,
+                   unsigned long long& m0, unsigned long long& m1) {
+  m0 = m1 = 0;
+  const double* pd = reinterpret_cast<const double*>(p);
+  for (int k = k0 + t; k < k1; k += nt) {
+    if constexpr (MODE == kDouble) {
+      m0 = max(m0, absbits(pd[k]));
+    } else {
+      const z_t v = p[k];
+      m0 = max(m0, absbits(v.x));
+      m1 = max(m1, absbits(v.y));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+}
+template <int MODE>
+AFQ_D void put_scales(const Slices& s, int rb, int r0, const RowScale& s0, const RowScale& s1) {
+  double* sc = s.scale + (long long)rb * s.rows + r0;
+  sc[0] = s0.scale;
+  if constexpr (MODE == kSplitRe || MODE == kSplitCx) sc[1] = s1.scale;
+}
+AFQ_D const z_t* src_row(const RowSrc& src, int r, bool dbl) {
+  if (!dbl) return src.row(r);
+  return reinterpret_cast<const z_t*>(reinterpret_cast<const double*>(src.p) +
+                                      (r / src.per) * src.hi + (r % src.per) * src.lo);
+}
 
-// Slices nrows source rows of K complex entries into `s` (its first rows).
+// One warp per source row: the row's maximum, then its digits (the second read hits L1 or
+// L2).  Memory bound: 16 bytes read per complex entry, 14 (28 for kSplitCx) written.
+template <int MODE>
+__global__ void __launch_bounds__(256)
+slice_kernel(RowSrc src, int nrows, int K, Slices s) {
+  constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
+  const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= nrows) return;
+  const z_t* p = src_row(src, r, MODE == kDouble);
+  unsigned long long m0, m1;
+  row_max<MODE>(p, 0, K, lane, 32, m0, m1);
+  if constexpr (MODE == kPairs || MODE == kSplitCx) m0 = m1 = max(m0, m1);
+  const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
+  const int rb = r / s.per_batch(TWO), r0 = (r - rb * s.per_batch(TWO)) * (TWO ? 2 : 1);
+  if (lane == 0) put_scales<MODE>(s, rb, r0, s0, s1);
+  slice_row<MODE>(p, K, s, rb, r0, s0, s1, 0, s.nslab * oz::kSlab, lane, 32);
+}
+// One cluster of 8 CTAs per source row (long rows: the 2nN entries of a walker's density
+// matrix, 590 KB at 384 orbitals): each CTA takes an eighth of the row and reads the others'
+// maxima from their shared memory.
+constexpr int kSliceCluster = 8;
+template <int MODE>
+__global__ void __cluster_dims__(kSliceCluster, 1, 1) __launch_bounds__(256)
+slice_cluster_kernel(RowSrc src, int K, Slices s) {
+  constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
+  constexpr bool PAIR = MODE == kPairs || MODE == kSplitCx;   // two digits per entry
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ unsigned long long red[2][8], mx[2];
+  const int r = blockIdx.x / kSliceCluster, part = blockIdx.x % kSliceCluster;
+  const z_t* p = src_row(src, r, MODE == kDouble);
+  const int Kp = s.nslab * oz::kSlab;
+  const int per = (s.nslab + kSliceCluster - 1) / kSliceCluster * oz::kSlab;
+  const int kd0 = min(Kp, part * per), kd1 = min(Kp, kd0 + per);
+  unsigned long long m0, m1;
+  row_max<MODE>(p, PAIR ? kd0 / 2 : kd0, min(K, PAIR ? kd1 / 2 : kd1), threadIdx.x, 256, m0, m1);
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = m0;
+    red[1][threadIdx.x >> 5] = m1;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned long long m = 0;
+    for (int i = 0; i < 8; i++) m = max(m, red[threadIdx.x][i]);
+    mx[threadIdx.x] = m;
+  }
+  cl.sync();
+  m0 = m1 = 0;
+#pragma unroll
+  for (int q = 0; q < kSliceCluster; q++) {
+    const unsigned long long* o = cl.map_shared_rank(mx, q);
+    m0 = max(m0, o[0]);
+    m1 = max(m1, o[1]);
+  }
+  cl.sync();   // every CTA's shared memory stays until all have read it
+  if constexpr (PAIR) m0 = m1 = max(m0, m1);
+  const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
+  const int rb = r / s.per_batch(TWO), r0 = (r - rb * s.per_batch(TWO)) * (TWO ? 2 : 1);
+  if (part == 0 && threadIdx.x == 0) put_scales<MODE>(s, rb, r0, s0, s1);
+  slice_row<MODE>(p, K, s, rb, r0, s0, s1, kd0, kd1, threadIdx.x, 256);
+}
+
+// Slices nrows source rows of K entries into `s` (its first rows).  Rows above 1024 entries
+// get a cluster each (16 rows of 2048 entries at one warp a row would fill two SMs).
 template <int MODE>
 cudaError_t slice_rows(const RowSrc& src, int nrows, int K, const Slices& s, cudaStream_t st) {
   if (nrows <= 0) return cudaSuccess;
-  if (K > 2048)
-    slice_kernel<MODE, true><<<nrows, 256, 0, st>>>(src, nrows, K, s);
+  if (K > 1024)
+    slice_cluster_kernel<MODE><<<nrows * kSliceCluster, 256, 0, st>>>(src, K, s);
   else
-    slice_kernel<MODE, false><<<(nrows + 7) / 8, 256, 0, st>>>(src, nrows, K, s);
+    slice_kernel<MODE><<<(nrows + 7) / 8, 256, 0, st>>>(src, nrows, K, s);
   return cudaGetLastError();
+}
+
+// X [nchol][nw] -> rows (w, re | im): a cluster of 8 CTAs per 32 walkers, lanes on walkers
+// (coalesced reads of X's rows), 16 digits per thread and store.
+template <bool REALA>
+__global__ void __cluster_dims__(kSliceCluster, 1, 1) __launch_bounds__(256)
+slice_x_kernel(const z_t* __restrict__ X, int nc, int nw, Slices s) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ unsigned long long red[2][8][32], mx[2][32];
+  const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+  const int w = blockIdx.x / kSliceCluster * 32 + lane, part = blockIdx.x % kSliceCluster;
+  unsigned long long m0 = 0, m1 = 0;
+  if (w < nw)
+    for (int c = part * 8 + wy; c < nc; c += 8 * kSliceCluster) {
+      const z_t v = X[(long long)c * nw + w];
+      m0 = max(m0, absbits(v.x));
+      m1 = max(m1, absbits(v.y));
+    }
+  red[0][wy][lane] = m0;
+  red[1][wy][lane] = m1;
+  __syncthreads();
+  if (wy < 2) {
+    unsigned long long m = 0;
+    for (int i = 0; i < 8; i++) m = max(m, red[wy][i][lane]);
+    mx[wy][lane] = m;
+  }
+  cl.sync();
+  m0 = m1 = 0;
+#pragma unroll
+  for (int q = 0; q < kSliceCluster; q++) {
+    const unsigned long long* o = cl.map_shared_rank(&mx[0][0], q);
+    m0 = max(m0, o[lane]);
+    m1 = max(m1, o[32 + lane]);
+  }
+  cl.sync();   // every CTA's shared memory stays until all have read it
+  if (w >= nw) return;
+  if (!REALA) m0 = m1 = max(m0, m1);
+  const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
+  if (part == 0 && wy == 0) {
+    s.scale[2 * w] = s0.scale;
+    s.scale[2 * w + 1] = s1.scale;
+  }
+  const int plane = s.tile * oz::kSlab, Kp = s.nslab * oz::kSlab;
+  constexpr int NE = REALA ? 16 : 8;   // source entries per 16 digits
+  for (int k = 16 * (part * 8 + wy); k < Kp; k += 16 * 8 * kSliceCluster) {
+    z_t v[NE];
+#pragma unroll
+    for (int e = 0; e < NE; e++) {
+      const int c = (REALA ? k : k / 2) + e;
+      v[e] = c < nc ? X[(long long)c * nw + w] : zmk(0, 0);
+    }
+    int8_t* o = s.d + oz::slice_offset(s, 0, 2 * w, k);
+#pragma unroll
+    for (int row = 0; row < 2; row++) {
+      unsigned q[4][kS];
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
+        double x[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          if (REALA) {
+            x[e] = row ? v[4 * g + e].y : v[4 * g + e].x;
+          } else {   // row 0: (re, -im) pairs, row 1: (im, re) pairs
+            const z_t z = v[2 * g + e / 2];
+            x[e] = row ? (e & 1 ? z.x : z.y) : (e & 1 ? -z.y : z.x);
+          }
+        }
+        digits4(x, row ? s1 : s0, q[g]);
+      }
+#pragma unroll
+      for (int i = 0; i < kS; i++)
+        *reinterpret_cast<uint4*>(o + i * plane + row * oz::kSlab) =
+            make_uint4(q[0][i], q[1][i], q[2][i], q[3][i]);
+    }
+  }
+}
+
+// W [nw][N][n2] -> Wt [nw][n2][N]
+__global__ void __launch_bounds__(256)
+transpose_kernel(const z_t* __restrict__ W, int N, int n2, z_t* __restrict__ Wt) {
+  __shared__ z_t t[32][33];
+  const int w = blockIdx.z, k0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  const z_t* src = W + (long long)w * N * n2;
+  z_t* dst = Wt + (long long)w * N * n2;
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  for (int i = y; i < 32; i += 8)
+    if (k0 + i < N && j0 + x < n2) t[i][x] = src[(long long)(k0 + i) * n2 + j0 + x];
+  __syncthreads();
+  for (int i = y; i < 32; i += 8)
+    if (j0 + i < n2 && k0 + x < N) dst[(long long)(j0 + i) * N + k0 + x] = t[x][i];
 }
 
 __global__ void oz_check_imag_kernel(const z_t* __restrict__ src, long long count, int* flag) {
@@ -232,6 +407,81 @@ struct EpiRows {
       if (n0 + i < ld) oz::store4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
   }
 };
+
+// Partial products of a K split: part[z][m][n] (ld a multiple of 4).
+struct EpiPart {
+  double* C;
+  long long ld, sz;
+  int M;
+  AFQ_D void operator()(int z, int m, int n0, const double* v) const {
+    EpiRows{C + z * sz, ld, M}(0, m, n0, v);
+  }
+};
+// vHS: row m = ik, columns (w, re | im); lanes on consecutive ik.
+struct EpiV {
+  z_t* V;
+  long long N2;
+  int nw;
+  AFQ_D void operator()(int, int m, int n0, const double* v) const {
+    if (m >= N2) return;
+    const int w0 = n0 / 2;
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (w0 + i < nw) V[(w0 + i) * N2 + m] = zmk(v[2 * i], v[2 * i + 1]);
+  }
+};
+// Propagation, columns (j, re | im) of walker z, S and T [nw][2n][N] (lanes on consecutive
+// rows).  k = 0: S = v.  k > 0: T = (i / k) v, S += T, T stored unless last.
+struct EpiChain {
+  z_t *S, *T;
+  int N, n2, k, last;
+  AFQ_D void operator()(int z, int m, int n0, const double* v) const {
+    if (m >= N) return;
+    const int j0 = n0 / 2;
+    const long long o = ((long long)z * n2 + j0) * N + m;
+    if (k == 0) {
+#pragma unroll
+      for (int i = 0; i < 16; i++)
+        if (j0 + i < n2) S[o + (long long)i * N] = zmk(v[2 * i], v[2 * i + 1]);
+      return;
+    }
+    const double f = 1.0 / (double)k;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      if (j0 + i >= n2) break;
+      const z_t t = zmk(-f * v[2 * i + 1], f * v[2 * i]);
+      z_t* s = S + o + (long long)i * N;
+      *s = zadd(*s, t);
+      if (!last) T[o + (long long)i * N] = t;
+    }
+  }
+};
+// W[z][m][j]: a lane owns an orbital row (32-byte stores; 2n is even).
+struct EpiW {
+  z_t* W;
+  int N, n2;
+  AFQ_D void operator()(int z, int m, int n0, const double* v) const {
+    if (m >= N) return;
+    const int j0 = n0 / 2;
+    double* p = reinterpret_cast<double*>(W + ((long long)z * N + m) * n2 + j0);
+#pragma unroll
+    for (int i = 0; i < 32; i += 4)
+      if (j0 + i / 2 < n2) oz::store4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+  }
+};
+// out[r][w] = sum over the K splits of the partial products, in order.
+__global__ void __launch_bounds__(256)
+part_sum_kernel(const double* __restrict__ part, long long ld, long long sz, int splits, int rows,
+                int nw, z_t* __restrict__ out) {
+  const long long tot = (long long)rows * nw;
+  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < tot; e += gridDim.x * 256LL) {
+    const long long r = e / nw, w = e - r * nw;
+    const z_t* p = reinterpret_cast<const z_t*>(part + r * ld) + w;
+    z_t t = p[0];
+    for (int q = 1; q < splits; q++) t = zadd(t, p[q * (sz / 2)]);
+    out[e] = t;
+  }
+}
 
 // Kpart[w][s][c] = tr(T T), T the n x n block of (c, w) in the chunk's product (rows
 // row0 + c n + a, columns w n + b).  One CTA per block, which passes through shared memory
@@ -275,52 +525,168 @@ trace_kernel(const z_t* __restrict__ T, int n, long long ld, int row0, int c_fir
 
 }  // namespace
 
-cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
-  *out = nullptr;
+namespace {
+
+// device bytes left for the next group of allocations: none takes more than a third
+bool fits(cudaError_t& e, size_t need) {
+  size_t free_b = 0, total_b = 0;
+  if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total_b);
+  return e == cudaSuccess && need < free_b / 3;
+}
+size_t slice_bytes(long long rows, long long K) { return (size_t)kS * (rows + 128) * (K + 64); }
+
+cudaError_t create_exchange(OzState* o, cudaStream_t st) {
+  const OzInit& in = o->in;
   const int N = in.N, n = in.n, nc = in.nchol, nw = in.nw;
   const long long NAK = 2LL * n * N;
+  cudaError_t e = is_real(o, in.Lh, (long long)nc * NAK, &o->lreal, st);
+  const int K = o->lreal ? N : 2 * N;
+  // chunk of T: walkers first (in whole 64-column tiles, up to 32 MB per 128 rows), then
+  // Cholesky vectors, up to 64 MB (half of L2)
+  const long long cap = 64LL << 20;
+  o->ex_w = (int)std::min<long long>(nw, std::max(32LL, (32LL << 20) / (16LL * 128 * n) / 32 * 32));
+  const long long per_c = 16LL * (o->ex_w + 1) * n * n;
+  o->ex_c = (int)std::max(1LL, std::min<long long>(nc, cap / per_c));
+  int whole = oz::kBM;   // Cholesky vectors that fill whole row tiles, within 1.25 caps
+  while (whole > 1 && (whole / 2 * n) % oz::kBM == 0) whole /= 2;
+  if (o->ex_c < nc && whole * per_c <= cap + cap / 4)
+    o->ex_c = (int)((cap + cap / 4) / per_c / whole) * whole;
+  const size_t tb = per_c * o->ex_c + 256LL * 16 * (o->ex_w + 1) * n;   // whole row tiles
+  if (!fits(e, 2 * slice_bytes((long long)nc * n, K) + slice_bytes(2LL * nw * n, K) + tb)) return e;
+  for (int s = 0; s < 2 && e == cudaSuccess; s++) {
+    e = alloc_slices(o, &o->lx[s], oz::kBM, nc * n, 1, K);
+    if (e != cudaSuccess) break;
+    const RowSrc src{in.Lh + (long long)s * n * N, n, NAK, N};
+    e = o->lreal ? slice_rows<kReal>(src, nc * n, N, o->lx[s], st)
+                 : slice_rows<kPairs>(src, nc * n, N, o->lx[s], st);
+  }
+  if (e == cudaSuccess) e = alloc_slices(o, &o->gx, oz::kBN, 2 * nw * n, 1, K);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->T, tb / sizeof(double));
+  o->exchange = e == cudaSuccess;
+  return e;
+}
+
+// Products with G.  K splits fill the SMs when the output tiles do not (and bound a split's
+// K for the int32 accumulators), at least two slabs each.
+cudaError_t create_gsites(OzState* o, cudaStream_t st) {
+  const OzInit& in = o->in;
+  const int nw = in.nw;
+  const long long NAK = 2LL * in.n * in.N;
+  const z_t* src[OZ_NG] = {in.SpvnT, in.Lh, in.Vakbl};
+  const long long rows[OZ_NG] = {in.nchol, in.nchol, NAK};
+  cudaError_t e = cudaSuccess;
+  o->greal = true;
+  size_t need = 0;
+  for (int i = 0; i < OZ_NG; i++)
+    if (src[i]) {
+      bool real = false;
+      if (e == cudaSuccess) e = is_real(o, src[i], rows[i] * NAK, &real, st);
+      o->greal = o->greal && real;
+      need += slice_bytes(rows[i], NAK);
+    }
+  const int K = (int)(o->greal ? NAK : 2 * NAK);
+  if (!o->greal) need *= 2;
+  o->part_ld = (2LL * nw + 3) / 4 * 4;
+  size_t pmax = 0;
+  for (int i = 0; i < OZ_NG; i++) {
+    if (!src[i]) continue;
+    OzState::GSite& g = o->gs[i];
+    g.rows = (int)rows[i];
+    const int nslab = (K + oz::kSlab - 1) / oz::kSlab;
+    const int tiles = ((g.rows + oz::kBM - 1) / oz::kBM) * ((2 * nw + oz::kBN - 1) / oz::kBN);
+    const int least = (K + oz::kMaxK - 1) / oz::kMaxK;
+    const int sp = std::max(least, std::min(std::max(1, tc::sm_count() / tiles), nslab / 2));
+    g.slab_split = (nslab + sp - 1) / sp;
+    g.splits = (nslab + g.slab_split - 1) / g.slab_split;
+    pmax = std::max(pmax, (size_t)(g.splits * rows[i] * o->part_ld));
+  }
+  if (!pmax || !fits(e, need + slice_bytes(2 * nw, K) + 8 * pmax)) return e;
+  if (e == cudaSuccess) e = alloc_slices(o, &o->gb, oz::kBN, 2 * nw, 1, K);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->part, pmax);
+  for (int i = 0; i < OZ_NG && e == cudaSuccess; i++) {
+    if (!src[i]) continue;
+    OzState::GSite& g = o->gs[i];
+    e = alloc_slices(o, &g.a, oz::kBM, g.rows, 1, K);
+    const RowSrc rs{src[i], 1, NAK, 0};
+    if (e == cudaSuccess)
+      e = o->greal ? slice_rows<kReal>(rs, g.rows, (int)NAK, g.a, st)
+                   : slice_rows<kPairs>(rs, g.rows, (int)NAK, g.a, st);
+    g.on = e == cudaSuccess;
+  }
+  return e;
+}
+
+// vHS as a dense product.  The CSR kernel does nnz x nw real (complex) multiply-adds at about
+// 2.9e12 (1.4e12) a second (C4's 45.3 M nonzeros x 128 walkers: 3.89 ms; 0.42 M x 256: 90
+// us), a tile slab here takes about 0.55 us of one SM plus 2 us per tile and 15 us of
+// launches: the smaller of the two estimates.
+cudaError_t create_vhs(OzState* o, cudaStream_t st) {
+  const OzInit& in = o->in;
+  const long long N2 = (long long)in.N * in.N;
+  cudaError_t e = cudaSuccess;
+  o->sreal = in.Spvn_r != nullptr;
+  if ((!in.Spvn_r && !in.Spvn) || N2 > (1LL << 30)) return e;
+  const int K = o->sreal ? in.nchol : 2 * in.nchol;
+  if (K > oz::kMaxK) return e;
+  const double csr = (double)in.spvn_nnz * in.nw / (o->sreal ? 2.9e12 : 1.45e12);
+  const long long tiles = (N2 + oz::kBM - 1) / oz::kBM * ((2LL * in.nw + oz::kBN - 1) / oz::kBN);
+  const double dense = 15e-6 + (double)((tiles + 147) / 148) *
+                                   (2e-6 + 1.0e-6 * ((K + oz::kSlab - 1) / oz::kSlab));
+  if (dense >= csr) return e;
+  if (!fits(e, slice_bytes(N2, K) + slice_bytes(2LL * in.nw, K))) return e;
+  e = alloc_slices(o, &o->sp, oz::kBM, (int)N2, 1, K);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->xb, oz::kBN, 2 * in.nw, 1, K);
+  if (e == cudaSuccess)
+    e = o->sreal ? slice_rows<kDouble>(
+                       RowSrc{reinterpret_cast<const z_t*>(in.Spvn_r), 1, in.nchol, 0}, (int)N2,
+                       in.nchol, o->sp, st)
+                 : slice_rows<kPairs>(RowSrc{in.Spvn, 1, in.nchol, 0}, (int)N2, in.nchol, o->sp, st);
+  o->vhs = e == cudaSuccess;
+  return e;
+}
+
+// Propagation: from 3e8 real operations per product (14 us of the FP64 pipe at the measured
+// 22 TFLOP/s, above the launches of the splitting kernels).
+cudaError_t create_propagate(OzState* o, cudaStream_t st) {
+  const OzInit& in = o->in;
+  const int N = in.N, n2 = 2 * in.n, nw = in.nw;
+  cudaError_t e = cudaSuccess;
+  if (8.0 * N * (double)N * n2 * nw < 3e8 || 2 * N > oz::kMaxK || nw > 65535) return e;
+  e = is_real(o, in.P, (long long)N * N, &o->preal, st);
+  const int Kp = o->preal ? N : 2 * N;
+  if (!fits(e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
+                                                  slice_bytes(2 * n2, 2 * N))))
+    return e;
+  if (e == cudaSuccess) e = alloc_slices(o, &o->pa, oz::kBM, N, 1, Kp);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->va, oz::kBM, N, nw, 2 * N);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->pb, oz::kBN, 2 * n2, nw, Kp);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->tb, oz::kBN, 2 * n2, nw, 2 * N);
+  if (e == cudaSuccess)
+    e = o->preal ? slice_rows<kReal>(RowSrc{in.P, 1, N, 0}, N, N, o->pa, st)
+                 : slice_rows<kPairs>(RowSrc{in.P, 1, N, 0}, N, N, o->pa, st);
+  o->prop = e == cudaSuccess;
+  return e;
+}
+
+}  // namespace
+
+cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
+  *out = nullptr;
   OzState* o = new OzState();
   o->in = in;
   cudaError_t e = oz_alloc(o, &o->err, 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
-  if (e == cudaSuccess && in.Lh && n <= 64) {
-    e = is_real(o, in.Lh, (long long)nc * NAK, &o->lreal, st);
-    const int K = o->lreal ? N : 2 * N;
-    // chunk of T: walkers first (in whole 64-column tiles, up to 32 MB per 128 rows), then
-    // Cholesky vectors, up to 64 MB (half of L2)
-    const long long cap = 64LL << 20;
-    o->ex_w = (int)std::min<long long>(nw, std::max(32LL, (32LL << 20) / (16LL * 128 * n) / 32 * 32));
-    const long long per_c = 16LL * (o->ex_w + 1) * n * n;
-    o->ex_c = (int)std::max(1LL, std::min<long long>(nc, cap / per_c));
-    int whole = oz::kBM;   // Cholesky vectors that fill whole row tiles, within 1.25 caps
-    while (whole > 1 && (whole / 2 * n) % oz::kBM == 0) whole /= 2;
-    if (o->ex_c < nc && whole * per_c <= cap + cap / 4)
-      o->ex_c = (int)((cap + cap / 4) / per_c / whole) * whole;
-    const size_t tb = per_c * o->ex_c + 256LL * 16 * (o->ex_w + 1) * n;   // whole row tiles
-    size_t free_b = 0, total_b = 0;
-    if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total_b);
-    const size_t need = 2 * (size_t)kS * (nc * n + 128) * (K + 64) +
-                        (size_t)kS * (2 * nw * n + 64) * (K + 64) + tb;
-    if (e == cudaSuccess && need < free_b / 2) {
-      for (int s = 0; s < 2 && e == cudaSuccess; s++) {
-        e = alloc_slices(o, &o->lx[s], oz::kBM, nc * n, 1, K);
-        if (e != cudaSuccess) break;
-        const RowSrc src{in.Lh + (long long)s * n * N, n, NAK, N};
-        e = o->lreal ? slice_rows<kReal>(src, nc * n, N, o->lx[s], st)
-                     : slice_rows<kPairs>(src, nc * n, N, o->lx[s], st);
-      }
-      if (e == cudaSuccess) e = alloc_slices(o, &o->gx, oz::kBN, 2 * nw * n, 1, K);
-      if (e == cudaSuccess) e = oz_alloc(o, &o->T, tb / sizeof(double));
-      if (e == cudaSuccess) o->exchange = true;
-    }
-  }
+  if (e == cudaSuccess && in.Lh && in.n <= 64) e = create_exchange(o, st);
+  if (e == cudaSuccess) e = create_gsites(o, st);
+  if (e == cudaSuccess) e = create_vhs(o, st);
+  if (e == cudaSuccess) e = create_propagate(o, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaErrorMemoryAllocation) {   // the FP64 pipe's kernels need none of this
     cudaGetLastError();
     oz_destroy(o);
     return cudaSuccess;
   }
-  if (e != cudaSuccess || !o->exchange) {
+  if (e != cudaSuccess) {
     oz_destroy(o);
     return e;
   }
@@ -332,6 +698,71 @@ void oz_destroy(OzState* o) {
   if (!o) return;
   for (void* p : o->allocs) cudaFree(p);
   delete o;
+}
+
+bool oz_has_gsite(const OzState* o, int site) { return o && o->gs[site].on; }
+int oz_gsite_launches(const OzState*, int) { return 3; }
+
+cudaError_t oz_gsite(OzState* o, int site, const z_t* Gc, z_t* out, cudaStream_t st) {
+  const OzState::GSite& g = o->gs[site];
+  const int nw = o->in.nw, NAK = 2 * o->in.n * o->in.N;
+  const RowSrc src{Gc, 1, NAK, 0};
+  cudaError_t e = o->greal ? slice_rows<kSplitRe>(src, nw, NAK, o->gb, st)
+                           : slice_rows<kSplitCx>(src, nw, NAK, o->gb, st);
+  if (e != cudaSuccess) return e;
+  const long long sz = g.rows * o->part_ld;
+  oz::Gemm gm{&g.a, &o->gb, g.rows, 2 * nw, g.splits, 0, 0, g.slab_split};
+  e = oz::launch<7>(gm, EpiPart{o->part, o->part_ld, sz, g.rows}, o->err, st);
+  if (e != cudaSuccess) return e;
+  const long long tot = (long long)g.rows * nw;
+  part_sum_kernel<<<(unsigned)std::min<long long>((tot + 255) / 256, 148 * 16), 256, 0, st>>>(
+      o->part, o->part_ld, sz, g.splits, g.rows, nw, out);
+  return cudaGetLastError();
+}
+
+bool oz_has_vhs(const OzState* o) { return o && o->vhs; }
+
+cudaError_t oz_vhs(OzState* o, const z_t* X, z_t* vHS, cudaStream_t st) {
+  const int nw = o->in.nw, nc = o->in.nchol;
+  const int grid = (nw + 31) / 32 * kSliceCluster;
+  if (o->sreal)
+    slice_x_kernel<true><<<grid, 256, 0, st>>>(X, nc, nw, o->xb);
+  else
+    slice_x_kernel<false><<<grid, 256, 0, st>>>(X, nc, nw, o->xb);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const long long N2 = (long long)o->in.N * o->in.N;
+  oz::Gemm g{&o->sp, &o->xb, (int)N2, 2 * nw, 1};
+  g.m_fast = false;   // the CTAs that share an Spvn tile run together
+  return oz::launch<7>(g, EpiV{vHS, N2, nw}, o->err, st);
+}
+
+bool oz_has_propagate(const OzState* o) { return o && o->prop; }
+int oz_propagate_launches(const OzState* o) { return 1 + 1 + 2 * (2 + o->in.order); }
+
+cudaError_t oz_propagate(OzState* o, z_t* W, const z_t* vHS, z_t* S, z_t* T, cudaStream_t st) {
+  const int N = o->in.N, n2 = 2 * o->in.n, nw = o->in.nw, order = o->in.order;
+  transpose_kernel<<<dim3((N + 31) / 32, (n2 + 31) / 32, nw), 256, 0, st>>>(W, N, n2, T);
+  cudaError_t e = cudaGetLastError();
+  auto pslice = [&](const z_t* src) {   // walker columns as the B operand of Propg1
+    const RowSrc rs{src, 1, N, 0};
+    return o->preal ? slice_rows<kSplitRe>(rs, nw * n2, N, o->pb, st)
+                    : slice_rows<kSplitCx>(rs, nw * n2, N, o->pb, st);
+  };
+  if (e == cudaSuccess) e = pslice(T);
+  oz::Gemm g{&o->pa, &o->pb, N, 2 * n2, nw};
+  if (e == cudaSuccess) e = oz::launch<8>(g, EpiChain{S, T, N, n2, 0, 0}, o->err, st);
+  if (e == cudaSuccess && order > 0)
+    e = slice_rows<kPairs>(RowSrc{vHS, 1, N, 0}, nw * N, N, o->va, st);
+  oz::Gemm gv{&o->va, &o->tb, N, 2 * n2, nw};
+  for (int k = 1; k <= order && e == cudaSuccess; k++) {
+    e = slice_rows<kSplitCx>(RowSrc{k == 1 ? S : T, 1, N, 0}, nw * n2, N, o->tb, st);
+    if (e == cudaSuccess)
+      e = oz::launch<8>(gv, EpiChain{S, T, N, n2, k, k == order}, o->err, st);
+  }
+  if (e == cudaSuccess) e = pslice(S);
+  if (e == cudaSuccess) e = oz::launch<8>(g, EpiW{W, N, n2}, o->err, st);
+  return e;
 }
 
 bool oz_has_exchange(const OzState* o, int nwalk) { return o && o->exchange && nwalk <= o->in.nw; }
@@ -369,7 +800,7 @@ cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nb
         oz::Gemm g{&o->lx[s], &o->gx, row0 + c * n, 2 * w * n, 1, t0, 2 * w0 * n / oz::kBN};
         const long long ld = (2LL * w * n + 3) / 4 * 4;
         EpiRows epi{o->T, ld, row0 + c * n};
-        if ((e = oz::launch(g, epi, o->err, st)) != cudaSuccess) break;
+        if ((e = oz::launch<7>(g, epi, o->err, st)) != cudaSuccess) break;
         trace_kernel<<<dim3(c, w), kTraceThreads, smem, st>>>(
             reinterpret_cast<const z_t*>(o->T), n, ld / 2, row0, c0, Kpart, nblk, w0, s);
         e = cudaGetLastError();

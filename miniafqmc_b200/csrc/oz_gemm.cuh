@@ -5,17 +5,22 @@
 // al., "Error-free transformations of matrix multiplication", 2012):
 //   x = 2^e sum_{i=1..S} d_i 2^-(8i - 1),   d_i in [-128, 127]
 // (55 bits below the row's power of two for S = 7).  The products d_i d_j with i + j = D
-// share one weight, so D' = S accumulators per output hold all pairs with i + j <= S + 1,
+// share one weight, so ND accumulators per output hold all pairs with i + j <= ND + 1,
 //   acc_D = sum_{i + j = D} sum_k a_i[m][k] b_j[n][k]      (exact in int32),
-// and the FP64 result is sum_D acc_D 2^(2 - 8D), times the two row scales.  The dropped
-// pairs lie below 2^-57 of (row maximum) x (column maximum).
+// and the FP64 result is sum_D acc_D 2^(2 - 8D), times the two row scales.  With ND = 7 (28
+// pairs) the dropped pairs add an error of about 2^-56 sqrt(K) (row scale) x (column
+// scale): below an FP64 chain's rounding where the sums are as large as their terms.  ND = 8
+// (34 pairs, 2^-63) serves the propagation, whose operands are near the identity: the row
+// scale is that of the diagonal, the results are 20 times smaller (measured over a
+// substep at 128 and 384 orbitals: ND = 7 3.0e-15 and 4.9e-15 of W, the FP64 pipe 6.4e-16
+// and 1.1e-15).
 //
-// Layout and tile.  TMEM holds 512 columns of 32-bit accumulators, so S = 7 accumulators
-// allow a 128 x 64 output tile (448 columns).  The seven B slices of a tile sit one after
+// Layout and tile.  TMEM holds 512 columns of 32-bit accumulators, so 7 or 8 accumulators
+// allow a 128 x 64 output tile.  The seven B slices of a tile sit one after
 // the other in shared memory (64 rows each), so the products of A slice i with B slices
 // 1 .. S + 1 - i are ONE matrix product of N = 64 (S + 1 - i) columns whose accumulators
 // are consecutive in TMEM, starting at accumulator i: ten tcgen05.mma per 32 bytes of K
-// instead of 28, and each A slice is read from shared memory once or twice.
+// instead of 28 (ND = 7), and each A slice is read from shared memory once or twice.
 // What bounds it: operand supply.  A K slab of 64 bytes costs 7 x (128 + 64) x 64 = 86 KB
 // for 1792 tensor-pipe clocks (48 bytes per clock and SM from L2).
 //
@@ -42,7 +47,7 @@ static_assert((long long)kS * 128 * 128 * kMaxK < (1LL << 31), "int32 accumulati
 // acc_5 2^24 + acc_6 2^16 + acc_7 2^8 + acc_8 (4, 5, 6 and 7 pairs) below 2^51 for K <= 1024
 static_assert((4LL * (1 << 24) + 5 * (1 << 16) + 6 * (1 << 8) + 7) * 128 * 128 * 1024 < (1LL << 51),
               "one integer for the four low accumulators");
-static_assert(kS * kBN <= 512 && kSmem <= 227 * 1024, "TMEM / shared memory");
+static_assert((kS + 1) * kBN <= 512 && kSmem <= 227 * 1024, "TMEM / shared memory");
 
 // Digit slices of a batch of rows, stored as the shared-memory images the MMAs read: for
 // each batch, tile of R rows (R = 128 for an A operand, 64 for a B operand) and K slab, the
@@ -123,13 +128,15 @@ AFQ_D long long mad_wide(int a, int b, long long c) {
   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
   return d;
 }
-template <bool SHORT>
-AFQ_D double combine(const int (&a)[kS]) {
+// The low part of the 8-accumulator form is acc_8 2^8 + acc_9.
+template <int ND, bool SHORT>
+AFQ_D double combine(const int (&a)[ND]) {
   constexpr double kMagic = 6755399441055744.0;
   const double hi = __longlong_as_double(mad_wide(
                         a[2], 1, mad_wide(a[1], 1 << 8, mad_wide(a[0], 1 << 16, kMagicBits)))) -
                     kMagic;
   if constexpr (SHORT) {
+    static_assert(ND == 7, "one low sum: seven accumulators");
     const double lo = __longlong_as_double(mad_wide(
                           a[6], 1, mad_wide(a[5], 1 << 8, mad_wide(a[4], 1 << 16,
                                    mad_wide(a[3], 1 << 24, kMagicBits))))) -
@@ -139,32 +146,62 @@ AFQ_D double combine(const int (&a)[kS]) {
   const double mid = __longlong_as_double(mad_wide(
                          a[5], 1, mad_wide(a[4], 1 << 8, mad_wide(a[3], 1 << 16, kMagicBits)))) -
                      kMagic;
-  const double lo = __longlong_as_double(mad_wide(a[6], 1, kMagicBits)) - kMagic;
-  return fma(fma(lo, 0x1p-8, mid), 0x1p-24, hi);
+  if constexpr (ND == 7) {
+    const double lo = __longlong_as_double(mad_wide(a[6], 1, kMagicBits)) - kMagic;
+    return fma(fma(lo, 0x1p-8, mid), 0x1p-24, hi);
+  } else {
+    const double lo =
+        __longlong_as_double(mad_wide(a[7], 1, mad_wide(a[6], 1 << 8, kMagicBits))) - kMagic;
+    return fma(fma(lo, 0x1p-16, mid), 0x1p-24, hi);
+  }
 }
 
 // The 32 columns of this thread's lane at trow (accumulators kBN columns apart).
-template <bool SHORT>
+template <int ND, bool SHORT>
 AFQ_D void drain(uint32_t trow, double (&v)[32]) {
 #pragma unroll
   for (int c = 0; c < 32; c += 8) {
-    int r[kS][8];
+    int r[ND][8];
 #pragma unroll
-    for (int d = 0; d < kS; d++) tmem_ld8(trow + d * kBN + c, r[d]);
+    for (int d = 0; d < ND; d++) tmem_ld8(trow + d * kBN + c, r[d]);
     tmem_wait_ld();
 #pragma unroll
     for (int q = 0; q < 8; q++) {
-      int a[kS];
+      int a[ND];
 #pragma unroll
-      for (int d = 0; d < kS; d++) a[d] = r[d][q];
-      v[c + q] = combine<SHORT>(a);
+      for (int d = 0; d < ND; d++) a[d] = r[d][q];
+      v[c + q] = combine<ND, SHORT>(a);
+    }
+  }
+}
+
+// The MMAs of 32 bytes of K: A slice i times B slices 0 .. min(S, ND - i) - 1, whose
+// accumulators are i, i + 1, ...  FIRST starts the accumulators (slice 0 the first S, the
+// last pair of slice 1 the eighth).
+template <int ND, bool FIRST>
+AFQ_D void mma_step(uint32_t tmem, uint64_t ad, uint64_t bd) {
+#pragma unroll
+  for (int i = 0; i < kS; i++) {
+    const uint64_t ai = ad + (uint64_t)((i * kBM * kSlab) >> 4);
+    const int nj = kS < ND - i ? kS : ND - i;
+    constexpr bool kApart = FIRST && ND > kS;
+#pragma unroll
+    for (int j = 0; j < nj; j += 4) {
+      int w = nj - j < 4 ? nj - j : 4;
+      const bool tail = kApart && i == 1 && j + w == kS;   // its last column starts acc 7
+      if (tail) w--;
+      const uint64_t bj = bd + (uint64_t)((j * kBN * kSlab) >> 4);
+      umma_i8(tmem + (i + j) * kBN, ai, bj, idesc_i8(kBM, w * kBN), FIRST ? i != 0 : 1);
+      if (tail)
+        umma_i8(tmem + (i + j + w) * kBN, ai, bj + (uint64_t)((w * kBN * kSlab) >> 4),
+                idesc_i8(kBM, kBN), 0);
     }
   }
 }
 
 // Epilogue functor: epi(z, m, n, v) with v[32] the results of row m, columns n .. n + 31 of
 // the launch (rows >= M and columns >= N included: the functor checks).
-template <class Epi>
+template <int ND, class Epi>
 __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi, int* err) {
   extern __shared__ __align__(1024) uint8_t oz_smem_raw[];
@@ -253,20 +290,12 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
         tc::tc_fence_after();
         const uint64_t ad = tc::sdesc_k<kSlab>(tc::smem_u32(stA(s)));
         const uint64_t bd = tc::sdesc_k<kSlab>(tc::smem_u32(stB(s)));
+        if (k == 0)
+          mma_step<ND, true>(tmem, ad, bd);
+        else
+          mma_step<ND, false>(tmem, ad, bd);
 #pragma unroll
-        for (int u = 0; u < kSlab / 32; u++) {
-#pragma unroll
-          for (int i = 0; i < kS; i++) {   // A slice i times B slices 0 .. S - 1 - i
-            const uint64_t ai = ad + (uint64_t)((i * kBM * kSlab) >> 4) + 2 * u;
-            const uint32_t first = (k | u | i) != 0;
-#pragma unroll
-            for (int j = 0; j < kS - i; j += 4) {
-              const int nc = (kS - i - j < 4 ? kS - i - j : 4) * kBN;
-              umma_i8(tmem + (i + j) * kBN, ai, bd + (uint64_t)((j * kBN * kSlab) >> 4) + 2 * u,
-                      idesc_i8(kBM, nc), first);
-            }
-          }
-        }
+        for (int u = 1; u < kSlab / 32; u++) mma_step<ND, false>(tmem, ad + 2 * u, bd + 2 * u);
         tc::umma_commit(&empty[s]);
       }
       if (!ok) break;
@@ -296,10 +325,10 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
       }
       tc::tc_fence_after();
       double v[32];
-      if (job.slab_split ? job.slab_split <= kShortSlabs : job.nslab <= kShortSlabs)
-        drain<true>(trow, v);
+      if (ND == 7 && (job.slab_split ? job.slab_split : job.nslab) <= kShortSlabs)
+        drain<ND, ND == 7>(trow, v);
       else
-        drain<false>(trow, v);
+        drain<ND, false>(trow, v);
       tc::tc_fence_before();
       tc::mbar_arrive(acce);
       const double sa30 = sa * 0x1p-30;
@@ -325,11 +354,12 @@ struct Gemm {
   bool m_fast = true;
 };
 
-template <class Epi>
+// ND: accumulators (7, or 8 for the digit pairs one step further down).
+template <int ND, class Epi>
 cudaError_t launch(const Gemm& g, const Epi& epi, int* err, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0 || g.nbatch <= 0) return cudaSuccess;
   if (g.a->tile != kBM || g.b->tile != kBN || g.a->nslab != g.b->nslab) return cudaErrorInvalidValue;
-  auto kern = oz_gemm_kernel<Epi>;
+  auto kern = oz_gemm_kernel<ND, Epi>;
   static DeviceAttr attr;
   cudaError_t e = attr.ensure(kSmem, [kern](size_t b) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);

@@ -61,3 +61,58 @@ def test_exchange_of_a_non_finite_walker_stays_its_own():
     want, size = exchange(s.Lh, gc(e)[keep])
     assert np.all(np.abs(got[keep] - want.real) <= 64 * 33 * EPS * size)
     e.close()
+
+
+def stages(nmo, nel, nchol, nw, cplx, **kw):
+    s, e = engine(nmo, nel, nchol, nw, cplx, **kw)
+    e.calculate_mixed_density_matrix()
+    e.get_vbias()
+    e.sigma_from(np.random.default_rng(3).normal(size=(nchol, nw)))
+    return s, e
+
+
+@pytest.mark.parametrize("nmo,nel,nchol,nw,cplx", SHAPES)
+def test_vbias_and_coulomb_match_fp64(nmo, nel, nchol, nw, cplx):
+    """Products with G over K splits (a K of one slab up to several slabs per split)."""
+    s, e = stages(nmo, nel, nchol, nw, cplx)
+    G = e.copy_out("Gc")
+    A = s.SpvnT.todense()
+    size = np.abs(A) @ np.abs(G)
+    big = np.abs(A).max(1)[:, None] * np.abs(G).max(0)[None] * np.sqrt(A.shape[1])
+    assert np.all(np.abs(e.copy_out("vbias") - A @ G) <= 64 * EPS * (np.sqrt(A.shape[1]) * size + big))
+    e.calculate_energy("chol")
+    L = s.Lh.reshape(nchol, -1)
+    c, csize = L @ G, np.abs(L) @ np.abs(G)
+    ej = 0.5 * (c * c).sum(0).real
+    assert np.all(np.abs(e.copy_out("energy_parts")[:, 1] - ej)
+                  <= 256 * np.sqrt(A.shape[1]) * EPS * (csize ** 2).sum(0))
+    e.close()
+
+
+# large enough for the digit products by the rules of oz.cu: tile edges in every direction,
+# real and complex Hamiltonians, one and two row tiles, odd electron and walker counts
+@pytest.mark.parametrize("nmo,nel,nchol,nw,cplx", [(130, 9, 96, 131, False), (67, 21, 150, 83, True),
+                                                   (128, 16, 64, 80, False)])
+def test_vhs_and_propagation_match_fp64(nmo, nel, nchol, nw, cplx):
+    s, e = stages(nmo, nel, nchol, nw, cplx)
+    X = e.copy_out("X")
+    e.get_vHS()
+    V = e.copy_out("vHS")
+    A = s.Spvn.todense()
+    big = np.abs(A).max(1)[:, None] * np.abs(X).max(0)[None] * np.sqrt(nchol)
+    assert np.all(np.abs(V - A @ X) <= 64 * EPS * (np.sqrt(nchol) * (np.abs(A) @ np.abs(X)) + big))
+    W0 = e.get_walkers()[0]
+    e.propagate()
+    W1 = e.get_walkers()[0]
+    P = s.Propg1
+    for w in range(0, nw, 7):
+        Vw = V[:, w].reshape(nmo, nmo)
+        for sp in range(2):
+            T = P @ W0[w, sp]
+            S = T.copy()
+            for k in range(1, 7):
+                T = (1j / k) * (Vw @ T)
+                S = S + T
+            want = P @ S
+            assert np.max(np.abs(W1[w, sp] - want)) <= 1e-13 * np.max(np.abs(want))
+    e.close()
