@@ -16,6 +16,8 @@ using oz::Slices;
 struct OzState {
   OzInit in{};
   std::vector<void*> allocs;
+  char* block = nullptr;    // rest of the last shared block
+  size_t block_left = 0;
   int* err = nullptr;
   // exchange: rows (c, a) of Lh per spin, columns (w, b, re | im) of G, T = Lh_c Gc_w^T of a
   // chunk of Cholesky vectors and walkers
@@ -45,13 +47,27 @@ struct OzState {
 
 namespace {
 
+// Device memory of the state: small buffers share blocks (a cudaMalloc costs 0.1 to 0.2 ms,
+// most of a small system's set-up).
+constexpr size_t kBlock = 32u << 20;
 template <class T>
 cudaError_t oz_alloc(OzState* o, T** p, size_t count) {
+  const size_t bytes = (sizeof(T) * (count ? count : 1) + 255) / 256 * 256;
+  if (bytes <= o->block_left) {
+    *p = reinterpret_cast<T*>(o->block);
+    o->block += bytes;
+    o->block_left -= bytes;
+    return cudaSuccess;
+  }
   void* q = nullptr;
-  const cudaError_t e = cudaMalloc(&q, sizeof(T) * (count ? count : 1));
-  if (e == cudaSuccess) {
-    o->allocs.push_back(q);
-    *p = static_cast<T*>(q);
+  const bool shared = bytes <= kBlock / 2;
+  const cudaError_t e = cudaMalloc(&q, shared ? kBlock : bytes);
+  if (e != cudaSuccess) return e;
+  o->allocs.push_back(q);
+  *p = static_cast<T*>(q);
+  if (shared) {
+    o->block = static_cast<char*>(q) + bytes;
+    o->block_left = kBlock - bytes;
   }
   return e;
 }
@@ -375,17 +391,26 @@ __global__ void oz_check_imag_kernel(const z_t* __restrict__ src, long long coun
        e += (long long)gridDim.x * blockDim.x)
     if (src[e].y != 0.0) *flag = 1;
 }
-// every value real?  (synchronises the stream)
-cudaError_t is_real(OzState* o, const z_t* p, long long count, bool* real, cudaStream_t st) {
-  int flag = 1;
-  cudaError_t e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  oz_check_imag_kernel<<<148 * 8, 256, 0, st>>>(p, count, o->err);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  e = cudaMemcpyAsync(&flag, o->err, sizeof(int), cudaMemcpyDeviceToHost, st);
+// Which of the operands are real (synchronises the stream; null operands count as real).
+struct RealCheck {
+  const z_t* p;
+  long long count;
+  bool real;
+};
+cudaError_t check_real(OzState* o, RealCheck* c, int n, cudaStream_t st) {
+  int* flags = nullptr;
+  int host[8] = {};
+  cudaError_t e = oz_alloc(o, &flags, 8);
+  if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 8 * sizeof(int), st);
+  for (int i = 0; i < n && e == cudaSuccess; i++)
+    if (c[i].p) {
+      oz_check_imag_kernel<<<148 * 8, 256, 0, st>>>(c[i].p, c[i].count, flags + i);
+      e = cudaGetLastError();
+    }
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(host, flags, n * sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
-  *real = flag == 0;
+  for (int i = 0; i < n; i++) c[i].real = host[i] == 0;
   return e;
 }
 
@@ -539,7 +564,7 @@ cudaError_t create_exchange(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;
   const int N = in.N, n = in.n, nc = in.nchol, nw = in.nw;
   const long long NAK = 2LL * n * N;
-  cudaError_t e = is_real(o, in.Lh, (long long)nc * NAK, &o->lreal, st);
+  cudaError_t e = cudaSuccess;
   const int K = o->lreal ? N : 2 * N;
   // chunk of T: walkers first (in whole 64-column tiles, up to 32 MB per 128 rows), then
   // Cholesky vectors, up to 64 MB (half of L2)
@@ -575,15 +600,9 @@ cudaError_t create_gsites(OzState* o, cudaStream_t st) {
   const z_t* src[OZ_NG] = {in.SpvnT, in.Lh, in.Vakbl};
   const long long rows[OZ_NG] = {in.nchol, in.nchol, NAK};
   cudaError_t e = cudaSuccess;
-  o->greal = true;
   size_t need = 0;
   for (int i = 0; i < OZ_NG; i++)
-    if (src[i]) {
-      bool real = false;
-      if (e == cudaSuccess) e = is_real(o, src[i], rows[i] * NAK, &real, st);
-      o->greal = o->greal && real;
-      need += slice_bytes(rows[i], NAK);
-    }
+    if (src[i]) need += slice_bytes(rows[i], NAK);
   const int K = (int)(o->greal ? NAK : 2 * NAK);
   if (!o->greal) need *= 2;
   o->part_ld = (2LL * nw + 3) / 4 * 4;
@@ -652,7 +671,6 @@ cudaError_t create_propagate(OzState* o, cudaStream_t st) {
   const int N = in.N, n2 = 2 * in.n, nw = in.nw;
   cudaError_t e = cudaSuccess;
   if (8.0 * N * (double)N * n2 * nw < 3e8 || 2 * N > oz::kMaxK || nw > 65535) return e;
-  e = is_real(o, in.P, (long long)N * N, &o->preal, st);
   const int Kp = o->preal ? N : 2 * N;
   if (!fits(e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
                                                   slice_bytes(2 * n2, 2 * N))))
@@ -676,6 +694,15 @@ cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
   o->in = in;
   cudaError_t e = oz_alloc(o, &o->err, 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
+  const long long NAK = 2LL * in.n * in.N;
+  RealCheck rc[4] = {{in.Lh, in.nchol * NAK, true},
+                     {in.SpvnT, in.nchol * NAK, true},
+                     {in.Vakbl, NAK * NAK, true},
+                     {in.P, (long long)in.N * in.N, true}};
+  if (e == cudaSuccess) e = check_real(o, rc, 4, st);
+  o->lreal = rc[0].real;
+  o->greal = rc[0].real && rc[1].real && rc[2].real;   // one format of G for its three products
+  o->preal = rc[3].real;
   if (e == cudaSuccess && in.Lh && in.n <= 64) e = create_exchange(o, st);
   if (e == cudaSuccess) e = create_gsites(o, st);
   if (e == cudaSuccess) e = create_vhs(o, st);
