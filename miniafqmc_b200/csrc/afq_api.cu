@@ -17,6 +17,7 @@
 #include "afq_kernels.h"
 #include "afq_mixed.h"
 #include "afq_oz.h"
+#include "host_copy.h"
 #include "zgemm_fp64.cuh"
 
 using afq::launch_csr_gather;
@@ -85,6 +86,7 @@ struct afq_handle {
   int* comb_idx = nullptr;
 
   afq::MixedState* mixed = nullptr;
+  afq::HostRing* ring = nullptr;   // pinned staging of large walker copies
   afq::OzState* oz = nullptr;   // FP64 form: products on the int8 tensor cores
   afq::CvState* cv = nullptr;
   afq::CvConfig cv_cfg;
@@ -912,6 +914,7 @@ void afq_destroy(afq_handle* h) {
   }
   if (h->mixed) afq::mixed_destroy(h->mixed);
   if (h->oz) afq::oz_destroy(h->oz);
+  afq::host_ring_destroy(h->ring);
   if (h->cv) afq::cv_destroy(h->cv);
   if (h->st) cudaStreamSynchronize(h->st);
   for (void* p : h->allocs)
@@ -1039,18 +1042,15 @@ afq_status afq_set_hamiltonian(afq_handle* h, const afq_csr_z* Spvn, const afq_c
   return AFQ_OK;
 }
 
+// The reference's walker layout [nw][2][N][n] is rearranged on the device, through the
+// propagation's scratch: the caller's array crosses PCIe as it is (a host loop over the
+// entries took 16 ns each, 35 ms of a 65 MB set either way).
 afq_status afq_set_walkers(afq_handle* h, const double* W, const double* W_data) {
   if (!h || !W || !W_data) return AFQ_ERR_ARG;
-  const size_t N = h->N, n = h->n, nw = h->nw;
-  std::vector<z_t> t(nw * N * 2 * n);
-  const z_t* src = reinterpret_cast<const z_t*>(W);
-  for (size_t w = 0; w < nw; w++)
-    for (int s = 0; s < 2; s++)
-      for (size_t i = 0; i < N; i++)
-        for (size_t a = 0; a < n; a++)
-          t[(w * N + i) * 2 * n + s * n + a] = src[((w * 2 + s) * N + i) * n + a];
+  const size_t nw = h->nw, count = nw * h->N * 2 * h->n;
   cudaSetDevice(h->d.device);
-  AFQ_CUDA(h, cudaMemcpyAsync(h->W, t.data(), sizeof(z_t) * t.size(), cudaMemcpyHostToDevice, h->st));
+  AFQ_CUDA(h, afq::copy_to_device(&h->ring, h->T2, W, sizeof(z_t) * count, h->st));
+  AFQ_CUDA(h, afq::launch_walker_layout(h->T2, h->W, h->N, h->n, h->nw, 0, h->st));
   AFQ_CUDA(h, cudaMemcpyAsync(h->Wd, W_data, sizeof(z_t) * nw * 8, cudaMemcpyHostToDevice, h->st));
   AFQ_CUDA(h, cudaStreamSynchronize(h->st));
   h->have_walkers = true;
@@ -1061,18 +1061,11 @@ afq_status afq_set_walkers(afq_handle* h, const double* W, const double* W_data)
 
 afq_status afq_get_walkers(afq_handle* h, double* W, double* W_data) {
   if (!h) return AFQ_ERR_ARG;
-  const size_t N = h->N, n = h->n, nw = h->nw;
+  const size_t nw = h->nw, count = nw * h->N * 2 * h->n;
   cudaSetDevice(h->d.device);
   if (W) {
-    std::vector<z_t> t(nw * N * 2 * n);
-    AFQ_CUDA(h, cudaMemcpyAsync(t.data(), h->W, sizeof(z_t) * t.size(), cudaMemcpyDeviceToHost, h->st));
-    AFQ_CUDA(h, cudaStreamSynchronize(h->st));
-    z_t* dst = reinterpret_cast<z_t*>(W);
-    for (size_t w = 0; w < nw; w++)
-      for (int s = 0; s < 2; s++)
-        for (size_t i = 0; i < N; i++)
-          for (size_t a = 0; a < n; a++)
-            dst[((w * 2 + s) * N + i) * n + a] = t[(w * N + i) * 2 * n + s * n + a];
+    AFQ_CUDA(h, afq::launch_walker_layout(h->W, h->T2, h->N, h->n, h->nw, 1, h->st));
+    AFQ_CUDA(h, afq::copy_to_host(&h->ring, W, h->T2, sizeof(z_t) * count, h->st));
   }
   if (W_data) {
     AFQ_CUDA(h, cudaMemcpyAsync(W_data, h->Wd, sizeof(z_t) * nw * 8, cudaMemcpyDeviceToHost, h->st));

@@ -841,6 +841,32 @@ cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStr
   return cudaGetLastError();
 }
 
+// ============================================================ walker layout
+// Both layouts hold runs of n entries (orbital row i, spin s): one warp per device row,
+// 16-byte entries, coalesced on both sides.
+__global__ void __launch_bounds__(256)
+walker_layout_kernel(const z_t* __restrict__ src, z_t* __restrict__ dst, int N, int n,
+                     long long rows, int to_ref) {
+  const long long r = blockIdx.x * 8LL + (threadIdx.x >> 5);   // w N + i
+  if (r >= rows) return;
+  const long long w = r / N, i = r - w * N;
+  for (int j = threadIdx.x & 31; j < 2 * n; j += 32) {
+    const int s = j >= n;
+    const long long dev = r * 2 * n + j, ref = ((w * 2 + s) * N + i) * n + (j - s * n);
+    if (to_ref)
+      dst[ref] = src[dev];
+    else
+      dst[dev] = src[ref];
+  }
+}
+
+cudaError_t launch_walker_layout(const z_t* src, z_t* dst, int N, int n, int nw, int to_ref,
+                                 cudaStream_t st) {
+  const long long rows = (long long)nw * N;
+  walker_layout_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(src, dst, N, n, rows, to_ref);
+  return cudaGetLastError();
+}
+
 // ============================================================ exchange energy
 // K_w = 1/2 sum_{s,c} tr(T T), T = Lh_s[c] Gc_s^T (n x n), for Gn Cholesky vectors x Gw
 // walkers per CTA: a (Gn*n) x (Gw*n) complex tile over K = N, then the trace of each
