@@ -1318,17 +1318,26 @@ struct EpiExchangeStaged {
 // warpgroups, each owning BN / 2 columns = whole walkers): the K sum of T is chunked every
 // PKB slabs and added in fp32 registers.  Per walker, thread (cv, a) then sums
 // T[a][b] T[b][a] over b from its own row (registers) and column a of its Cholesky block,
-// which passes through shared memory as the real, then the imaginary parts of half the
-// block's rows at a time (scratch of 128 / n blocks x n / 2 rows x (n + 1) floats).
+// which passes through shared memory as the real, then the imaginary parts (of half the
+// block's rows at a time where the ring leaves less room).  What bounds it at C4: the trace
+// takes 4.4K of the 10.5K clocks of a tile and overlaps the next tile's first two chunks; in
+// four passes with scalar stores and 168 registers it took 8K and set the pace (tile 13.9K
+// clocks, 768 vectors x 256 walkers 5.25 -> 4.21 ms).
 template <int TWO_N, int PKB>
 struct EpiExchangePromoted {
   static constexpr bool kTile = false, kPair = false, kF16 = true, kRegs = true;
   static constexpr int kPromoteKB = PKB;
   static constexpr int NH = TWO_N / 2;       // n
-  static constexpr int BW = NH / 2;          // rows of a block staged per pass
+  // rows of a block staged per pass: all of them where the operand ring leaves the room
+  static constexpr int RC = NH == 32 || NH == 64 ? 2 : 1;
+  static constexpr int BW = NH / RC;
   static constexpr int GMAX = 128 / NH;      // Cholesky blocks of a tile
-  static constexpr int LD = NH + 1;          // conflict-free column reads (LD odd)
-  static constexpr int kScratchBytes = GMAX * BW * LD * 4;
+  static constexpr int LD = NH + 2;          // 8-byte rows: conflict-free pair stores (LD / 2
+                                             // odd), columns read across consecutive lanes
+  static_assert(NH % 2 == 0 && (LD / 2) % 2 == 1, "staging rows");
+  static constexpr int kStage = GMAX * BW * LD;              // floats
+  static constexpr int kScratchBytes = kStage * 4 + 128;     // and red[2][4][2] doubles
+  static_assert(kStage % 2 == 0, "doubles after the staged rows");
   int n, Gn, Gw, nc, nw, nblk;
   z_t* Kpart;
   float ascale;
@@ -1340,7 +1349,7 @@ struct EpiExchangePromoted {
       return;   // not launched: the host requires whole walkers per warpgroup
     } else {
       constexpr int WPG = CPW / TWO_N;
-      __shared__ double red[2][2][4][2];
+      double (*red)[4][2] = reinterpret_cast<double (*)[4][2]>(scr + kStage);
       const int lane = row & 31, warp = row >> 5;
       const int ncv = min(Gn, nc - mt * Gn);
       const bool act = row < ncv * NH;
@@ -1356,12 +1365,12 @@ struct EpiExchangePromoted {
         for (int part = 0; part < 2; part++) {   // real, then imaginary rows
           const float* mine = part ? im : re;
 #pragma unroll
-          for (int rc = 0; rc < 2; rc++) {
+          for (int rc = 0; rc < RC; rc++) {
             const int b0 = rc * BW;
-            if (slot && a >= b0 && a < b0 + BW) {
-              float* dst = scr + (cv * BW + a - b0) * LD;
+            if (slot && (RC == 1 || (a >= b0 && a < b0 + BW))) {
+              float2* dst = reinterpret_cast<float2*>(scr + (cv * BW + a - b0) * LD);
 #pragma unroll
-              for (int c = 0; c < NH; c++) dst[c] = mine[c];
+              for (int c = 0; c < NH; c += 2) dst[c / 2] = make_float2(mine[c], mine[c + 1]);
             }
             tc::epi_bar_group(wg);
             if (act) {
@@ -1387,13 +1396,13 @@ struct EpiExchangePromoted {
           si += __shfl_xor_sync(0xffffffffu, si, o);
         }
         if (lane == 0) {
-          red[wg][q & 1][warp][0] = sr;
-          red[wg][q & 1][warp][1] = si;
+          red[q & 1][warp][0] = sr;
+          red[q & 1][warp][1] = si;
         }
         tc::epi_bar_group(wg);
         const int w = nt * Gw + wg * WPG + q;
         if (row == 0 && w < nw) {
-          const double (*r)[2] = red[wg][q & 1];
+          const double (*r)[2] = red[q & 1];
           const double u = 1.0 / ((double)ascale * (wscale ? (double)wscale[w] : 1.0));
           Kpart[((long long)w * 2 + s) * nblk + mt] =
               zmk((((r[0][0] + r[1][0]) + r[2][0]) + r[3][0]) * u * u,
@@ -2342,6 +2351,10 @@ static cudaError_t exchange_product(MixedState* m, int nsub, z_t* Kpart, int nbl
   // width is a multiple of 2n the tile's last BN - Gw 2n columns are not used
   tc::GemmShape g{m->nc * n, nsub * 2 * n, m->greal ? m->N : 2 * m->N, 2, m->ex_Gn * n,
                   m->ex_mtiles, true, true, 0, false, m->ex_Gw * 2 * n};
+  // groups of half the SMs' M tiles: the G operand (150 MB per spin at C4 with 1024 walkers)
+  // crosses HBM once per 74 M tiles instead of once per M tile (energy 46.6 -> 41.6 ms; the
+  // same time within 2% where G fits L2)
+  g.m_group = tc::sm_count() / 2;
   const int v = m->tune[2 * nsub > m->nw ? TS_EXF : TS_EXS];
   const int pk = promote ? promote_kb(PROMOTE_EXCHANGE) : 0;
   if ((v == 1 || (v == 0 && tc_persistent())) && pk && m->ex80) {

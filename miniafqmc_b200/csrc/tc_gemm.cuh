@@ -515,13 +515,22 @@ tc_gemm_multi_kernel(const __grid_constant__ MultiJob<Epi, NP> job, int* err) {
 struct TileSched {
   int m_tiles, n_tiles, nbatch, m_fast;
   int z0 = 0;   // first batch index of the launch (a walker group of a larger batch)
+  // > 1: M tiles in groups of this many, N tiles in order within a group, the group's M
+  // tiles fastest: about group x (SMs / group) tiles run together, so each operand tile is
+  // read from L2 by several CTAs and the B operand crosses HBM once per group
+  int group = 0;
   AFQ_HD int total() const { return m_tiles * n_tiles * nbatch; }
   AFQ_D void decode(int t, int& z, int& mt, int& nt) const {
     const int per = m_tiles * n_tiles;
     const int zl = t / per;   // batch within the launch
     const int r = t - zl * per;
     z = z0 + zl;
-    if (m_fast) {
+    if (group > 1) {
+      const int g = r / (group * n_tiles), rg = r - g * group * n_tiles;
+      const int gm = min(group, m_tiles - g * group);
+      nt = rg / gm;
+      mt = g * group + rg - nt * gm;
+    } else if (m_fast) {
       mt = r % m_tiles;
       nt = r / m_tiles;
     } else {
@@ -534,7 +543,15 @@ struct TileSched {
 template <int BN, int STAGES, int FMT, bool SPLIT, class Epi, int EPI_WG, int SLAB = 128>
 struct PCfg {
   using C = Cfg<BN, STAGES, FMT, SPLIT, SLAB>;
-  static constexpr int NEPI = 128 * EPI_WG, THREADS = NEPI + 64;
+  static constexpr int NEPI = 128 * EPI_WG;
+  // Promoting epilogues hold their accumulators in registers beside the staged trace.  Ten
+  // warps cap a thread at 168 registers (three warps share a scheduler's file), which spilled
+  // 53 to 119 of them, and the spills' local loads and stores set the epilogue's pace (ncu:
+  // 94 loads and 118 stores per warp and tile, local throttle and long-scoreboard stalls
+  // first).  With the two issuing warps in a third warpgroup the launch's 168 x 384 registers
+  // are split 232 for the epilogue threads, 40 for the others.
+  static constexpr bool REGSPLIT = EpiPromote<Epi>::value > 0 && EPI_WG == 2;
+  static constexpr int THREADS = REGSPLIT ? NEPI + 128 : NEPI + 64;
   static constexpr uint32_t ACC_COLS = 2 * C::TMEM_COLS;
   static constexpr size_t SCRATCH = (size_t)EpiScratch<Epi>::value * EPI_WG;
   static constexpr size_t BAR = 8 * (2 * STAGES + 5);
@@ -637,7 +654,7 @@ AFQ_D void fence_proxy_async_global() {
 
 template <int BN, int STAGES, int FMT, bool SPLIT, class Epi, int EPI_WG, int SLAB = 128,
           int NP = 1, bool CHAIN = false>
-__global__ void __launch_bounds__(128 * EPI_WG + 64, 1)
+__global__ void __launch_bounds__((PCfg<BN, STAGES, FMT, SPLIT, Epi, EPI_WG, SLAB>::THREADS), 1)
 tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
   using C = Cfg<BN, STAGES, FMT, SPLIT, SLAB>;
   using P = PCfg<BN, STAGES, FMT, SPLIT, Epi, EPI_WG, SLAB>;
@@ -709,253 +726,258 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
     return (klen + C::BK - 1) / C::BK;
   };
 
-  if (warp == WPROD && lane == 0) {
-    // ---- TMA producer
-    int g = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-      int p, z, mt, nt, kbase;
-      where(t, p, z, mt, nt);
-      const int nk = kslabs(p, z, kbase);
-      const int za = (job.a_batched[p] && !job.k_split[p]) ? z : 0;
-      const int zb = (job.b_batched[p] && !job.k_split[p]) ? z : 0;
-      const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
-      const Maps& maps = job.maps[p];
-      const bool sp = split_of(p);
-      const uint32_t part_bytes = C::A_BYTES + (uint32_t)job.bn[p] * SLAB;
-      if constexpr (CHAIN) {
-        if (p > 0) {   // every tile of problem p - 1 of batch z has published
-          const unsigned target = (unsigned)(p * job.dep_per);
-          const long long t0 = clock64();
-          while (ld_acquire_gpu(job.dep + z) < target) {
-            if (clock64() - t0 > g_tc_wait_clocks) {
-              ok = false;
-              break;
-            }
-          }
-          if (!ok) {
-            atomicOr(err, ERR_TIMEOUT_PRODUCER);
-            break;
-          }
-          fence_proxy_async_global();
-        }
-      }
-      const int nf = fills(nk, sp);
-      for (int f = 0; f < nf; f++, g++) {
-        const int s = g % STAGES;
-        if (!mbar_wait(&empty[s], ((g / STAGES) & 1) ^ 1)) {
-          atomicOr(err, ERR_TIMEOUT_PRODUCER);
-          ok = false;
-          break;
-        }
-        if (CHAIN && !sp) {   // plain chain tile: K slabs 2f and 2f + 1 in parts 0 and 1
-          const int kb = 2 * f, two = kb + 1 < nk;
-          mbar_expect_tx(&full[s], part_bytes * (two ? 2u : 1u));
-          tma_load_3d(stA(s, 0), &maps.a, &full[s], kbase + kb * C::BK, m0, za);
-          tma_load_3d(stB(s, 0), &maps.b, &full[s], kbase + kb * C::BK, n0, zb);
-          if (two) {
-            tma_load_3d(stA(s, 1), &maps.a, &full[s], kbase + (kb + 1) * C::BK, m0, za);
-            tma_load_3d(stB(s, 1), &maps.b, &full[s], kbase + (kb + 1) * C::BK, n0, zb);
-          }
-          continue;
-        }
-        const int kx = kbase + f * C::BK;
-        mbar_expect_tx(&full[s], C::PARTS * part_bytes);
-        tma_load_3d(stA(s, 0), &maps.a, &full[s], kx, m0, za);
-        tma_load_3d(stB(s, 0), &maps.b, &full[s], kx, n0, zb);
-        if (SPLIT) {
-          tma_load_3d(stA(s, 1), &maps.a_lo, &full[s], kx, m0, za);
-          tma_load_3d(stB(s, 1), &maps.b_lo, &full[s], kx, n0, zb);
-        }
-      }
-    }
-    // the last fills of each stage land before the CTA can exit
-    for (int q = max(0, g - STAGES); q < g; q++)
-      mbar_wait_drain(&full[q % STAGES], (q / STAGES) & 1);
-  } else if (warp == WMMA && lane == 0) {
-    // ---- MMA issuer: one accumulator buffer per tile, or per K chunk when promoting
-    int g = 0, li = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-      int p, z, mt, nt, kbase;
-      where(t, p, z, mt, nt);
-      const int nk = kslabs(p, z, kbase);
-      const uint32_t ID = idesc(128, job.bn[p], FMT);
-      const int nch = PK ? (nk + PK - 1) / PK : 1;
-      const bool sp = split_of(p);
-      if (CHAIN && !sp) {   // plain chain tile: two K slabs per stage, one accumulator
-        const int b = li & 1;
-        if (!mbar_wait(&acce[b], ((li >> 1) & 1) ^ 1)) {
-          atomicOr(err, ERR_TIMEOUT_MMA);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d = tmem + b * C::TMEM_COLS;
-        const int nf = fills(nk, sp);
-        for (int f = 0; f < nf; f++, g++) {
-          const int s = g % STAGES;
-          if (!mbar_wait(&full[s], (g / STAGES) & 1)) {
-            atomicOr(err, ERR_TIMEOUT_MMA);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const int nparts = 2 * f + 1 < nk ? 2 : 1;
-          for (int part = 0; part < nparts; part++) {
-            const uint64_t ad = sdesc_k<SLAB>(smem_u32(stA(s, part)));
-            const uint64_t bd = sdesc_k<SLAB>(smem_u32(stB(s, part)));
-#pragma unroll
-            for (int k = 0; k < C::BK / C::UK; k++)
-              umma<FMT>(d, ad + 2 * k, bd + 2 * k, ID, (f != 0 || part != 0 || k != 0) ? 1u : 0u);
-          }
-          umma_commit(&empty[s]);
-        }
-        if (!ok) break;
-        umma_commit(&accf[b]);
-        li++;
-        continue;
-      }
-      for (int ch = 0; ch < nch && ok; ch++, li++) {
-        const int b = li & 1;
-        if (!mbar_wait(&acce[b], ((li >> 1) & 1) ^ 1)) {   // the epilogue released buffer b
-          atomicOr(err, ERR_TIMEOUT_MMA);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d = tmem + b * C::TMEM_COLS;
-        const int kb0 = PK ? ch * PK : 0, kb1 = PK ? min(nk, kb0 + PK) : nk;
-        for (int kb = kb0; kb < kb1; kb++, g++) {
-          const int s = g % STAGES;
-          if (!mbar_wait(&full[s], (g / STAGES) & 1)) {
-            atomicOr(err, ERR_TIMEOUT_MMA);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t ad = sdesc_k<SLAB>(smem_u32(stA(s, 0)));
-          const uint64_t bd = sdesc_k<SLAB>(smem_u32(stB(s, 0)));
-#pragma unroll
-          for (int k = 0; k < C::BK / C::UK; k++)
-            umma<FMT>(d, ad + 2 * k, bd + 2 * k, ID, (kb != kb0 || k != 0) ? 1u : 0u);
-          if (SPLIT) {
-            const uint64_t al = sdesc_k<SLAB>(smem_u32(stA(s, 1)));
-            const uint64_t bl = sdesc_k<SLAB>(smem_u32(stB(s, 1)));
-#pragma unroll
-            for (int k = 0; k < C::BK / C::UK; k++) {
-              umma<FMT>(d, ad + 2 * k, bl + 2 * k, ID, 1u);
-              umma<FMT>(d, al + 2 * k, bd + 2 * k, ID, 1u);
-            }
-          }
-          umma_commit(&empty[s]);
-        }
-        if (!ok) break;
-        umma_commit(&accf[b]);
-      }
-    }
-    umma_commit(fin);   // fires once every MMA issued above has completed
-    mbar_wait_drain(fin, 0);
-  }
-
-  if constexpr (PK > 0) {
-    if (warp < WPROD) {
-      // ---- promoting epilogue: warpgroup wg sums its columns over the K chunks
-      constexpr int CPW = BN / EPI_WG;
-      static_assert(CPW % 32 == 0, "promotion: whole 32-column chunks per warpgroup");
-      const int wg = warp >> 2, wq = warp & 3;
-      const int row = wq * 32 + lane;
-      float* scr = scratch + (size_t)wg * (EpiScratch<Epi>::value / 4);
-      float acc[CPW];
-      int li = 0;
+  if (warp >= WPROD) {
+    if constexpr (P::REGSPLIT)   // 168 x 384 registers at launch = 232 x 256 + 40 x 128
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == WPROD && lane == 0) {
+      // ---- TMA producer
+      int g = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
         int p, z, mt, nt, kbase;
-        job.locate(t, p, z, mt, nt);
+        where(t, p, z, mt, nt);
         const int nk = kslabs(p, z, kbase);
-        const int nch = (nk + PK - 1) / PK;
-        EpiHold epi = job.epi[p];
-        for (int ch = 0; ch < nch; ch++, li++) {
+        const int za = (job.a_batched[p] && !job.k_split[p]) ? z : 0;
+        const int zb = (job.b_batched[p] && !job.k_split[p]) ? z : 0;
+        const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
+        const Maps& maps = job.maps[p];
+        const bool sp = split_of(p);
+        const uint32_t part_bytes = C::A_BYTES + (uint32_t)job.bn[p] * SLAB;
+        if constexpr (CHAIN) {
+          if (p > 0) {   // every tile of problem p - 1 of batch z has published
+            const unsigned target = (unsigned)(p * job.dep_per);
+            const long long t0 = clock64();
+            while (ld_acquire_gpu(job.dep + z) < target) {
+              if (clock64() - t0 > g_tc_wait_clocks) {
+                ok = false;
+                break;
+              }
+            }
+            if (!ok) {
+              atomicOr(err, ERR_TIMEOUT_PRODUCER);
+              break;
+            }
+            fence_proxy_async_global();
+          }
+        }
+        const int nf = fills(nk, sp);
+        for (int f = 0; f < nf; f++, g++) {
+          const int s = g % STAGES;
+          if (!mbar_wait(&empty[s], ((g / STAGES) & 1) ^ 1)) {
+            atomicOr(err, ERR_TIMEOUT_PRODUCER);
+            ok = false;
+            break;
+          }
+          if (CHAIN && !sp) {   // plain chain tile: K slabs 2f and 2f + 1 in parts 0 and 1
+            const int kb = 2 * f, two = kb + 1 < nk;
+            mbar_expect_tx(&full[s], part_bytes * (two ? 2u : 1u));
+            tma_load_3d(stA(s, 0), &maps.a, &full[s], kbase + kb * C::BK, m0, za);
+            tma_load_3d(stB(s, 0), &maps.b, &full[s], kbase + kb * C::BK, n0, zb);
+            if (two) {
+              tma_load_3d(stA(s, 1), &maps.a, &full[s], kbase + (kb + 1) * C::BK, m0, za);
+              tma_load_3d(stB(s, 1), &maps.b, &full[s], kbase + (kb + 1) * C::BK, n0, zb);
+            }
+            continue;
+          }
+          const int kx = kbase + f * C::BK;
+          mbar_expect_tx(&full[s], C::PARTS * part_bytes);
+          tma_load_3d(stA(s, 0), &maps.a, &full[s], kx, m0, za);
+          tma_load_3d(stB(s, 0), &maps.b, &full[s], kx, n0, zb);
+          if (SPLIT) {
+            tma_load_3d(stA(s, 1), &maps.a_lo, &full[s], kx, m0, za);
+            tma_load_3d(stB(s, 1), &maps.b_lo, &full[s], kx, n0, zb);
+          }
+        }
+      }
+      // the last fills of each stage land before the CTA can exit
+      for (int q = max(0, g - STAGES); q < g; q++)
+        mbar_wait_drain(&full[q % STAGES], (q / STAGES) & 1);
+    } else if (warp == WMMA && lane == 0) {
+      // ---- MMA issuer: one accumulator buffer per tile, or per K chunk when promoting
+      int g = 0, li = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        int p, z, mt, nt, kbase;
+        where(t, p, z, mt, nt);
+        const int nk = kslabs(p, z, kbase);
+        const uint32_t ID = idesc(128, job.bn[p], FMT);
+        const int nch = PK ? (nk + PK - 1) / PK : 1;
+        const bool sp = split_of(p);
+        if (CHAIN && !sp) {   // plain chain tile: two K slabs per stage, one accumulator
           const int b = li & 1;
-          if (!mbar_wait(&accf[b], (li >> 1) & 1)) {
-            if (lane == 0) atomicOr(err, ERR_TIMEOUT_EPILOGUE);
+          if (!mbar_wait(&acce[b], ((li >> 1) & 1) ^ 1)) {
+            atomicOr(err, ERR_TIMEOUT_MMA);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t trow =
-              tmem + b * C::TMEM_COLS + ((uint32_t)(wq * 32) << 16) + (uint32_t)(wg * CPW);
-          if (ch == 0) {
-#pragma unroll
-            for (int j = 0; j < CPW / 32; j++) tmem_ld32(trow + j * 32, acc + j * 32);
-          } else {
-#pragma unroll
-            for (int j = 0; j < CPW / 32; j++) tmem_ld32_add(trow + j * 32, acc + j * 32);
+          const uint32_t d = tmem + b * C::TMEM_COLS;
+          const int nf = fills(nk, sp);
+          for (int f = 0; f < nf; f++, g++) {
+            const int s = g % STAGES;
+            if (!mbar_wait(&full[s], (g / STAGES) & 1)) {
+              atomicOr(err, ERR_TIMEOUT_MMA);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const int nparts = 2 * f + 1 < nk ? 2 : 1;
+            for (int part = 0; part < nparts; part++) {
+              const uint64_t ad = sdesc_k<SLAB>(smem_u32(stA(s, part)));
+              const uint64_t bd = sdesc_k<SLAB>(smem_u32(stB(s, part)));
+  #pragma unroll
+              for (int k = 0; k < C::BK / C::UK; k++)
+                umma<FMT>(d, ad + 2 * k, bd + 2 * k, ID, (f != 0 || part != 0 || k != 0) ? 1u : 0u);
+            }
+            umma_commit(&empty[s]);
           }
-          tc_fence_before();
-          mbar_arrive(&acce[b]);
+          if (!ok) break;
+          umma_commit(&accf[b]);
+          li++;
+          continue;
         }
-        if (!ok) break;
-        if constexpr (EpiRegs<Epi>::value) {
-          epi.regs(z, mt, nt, row, acc, scr, wg);
-        } else {
-          const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
-#pragma unroll
-          for (int j = 0; j < CPW / 32; j++) epi(z, row, m0 + row, n0 + wg * CPW + j * 32, acc + j * 32);
+        for (int ch = 0; ch < nch && ok; ch++, li++) {
+          const int b = li & 1;
+          if (!mbar_wait(&acce[b], ((li >> 1) & 1) ^ 1)) {   // the epilogue released buffer b
+            atomicOr(err, ERR_TIMEOUT_MMA);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d = tmem + b * C::TMEM_COLS;
+          const int kb0 = PK ? ch * PK : 0, kb1 = PK ? min(nk, kb0 + PK) : nk;
+          for (int kb = kb0; kb < kb1; kb++, g++) {
+            const int s = g % STAGES;
+            if (!mbar_wait(&full[s], (g / STAGES) & 1)) {
+              atomicOr(err, ERR_TIMEOUT_MMA);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t ad = sdesc_k<SLAB>(smem_u32(stA(s, 0)));
+            const uint64_t bd = sdesc_k<SLAB>(smem_u32(stB(s, 0)));
+  #pragma unroll
+            for (int k = 0; k < C::BK / C::UK; k++)
+              umma<FMT>(d, ad + 2 * k, bd + 2 * k, ID, (kb != kb0 || k != 0) ? 1u : 0u);
+            if (SPLIT) {
+              const uint64_t al = sdesc_k<SLAB>(smem_u32(stA(s, 1)));
+              const uint64_t bl = sdesc_k<SLAB>(smem_u32(stB(s, 1)));
+  #pragma unroll
+              for (int k = 0; k < C::BK / C::UK; k++) {
+                umma<FMT>(d, ad + 2 * k, bl + 2 * k, ID, 1u);
+                umma<FMT>(d, al + 2 * k, bd + 2 * k, ID, 1u);
+              }
+            }
+            umma_commit(&empty[s]);
+          }
+          if (!ok) break;
+          umma_commit(&accf[b]);
         }
       }
+      umma_commit(fin);   // fires once every MMA issued above has completed
+      mbar_wait_drain(fin, 0);
     }
-  } else if (warp < WPROD) {
-    // ---- epilogue: warpgroup wg takes chunks wg, wg + EPI_WG, ...; TMEM lane = tile row
-    const int wg = warp >> 2, wq = warp & 3;
-    const int row = wq * 32 + lane;
-    int li = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x, li++) {
-      int p, z, mt, nt;
-      where(t, p, z, mt, nt);
-      EpiHold epi = job.epi[p];
-      const int bn = job.bn[p];
-      const int b = li & 1;
-      bool got = mbar_wait(&accf[b], (li >> 1) & 1);
-      // chain launches publish per warp: the warp decides as one whether to go on
-      if constexpr (CHAIN) got = __all_sync(0xffffffffu, got);
-      if (!got) {
-        if (lane == 0) atomicOr(err, ERR_TIMEOUT_EPILOGUE);
-        break;
-      }
-      tc_fence_after();
-      if constexpr (CHAIN) {   // see what problem p - 1 published before reading its output
-        if (p > 0) (void)ld_acquire_gpu(job.dep + z);
-      }
-      const uint32_t trow = tmem + b * C::TMEM_COLS + ((uint32_t)(wq * 32) << 16);
-      const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
-      float v[32];
-      if constexpr (Epi::kPair) {
-        const int Pw = epi.pair_stride();
-        float u[32];
-#pragma unroll 1
-        for (int c0 = wg * 32; c0 < Pw && c0 + Pw < bn + 1; c0 += 32 * EPI_WG) {
-          tmem_ld32(trow + c0, v);
-          tmem_ld32(trow + c0 + Pw, u);
-          epi.pair(z, row, m0 + row, c0, v, u);
-        }
-      } else if constexpr (EpiStaged<Epi>::value) {
+  } else {
+    if constexpr (P::REGSPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    if constexpr (PK > 0) {
+      {
+        // ---- promoting epilogue: warpgroup wg sums its columns over the K chunks
+        constexpr int CPW = BN / EPI_WG;
+        static_assert(CPW % 32 == 0, "promotion: whole 32-column chunks per warpgroup");
+        const int wg = warp >> 2, wq = warp & 3;
+        const int row = wq * 32 + lane;
         float* scr = scratch + (size_t)wg * (EpiScratch<Epi>::value / 4);
-        auto ld = [&](int col, float* out) { tmem_ld32(trow + col, out); };
-        epi.staged(z, mt, nt, row, ld, scr, wg);
-      } else {
-#pragma unroll 1
-        for (int c0 = wg * 32; c0 < bn; c0 += 32 * EPI_WG) {
-          tmem_ld32(trow + c0, v);
-          epi(z, row, m0 + row, n0 + c0, v);
+        float acc[CPW];
+        int li = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+          int p, z, mt, nt, kbase;
+          job.locate(t, p, z, mt, nt);
+          const int nk = kslabs(p, z, kbase);
+          const int nch = (nk + PK - 1) / PK;
+          EpiHold epi = job.epi[p];
+          for (int ch = 0; ch < nch; ch++, li++) {
+            const int b = li & 1;
+            if (!mbar_wait(&accf[b], (li >> 1) & 1)) {
+              if (lane == 0) atomicOr(err, ERR_TIMEOUT_EPILOGUE);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t trow =
+                tmem + b * C::TMEM_COLS + ((uint32_t)(wq * 32) << 16) + (uint32_t)(wg * CPW);
+            if (ch == 0) {
+  #pragma unroll
+              for (int j = 0; j < CPW / 32; j++) tmem_ld32(trow + j * 32, acc + j * 32);
+            } else {
+  #pragma unroll
+              for (int j = 0; j < CPW / 32; j++) tmem_ld32_add(trow + j * 32, acc + j * 32);
+            }
+            tc_fence_before();
+            mbar_arrive(&acce[b]);
+          }
+          if (!ok) break;
+          if constexpr (EpiRegs<Epi>::value) {
+            epi.regs(z, mt, nt, row, acc, scr, wg);
+          } else {
+            const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
+  #pragma unroll
+            for (int j = 0; j < CPW / 32; j++) epi(z, row, m0 + row, n0 + wg * CPW + j * 32, acc + j * 32);
+          }
         }
       }
-      tc_fence_before();
-      mbar_arrive(&acce[b]);
-      if constexpr (CHAIN) {   // publish: this warp's writes of the tile are done
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) red_release_gpu_add(job.dep + z, 1u);
+    } else {
+      // ---- epilogue: warpgroup wg takes chunks wg, wg + EPI_WG, ...; TMEM lane = tile row
+      const int wg = warp >> 2, wq = warp & 3;
+      const int row = wq * 32 + lane;
+      int li = 0;
+      for (int t = blockIdx.x; t < total; t += gridDim.x, li++) {
+        int p, z, mt, nt;
+        where(t, p, z, mt, nt);
+        EpiHold epi = job.epi[p];
+        const int bn = job.bn[p];
+        const int b = li & 1;
+        bool got = mbar_wait(&accf[b], (li >> 1) & 1);
+        // chain launches publish per warp: the warp decides as one whether to go on
+        if constexpr (CHAIN) got = __all_sync(0xffffffffu, got);
+        if (!got) {
+          if (lane == 0) atomicOr(err, ERR_TIMEOUT_EPILOGUE);
+          break;
+        }
+        tc_fence_after();
+        if constexpr (CHAIN) {   // see what problem p - 1 published before reading its output
+          if (p > 0) (void)ld_acquire_gpu(job.dep + z);
+        }
+        const uint32_t trow = tmem + b * C::TMEM_COLS + ((uint32_t)(wq * 32) << 16);
+        const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
+        float v[32];
+        if constexpr (Epi::kPair) {
+          const int Pw = epi.pair_stride();
+          float u[32];
+  #pragma unroll 1
+          for (int c0 = wg * 32; c0 < Pw && c0 + Pw < bn + 1; c0 += 32 * EPI_WG) {
+            tmem_ld32(trow + c0, v);
+            tmem_ld32(trow + c0 + Pw, u);
+            epi.pair(z, row, m0 + row, c0, v, u);
+          }
+        } else if constexpr (EpiStaged<Epi>::value) {
+          float* scr = scratch + (size_t)wg * (EpiScratch<Epi>::value / 4);
+          auto ld = [&](int col, float* out) { tmem_ld32(trow + col, out); };
+          epi.staged(z, mt, nt, row, ld, scr, wg);
+        } else {
+  #pragma unroll 1
+          for (int c0 = wg * 32; c0 < bn; c0 += 32 * EPI_WG) {
+            tmem_ld32(trow + c0, v);
+            epi(z, row, m0 + row, n0 + c0, v);
+          }
+        }
+        tc_fence_before();
+        mbar_arrive(&acce[b]);
+        if constexpr (CHAIN) {   // publish: this warp's writes of the tile are done
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) red_release_gpu_add(job.dep + z, 1u);
+        }
       }
     }
   }
@@ -1002,6 +1024,7 @@ struct GemmShape {
                        // tile hold whole column groups that do not fill BN
   int z0 = 0;          // first batch of the launch: batches z0 .. z0 + batch - 1 of operands
                        // (and epilogue outputs) that hold more (no split-K)
+  int m_group = 0;     // persistent kernel: TileSched::group
 };
 
 template <int BN, int STAGES, int FMT, bool SPLIT, class Epi, int MINB = 1, int SLAB = 128>
@@ -1087,7 +1110,7 @@ cudaError_t launch_persistent(const Maps& maps, const GemmShape& g, const Epi& e
   PJob<Epi, 1> job;
   job.maps[0] = maps;
   job.epi[0] = epi;
-  job.sched[0] = TileSched{g.m_tiles, (g.N + ns - 1) / ns, g.batch, g.m_fast ? 1 : 0, g.z0};
+  job.sched[0] = TileSched{g.m_tiles, (g.N + ns - 1) / ns, g.batch, g.m_fast ? 1 : 0, g.z0, g.m_group};
   job.K[0] = g.K;
   job.m_step[0] = g.m_step;
   job.n_step[0] = ns;
