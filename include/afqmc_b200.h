@@ -319,8 +319,9 @@ afq_status afq_copy_out(afq_handle* h, int which, void* host);
  * Lh, Gc and ek must be 16-byte aligned (the kernels move whole complex values);
  * other pointers are rejected with AFQ_ERR_ARG before any device work.
  * Asynchronous on `stream` (a cudaStream_t, NULL for the default stream).  The partial
- * sums live in one file-scope device array of 2^18 complex values (4 MiB, held by every
- * GPU that loads the library until exit): calls with 2 * nwalk * ceil(nchol / (96 /
+ * sums live in one file-scope device array of 2^18 complex values, operand digits and a
+ * chunk of the products in a second one (4 and 79 MiB, held from the first call on a GPU
+ * until exit): calls with 2 * nwalk * ceil(nchol / (96 /
  * naea)) above that, or with ceil(nwalk / (96 / naea)) above 65535, are rejected with
  * AFQ_ERR_UNSUPPORTED (split the walkers into batches); naea must be <= 96.  The first
  * call on a device looks up the array's device address (cudaGetSymbolAddress) with that

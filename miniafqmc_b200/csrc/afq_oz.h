@@ -2,6 +2,7 @@
 // are written as signed 8-bit digits.  Results agree with an FP64 product to FP64 rounding
 // (the digits keep 55 bits below each row's power of two).
 #pragma once
+#include <stdint.h>
 #include "afq_common.cuh"
 
 namespace afq {
@@ -42,6 +43,22 @@ int oz_exchange_launches(const OzState* o, int nwalk);
 // nblk = nchol.
 cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nblk,
                         cudaStream_t st);
+// Exchange energies of caller-owned device buffers through a fixed scratch (no allocation, no
+// synchronisation): ek[nwalk].  Whether Lh is real is found on the device.
+struct OzBuffers {
+  int8_t *a, *g;              // digits of a chunk of Lh rows and of G rows
+  size_t a_bytes, g_bytes;
+  double *a_scale, *g_scale;  // a_rows, g_rows row scales
+  int a_rows, g_rows;
+  double* T;
+  size_t t_bytes;
+  z_t* part;                  // partial sums
+  long long parts;
+  int* flags;                 // timeout flags, Lh complex
+};
+bool oz_exchange_buffers_fit(const OzBuffers& b, int N, int n, int nc, int nw);
+cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc, int N, int n,
+                                int nc, int nw, z_t* ek, cudaStream_t st);
 // Timeout flags raised by the kernels (0 when clean), and the bound of their waits.
 cudaError_t oz_error(OzState* o, int* flags);
 cudaError_t oz_set_wait_clocks(long long clocks);

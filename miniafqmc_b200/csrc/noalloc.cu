@@ -4,13 +4,14 @@
 // under stream capture (an allocation there breaks the capture), and host frameworks
 // that hand every byte of device memory to their own pool and forbid allocations after
 // start-up.  This entry point serves them: the caller passes device inputs and outputs,
-// and the partial sums the exchange kernel needs live in a fixed file-scope device
-// array instead of a per-handle buffer.
+// and what the exchange needs besides (partial sums, operand digits, a chunk of the products)
+// lives in fixed file-scope device arrays instead of per-handle buffers.
 #include <cstdint>
 #include <mutex>
 
 #include "../../include/afqmc_b200.h"
 #include "afq_kernels.h"
+#include "afq_oz.h"
 
 namespace {
 
@@ -19,9 +20,24 @@ namespace {
 constexpr long long kMaxExchangePartials = 1LL << 18;
 static __device__ __align__(256) z_t g_exchange_scratch[kMaxExchangePartials];
 
+// Chunks of the digit products (oz.cu): 48 MiB of T (five waves of 64 KB output tiles), 24
+// MiB of G digits and 6 MiB of Lh digits with their row scales, loaded with this file's
+// kernels by the first call on a device.  With 40 and 20 MiB, 96 walkers at 200 orbitals
+// split into two uneven chunks: 10.8 against 7.0 ms (28.0 ms on the FP64 pipe).
+constexpr size_t kTBytes = 48u << 20, kGBytes = 24u << 20, kABytes = 6u << 20;
+constexpr int kGRows = 16384, kARows = 4096;
+struct Scratch {
+  double T[kTBytes / 8];
+  int8_t g[kGBytes], a[kABytes];
+  double g_scale[kGRows], a_scale[kARows];
+  int flags[8];
+};
+static __device__ __align__(256) Scratch g_oz_scratch;
+
 constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mu;
 z_t* g_scratch_addr[kMaxDevices] = {};
+Scratch* g_oz_addr[kMaxDevices] = {};
 
 // EK[w] = 1/2 sum over spins and Cholesky blocks of the partials, in a fixed order.
 __global__ void __launch_bounds__(128)
@@ -58,6 +74,7 @@ extern "C" afq_status afq_exchange_energy_noalloc(const double* Lh, const double
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return AFQ_ERR_CUDA;
   z_t* scratch = nullptr;
+  Scratch* oz = nullptr;
   {
     // set-up, once per device with that device current: the host-side symbol is only a
     // stand-in, the kernels need the device address of the array
@@ -65,11 +82,23 @@ extern "C" afq_status afq_exchange_energy_noalloc(const double* Lh, const double
     if (!g_scratch_addr[dev]) {
       void* p = nullptr;
       if (cudaGetSymbolAddress(&p, g_exchange_scratch) != cudaSuccess || !p) return AFQ_ERR_CUDA;
+      void* q = nullptr;
+      if (cudaGetSymbolAddress(&q, g_oz_scratch) != cudaSuccess || !q) return AFQ_ERR_CUDA;
+      g_oz_addr[dev] = static_cast<Scratch*>(q);
       g_scratch_addr[dev] = static_cast<z_t*>(p);
     }
     scratch = g_scratch_addr[dev];
+    oz = g_oz_addr[dev];
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const afq::OzBuffers b{oz->a, oz->g, kABytes, kGBytes, oz->a_scale, oz->g_scale, kARows, kGRows,
+                         oz->T, kTBytes, scratch, kMaxExchangePartials, oz->flags};
+  if (afq::oz_exchange_buffers_fit(b, nmo, naea, nchol, nwalk))
+    return afq::oz_exchange_buffers(b, reinterpret_cast<const z_t*>(Lh),
+                                    reinterpret_cast<const z_t*>(Gc), nmo, naea, nchol, nwalk,
+                                    reinterpret_cast<z_t*>(ek), st) == cudaSuccess
+               ? AFQ_OK
+               : AFQ_ERR_CUDA;
   // the array keeps the previous call's contents: clear the part this call reads
   if (cudaMemsetAsync(scratch, 0, sizeof(z_t) * used, st) != cudaSuccess) return AFQ_ERR_CUDA;
   int nb = 0;

@@ -295,6 +295,31 @@ cudaError_t slice_rows(const RowSrc& src, int nrows, int K, const Slices& s, cud
   return cudaGetLastError();
 }
 
+// Rows of an A operand (TWO = false: one row of reals, or of pairs) or of a B operand (re and
+// im rows, or pair rows) as found on the device: *cplx == 0 means a real A operand.  `s`
+// describes the complex form; the real one has nslab_real slabs in the same buffers.
+template <bool TWO>
+__global__ void __launch_bounds__(256)
+slice_found_kernel(RowSrc src, int nrows, int K, Slices s, const int* __restrict__ cplx,
+                   int nslab_real) {
+  const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= nrows) return;
+  const z_t* p = src.row(r);
+  const bool cx = *cplx != 0;
+  if (!cx) s.nslab = nslab_real;
+  unsigned long long m0, m1;
+  row_max<kPairs>(p, 0, K, lane, 32, m0, m1);
+  if (cx) m0 = m1 = max(m0, m1);
+  const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
+  constexpr int REAL = TWO ? kSplitRe : kReal, CPLX = TWO ? kSplitCx : kPairs;
+  const int r0 = TWO ? 2 * r : r, Kp = s.nslab * oz::kSlab;
+  if (lane == 0) put_scales<REAL>(s, 0, r0, s0, s1);
+  if (cx)
+    slice_row<CPLX>(p, K, s, 0, r0, s0, s1, 0, Kp, lane, 32);
+  else
+    slice_row<REAL>(p, K, s, 0, r0, s0, s1, 0, Kp, lane, 32);
+}
+
 // X [nchol][nw] -> rows (w, re | im): a cluster of 8 CTAs per 32 walkers, lanes on walkers
 // (coalesced reads of X's rows), 16 digits per thread and store.
 template <bool REALA>
@@ -686,7 +711,121 @@ cudaError_t create_propagate(OzState* o, cudaStream_t st) {
   return e;
 }
 
+// The trace kernel's shared memory for n x n blocks.
+cudaError_t trace_attr(int n, size_t* smem) {
+  *smem = sizeof(z_t) * n * (n + 1);
+  static DeviceAttr attr;
+  return attr.ensure(*smem, [](size_t b) {
+    cudaError_t r = cudaFuncSetAttribute(trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)b);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(trace_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
+    return r;
+  });
+}
+
+// ek[w] = 1/2 sum of the walker's partial sums in a fixed order (NaN when a kernel timed out).
+__global__ void __launch_bounds__(128)
+ek_sum_kernel(const z_t* __restrict__ part, int count, const int* __restrict__ err,
+              z_t* __restrict__ ek) {
+  __shared__ z_t red[4];
+  const int w = blockIdx.x;
+  z_t s = zmk(0, 0);
+  for (int q = threadIdx.x; q < count; q += 128) s = zadd(s, part[(long long)w * count + q]);
+  s = block_zsum(s, red);
+  const double bad = __longlong_as_double(0x7ff8000000000000LL);
+  if (threadIdx.x == 0) ek[w] = *err ? zmk(bad, bad) : zscale(s, 0.5);
+}
+
+// Chunks of oz_exchange_buffers: w walkers and c Cholesky vectors at a time; false when even
+// one walker and one vector exceed the scratch.
+bool buffers_plan(const OzBuffers& b, int N, int n, int nc, int nw, int* w, int* c) {
+  const long long Kp = (2LL * N + oz::kSlab - 1) / oz::kSlab * oz::kSlab;
+  if (2 * N > oz::kMaxK || n > 96) return false;
+  const long long grows = std::min<long long>(b.g_bytes / (kS * Kp), b.g_rows) / oz::kBN * oz::kBN;
+  const long long arows = std::min<long long>(b.a_bytes / (kS * Kp), b.a_rows) / oz::kBM * oz::kBM;
+  long long cw = std::min<long long>(nw, grows / (2 * n));
+  cw = std::min<long long>(cw, b.parts / (2LL * nc));
+  if (cw < 1 || arows < n) return false;
+  cw = (nw + (nw + cw - 1) / cw - 1) / ((nw + cw - 1) / cw);   // chunks of even size
+  // Cholesky vectors: as many row tiles as T and A hold, of these the count whose tiles fill
+  // the last wave of SMs best
+  const long long ld = (2 * cw * n + 3) / 4 * 4, nt = (2 * cw * n + oz::kBN - 1) / oz::kBN;
+  const long long most = std::min<long long>(arows, b.t_bytes / (8 * ld)) / oz::kBM;
+  long long best = 0;
+  double eff = -1.0;
+  for (long long m = 1; m <= most; m++) {
+    const long long t = m * nt, sms = tc::sm_count();
+    const double f = (double)t / (double)((t + sms - 1) / sms * sms + sms / 4);
+    if (f > eff) {
+      eff = f;
+      best = m;
+    }
+  }
+  const long long cc = best * oz::kBM / n;
+  if (cc < 1) return false;
+  *w = (int)cw;
+  *c = (int)std::min<long long>(cc, nc);
+  return true;
+}
+
 }  // namespace
+
+// From 8e8 real operations (about 60 us of the FP64 pipe's exchange kernel, which runs at 14
+// TFLOP/s) the digit products' launches pay.
+bool oz_exchange_buffers_fit(const OzBuffers& b, int N, int n, int nc, int nw) {
+  int w, c;
+  return 16.0 * nc * n * (double)n * N * nw >= 8e8 && buffers_plan(b, N, n, nc, nw, &w, &c);
+}
+
+cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc, int N, int n,
+                                int nc, int nw, z_t* ek, cudaStream_t st) {
+  int cw = 0, cc = 0;
+  if (!buffers_plan(b, N, n, nc, nw, &cw, &cc)) return cudaErrorInvalidValue;
+  const long long NAK = 2LL * n * N;
+  size_t smem = 0;
+  cudaError_t e = trace_attr(n, &smem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.flags, 0, 2 * sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  int *err = b.flags, *cplx = b.flags + 1;
+  oz_check_imag_kernel<<<148 * 8, 256, 0, st>>>(Lh, nc * NAK, cplx);
+  Slices a, g;
+  a.d = b.a;
+  a.scale = b.a_scale;
+  a.tile = oz::kBM;
+  a.batch = 1;
+  g = a;
+  g.d = b.g;
+  g.scale = b.g_scale;
+  g.tile = oz::kBN;
+  a.nslab = g.nslab = (2 * N + oz::kSlab - 1) / oz::kSlab;
+  const int nslab_real = (N + oz::kSlab - 1) / oz::kSlab;
+  for (int w0 = 0; w0 < nw; w0 += cw) {
+    const int w = std::min(cw, nw - w0);
+    g.rows = 2 * w * n;
+    const long long ld = (2LL * w * n + 3) / 4 * 4;
+    for (int s = 0; s < 2; s++) {
+      const RowSrc gs{Gc + w0 * NAK + (long long)s * n * N, n, NAK, N};
+      slice_found_kernel<true><<<(w * n + 7) / 8, 256, 0, st>>>(gs, w * n, N, g, cplx, nslab_real);
+      for (int c0 = 0; c0 < nc; c0 += cc) {
+        const int c = std::min(cc, nc - c0);
+        a.rows = c * n;
+        const RowSrc as{Lh + c0 * NAK + (long long)s * n * N, n, NAK, N};
+        slice_found_kernel<false><<<(c * n + 7) / 8, 256, 0, st>>>(as, c * n, N, a, cplx,
+                                                                  nslab_real);
+        oz::Gemm gm{&a, &g, c * n, 2 * w * n, 1};
+        gm.cplx = cplx;
+        gm.nslab_real = nslab_real;
+        if ((e = oz::launch<7>(gm, EpiRows{b.T, ld, c * n}, err, st)) != cudaSuccess) return e;
+        trace_kernel<<<dim3(c, w), kTraceThreads, smem, st>>>(
+            reinterpret_cast<const z_t*>(b.T), n, ld / 2, 0, c0, b.part, nc, 0, s);
+      }
+    }
+    ek_sum_kernel<<<w, 128, 0, st>>>(b.part, 2 * nc, err, ek + w0);
+  }
+  return cudaGetLastError();
+}
 
 cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
   *out = nullptr;
@@ -804,16 +943,8 @@ cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nb
                         cudaStream_t st) {
   const int N = o->in.N, n = o->in.n, nc = o->in.nchol;
   const long long NAK = 2LL * n * N;
-  const size_t smem = sizeof(z_t) * n * (n + 1);
-  static DeviceAttr attr;
-  cudaError_t e = attr.ensure(smem, [](size_t b) {
-    cudaError_t r = cudaFuncSetAttribute(trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)b);
-    if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(trace_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared);
-    return r;
-  });
+  size_t smem = 0;
+  cudaError_t e = trace_attr(n, &smem);
   for (int s = 0; s < 2 && e == cudaSuccess; s++) {
     const RowSrc src{Gc + (long long)s * n * N, n, NAK, N};
     e = o->lreal ? slice_rows<kSplitRe>(src, nwalk * n, N, o->gx, st)

@@ -82,6 +82,8 @@ struct Job {
   int M, N;                         // output rows and columns per batch
   int m_tile, n_tile;               // first row tile of A and of B of the launch
   int nslab, slab_split;            // K slabs, and slabs per z when split along K (else 0)
+  const int* cplx;                  // non-null: *cplx == 0 (real A operand, found on the
+  int nslab_real;                   // device) means nslab_real slabs instead
 };
 
 AFQ_D void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -236,9 +238,10 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const int total = job.sched.total();
+  const int nslab = job.cplx && *job.cplx == 0 ? job.nslab_real : job.nslab;
   auto slabs = [&](int z, int& s0) {
     s0 = job.slab_split ? z * job.slab_split : 0;
-    return job.slab_split ? min(job.slab_split, job.nslab - s0) : job.nslab;
+    return job.slab_split ? min(job.slab_split, nslab - s0) : nslab;
   };
 
   if (warp == WPROD && lane == 0) {
@@ -250,9 +253,9 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
       job.sched.decode(t, z, mt, nt);
       const int ns = slabs(z, s0);
       const int8_t* pa =
-          job.a + ((long long)(z * job.a_tiles + job.m_tile + mt) * job.nslab + s0) * kABytes;
+          job.a + ((long long)(z * job.a_tiles + job.m_tile + mt) * nslab + s0) * kABytes;
       const int8_t* pb =
-          job.b + ((long long)(z * job.b_tiles + job.n_tile + nt) * job.nslab + s0) * kBBytes;
+          job.b + ((long long)(z * job.b_tiles + job.n_tile + nt) * nslab + s0) * kBBytes;
       for (int k = 0; k < ns; k++, g++) {
         const int s = g % kStages;
         if (!tc::mbar_wait(&empty[s], ((g / kStages) & 1) ^ 1)) {
@@ -325,7 +328,7 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
       }
       tc::tc_fence_after();
       double v[32];
-      if (ND == 7 && (job.slab_split ? job.slab_split : job.nslab) <= kShortSlabs)
+      if (ND == 7 && (job.slab_split ? job.slab_split : nslab) <= kShortSlabs)
         drain<ND, ND == 7>(trow, v);
       else
         drain<ND, false>(trow, v);
@@ -352,6 +355,8 @@ struct Gemm {
   int m_tile = 0, n_tile = 0;
   int slab_split = 0;
   bool m_fast = true;
+  const int* cplx = nullptr;   // as Job::cplx, Job::nslab_real
+  int nslab_real = 0;
 };
 
 // ND: accumulators (7, or 8 for the digit pairs one step further down).
@@ -383,6 +388,8 @@ cudaError_t launch(const Gemm& g, const Epi& epi, int* err, cudaStream_t st) {
   j.n_tile = g.n_tile;
   j.nslab = g.a->nslab;
   j.slab_split = g.slab_split;
+  j.cplx = g.cplx;
+  j.nslab_real = g.nslab_real;
   const int total = j.sched.total();
   const int grid = total < tc::sm_count() ? total : tc::sm_count();
   kern<<<grid, kThreads, kSmem, st>>>(j, epi, err);

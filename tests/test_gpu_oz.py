@@ -116,3 +116,40 @@ def test_vhs_and_propagation_match_fp64(nmo, nel, nchol, nw, cplx):
             want = P @ S
             assert np.max(np.abs(W1[w, sp] - want)) <= 1e-13 * np.max(np.abs(want))
     e.close()
+
+
+# the caller-owned buffers' path from its threshold on: several walker and Cholesky chunks,
+# chunks that end inside a row tile, n up to 96, real and complex factors, and the largest n
+@pytest.mark.parametrize("nmo,nel,nchol,nw,cplx", [(33, 20, 900, 131, False), (40, 40, 150, 61, True),
+                                                   (96, 96, 70, 33, False), (61, 3, 800, 700, True)])
+def test_exchange_of_buffers_matches_fp64(nmo, nel, nchol, nw, cplx):
+    import torch
+    from miniafqmc_b200.afqmc import load_library
+    g = torch.Generator("cuda").manual_seed(nmo)
+
+    def rand(*shape, imag=True):
+        x = torch.randn(*shape, generator=g, device="cuda", dtype=torch.float64)
+        y = torch.randn(*shape, generator=g, device="cuda", dtype=torch.float64)
+        return torch.complex(x, y if imag else torch.zeros_like(y))
+
+    L, G = rand(nchol, 2, nel, nmo, imag=cplx), rand(nw, 2, nel, nmo)
+    G[1] *= 1e-200   # a row scale of its own per walker; T T underflows to zero
+    G[2, 1, 0, 0] = float("inf")
+    ek = torch.empty(nw, dtype=torch.complex128, device="cuda")
+    lib = load_library()
+    for _ in range(2):
+        ek.fill_(7.0)
+        st = lib.afq_exchange_energy_noalloc(L.data_ptr(), G.data_ptr(), nmo, nel, nchol, nw,
+                                             ek.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+    want = torch.zeros(nw, dtype=torch.complex128, device="cuda")
+    size = torch.zeros(nw, dtype=torch.float64, device="cuda")
+    for s in range(2):
+        for c in range(nchol):
+            T = torch.einsum("ak,wbk->wab", L[c, s], G[:, s])
+            want += 0.5 * (T * T.transpose(1, 2)).sum((1, 2))
+            size += (T.abs() ** 2).sum((1, 2))
+    got, want, size = ek.cpu().numpy(), want.cpu().numpy(), size.cpu().numpy()
+    assert not np.isfinite(got[2])
+    keep = np.arange(nw) != 2
+    assert np.all(np.abs(got[keep] - want[keep]) <= 64 * nmo * EPS * size[keep])
