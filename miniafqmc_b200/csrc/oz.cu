@@ -18,6 +18,7 @@ struct OzState {
   std::vector<void*> allocs;
   char* block = nullptr;    // rest of the last shared block
   size_t block_left = 0;
+  size_t free_left = 0;     // device memory not yet planned for
   int* err = nullptr;
   // exchange: rows (c, a) of Lh per spin, columns (w, b, re | im) of G, T = Lh_c Gc_w^T of a
   // chunk of Cholesky vectors and walkers
@@ -577,11 +578,11 @@ trace_kernel(const z_t* __restrict__ T, int n, long long ld, int row0, int c_fir
 
 namespace {
 
-// device bytes left for the next group of allocations: none takes more than a third
-bool fits(cudaError_t& e, size_t need) {
-  size_t free_b = 0, total_b = 0;
-  if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total_b);
-  return e == cudaSuccess && need < free_b / 3;
+// Whether the next group of allocations takes less than a third of the device memory left.
+bool fits(OzState* o, cudaError_t e, size_t need) {
+  if (e != cudaSuccess || need >= o->free_left / 3) return false;
+  o->free_left -= need;
+  return true;
 }
 size_t slice_bytes(long long rows, long long K) { return (size_t)kS * (rows + 128) * (K + 64); }
 
@@ -602,7 +603,7 @@ cudaError_t create_exchange(OzState* o, cudaStream_t st) {
   if (o->ex_c < nc && whole * per_c <= cap + cap / 4)
     o->ex_c = (int)((cap + cap / 4) / per_c / whole) * whole;
   const size_t tb = per_c * o->ex_c + 256LL * 16 * (o->ex_w + 1) * n;   // whole row tiles
-  if (!fits(e, 2 * slice_bytes((long long)nc * n, K) + slice_bytes(2LL * nw * n, K) + tb)) return e;
+  if (!fits(o, e, 2 * slice_bytes((long long)nc * n, K) + slice_bytes(2LL * nw * n, K) + tb)) return e;
   for (int s = 0; s < 2 && e == cudaSuccess; s++) {
     e = alloc_slices(o, &o->lx[s], oz::kBM, nc * n, 1, K);
     if (e != cudaSuccess) break;
@@ -644,7 +645,7 @@ cudaError_t create_gsites(OzState* o, cudaStream_t st) {
     g.splits = (nslab + g.slab_split - 1) / g.slab_split;
     pmax = std::max(pmax, (size_t)(g.splits * rows[i] * o->part_ld));
   }
-  if (!pmax || !fits(e, need + slice_bytes(2 * nw, K) + 8 * pmax)) return e;
+  if (!pmax || !fits(o, e, need + slice_bytes(2 * nw, K) + 8 * pmax)) return e;
   if (e == cudaSuccess) e = alloc_slices(o, &o->gb, oz::kBN, 2 * nw, 1, K);
   if (e == cudaSuccess) e = oz_alloc(o, &o->part, pmax);
   for (int i = 0; i < OZ_NG && e == cudaSuccess; i++) {
@@ -677,7 +678,7 @@ cudaError_t create_vhs(OzState* o, cudaStream_t st) {
   const double dense = 15e-6 + (double)((tiles + 147) / 148) *
                                    (2e-6 + 1.0e-6 * ((K + oz::kSlab - 1) / oz::kSlab));
   if (dense >= csr) return e;
-  if (!fits(e, slice_bytes(N2, K) + slice_bytes(2LL * in.nw, K))) return e;
+  if (!fits(o, e, slice_bytes(N2, K) + slice_bytes(2LL * in.nw, K))) return e;
   e = alloc_slices(o, &o->sp, oz::kBM, (int)N2, 1, K);
   if (e == cudaSuccess) e = alloc_slices(o, &o->xb, oz::kBN, 2 * in.nw, 1, K);
   if (e == cudaSuccess)
@@ -697,7 +698,7 @@ cudaError_t create_propagate(OzState* o, cudaStream_t st) {
   cudaError_t e = cudaSuccess;
   if (8.0 * N * (double)N * n2 * nw < 3e8 || 2 * N > oz::kMaxK || nw > 65535) return e;
   const int Kp = o->preal ? N : 2 * N;
-  if (!fits(e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
+  if (!fits(o, e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
                                                   slice_bytes(2 * n2, 2 * N))))
     return e;
   if (e == cudaSuccess) e = alloc_slices(o, &o->pa, oz::kBM, N, 1, Kp);
@@ -831,7 +832,9 @@ cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
   *out = nullptr;
   OzState* o = new OzState();
   o->in = in;
-  cudaError_t e = oz_alloc(o, &o->err, 1);
+  size_t total_b = 0;
+  cudaError_t e = cudaMemGetInfo(&o->free_left, &total_b);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->err, 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
   const long long NAK = 2LL * in.n * in.N;
   RealCheck rc[4] = {{in.Lh, in.nchol * NAK, true},
