@@ -9,24 +9,26 @@
 
 #include "afq_kernels.h"
 #include "afq_common.cuh"
+#include "gj.cuh"
 
 namespace afq {
 
 // ============================================================ mixed density matrix
 // One CTA per (walker, spin).  T1 = W_s^T tw_s (n x n, mixed_density_matrix.hpp:83);
-// Gauss-Jordan with partial pivoting (max |re|+|im|, as izamax) gives det(T1) and
+// Gauss-Jordan with partial pivoting (max |re|+|im|, as izamax; gj.cuh) gives det(T1) and
 // T1^-1 (ma_operations.hpp:244-260); Gc_s = T1^-1 W_s^T (mixed_density_matrix.hpp:91).
-// want_gc == 0 runs only the LU elimination for the determinant (Overlap, :124-138).
+// want_gc == 0 runs only the elimination for the determinant (Overlap, :124-138).
 constexpr int DM_KC = 32;
 constexpr int DM_THREADS = 256;
 
 size_t dm_smem_bytes(int n) {
   size_t ldT = n + 1;
   size_t buf = std::max((size_t)2 * DM_KC * n, (size_t)n * 65);   // phase 1 slabs | W^T chunk
-  return sizeof(z_t) * (n * ldT + buf + n) + sizeof(int) * n;
+  return sizeof(z_t) * (n * ldT + buf);
 }
 
-__global__ void __launch_bounds__(DM_THREADS)
+template <int RPL>
+__global__ void __launch_bounds__(DM_THREADS, 2)
 dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
           z_t* __restrict__ Gc, z_t* __restrict__ Wd, int* __restrict__ info, int want_gc,
           int save_old) {
@@ -35,15 +37,11 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
   const int ldT = n + 1;
   z_t* T = reinterpret_cast<z_t*>(dm_smem);
   z_t* buf = T + n * ldT;
-  const int bufsz = max(2 * DM_KC * n, n * 65);
-  z_t* fcol = buf + bufsz;
-  int* perm = reinterpret_cast<int*>(fcol + n);
-  __shared__ int s_piv, s_sing;
+  __shared__ GjState gj;
   const long long ldw = 2 * n;
   const z_t* Ws = W + (long long)w * N * ldw + s * n;
   const z_t* ts = tw + s * n;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int nout = n * n;
 
   // ---- phase 1: T1 = W_s^T tw_s; thread (ta, tb) of a 16 x 16 grid owns rows
   // a = ta + 16i and columns b = tb + 16j (i, j < R = ceil(n/16)), a register block that
@@ -88,87 +86,20 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
         if (i < R && j < R && a < n && b < n) T[a * ldT + b] = acc[i][j];
       }
   }
-  if (tid == 0) s_sing = 0;
-  __syncthreads();
 
   // ---- phase 2: pivoted elimination
-  z_t det = zmk(1.0, 0.0);
-  for (int j = 0; j < n; j++) {
-    if (tid < 32) {
-      double best = -1.0;
-      int bi = n;
-      for (int i = j + tid; i < n; i += 32) {
-        double v = zabs1(T[i * ldT + j]);
-        if (v > best) { best = v; bi = i; }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (tid == 0) { s_piv = bi; perm[j] = bi; }
-    }
-    __syncthreads();
-    const int p = s_piv;
-    if (p != j)
-      for (int c = tid; c < n; c += nt) {
-        z_t t = T[j * ldT + c];
-        T[j * ldT + c] = T[p * ldT + c];
-        T[p * ldT + c] = t;
-      }
-    __syncthreads();
-    const z_t pv = T[j * ldT + j];
-    if (pv.x == 0.0 && pv.y == 0.0) {  // exactly singular: uniform across the CTA
-      if (tid == 0) s_sing = 1;
-      break;
-    }
-    if (tid == 0) {
-      det = zmul(det, pv);
-      if (p != j) det = zmk(-det.x, -det.y);
-    }
-    const z_t inv = zrecip(pv);
-    if (!want_gc) {
-      const int m = n - j - 1;
-      for (int e = tid; e < m * m; e += nt) {
-        int i = j + 1 + e / m, c = j + 1 + e % m;
-        z_t f = zmul(T[i * ldT + j], inv);
-        T[i * ldT + c] = zsub(T[i * ldT + c], zmul(f, T[j * ldT + c]));
-      }
-      __syncthreads();
-    } else {
-      for (int i = tid; i < n; i += nt) fcol[i] = T[i * ldT + j];
-      __syncthreads();
-      for (int c = tid; c < n; c += nt)
-        T[j * ldT + c] = (c == j) ? inv : zmul(T[j * ldT + c], inv);
-      __syncthreads();
-      for (int e = tid; e < nout; e += nt) {
-        int i = e / n, c = e % n;
-        if (i == j) continue;
-        z_t base = (c == j) ? zmk(0, 0) : T[i * ldT + c];
-        T[i * ldT + c] = zsub(base, zmul(fcol[i], T[j * ldT + c]));
-      }
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  const int sing = s_sing;
-  if (sing) det = zmk(0, 0);
+  gj_run<RPL, DM_THREADS / 32>(T, ldT, n, want_gc, 0, gj);
+  const int sing = gj.sing;
+  const z_t det = gj.det;
 
-  // ---- phase 3: Gc_s = T1^-1 W_s^T
+  // ---- phase 3: Gc_s = T1^-1 W_s^T, T1^-1[a][b] = T[pivrow[a]][invp[b]]
   if (want_gc) {
     z_t* Gout = Gc + ((long long)w * 2 + s) * n * N;
-    if (!sing) {
-      for (int j = n - 1; j >= 0; j--) {   // undo the row interchanges on the columns
-        int p = perm[j];
-        if (p != j)
-          for (int r = tid; r < n; r += nt) {
-            z_t t = T[r * ldT + j];
-            T[r * ldT + j] = T[r * ldT + p];
-            T[r * ldT + p] = t;
-          }
-        __syncthreads();
-      }
+    const z_t* Ta[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int a = ta + 16 * i;
+      Ta[i] = T + ((!sing && a < n) ? gj.pivrow[a] * ldT : 0);
     }
     // Gc[a][k] = sum_b Tinv[a][b] W[k][b] over 64-row chunks of W: thread (ta, tk) owns
     // rows a = ta + 16i (i < R) and chunk columns k = tk + 16j (j < 4)
@@ -189,10 +120,11 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
       if (!sing)
         for (int b = 0; b < n; b++) {
           z_t tv[4], wv[4];
+          const int ib = gj.invp[b];
 #pragma unroll
           for (int i = 0; i < 4; i++) {
             const int a = ta + 16 * i;
-            tv[i] = (i < R && a < n) ? T[a * ldT + b] : zmk(0, 0);
+            tv[i] = (i < R && a < n) ? Ta[i][ib] : zmk(0, 0);
             wv[i] = buf[b * (KC3 + 1) + tk + 16 * i];
           }
 #pragma unroll
@@ -222,21 +154,28 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
   }
 }
 
-cudaError_t launch_dm(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc, z_t* Wd,
-                      int* info, int want_gc, int save_old, cudaStream_t st) {
+template <int RPL>
+cudaError_t launch_dm_rpl(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc, z_t* Wd,
+                          int* info, int want_gc, int save_old, cudaStream_t st) {
   size_t smem = dm_smem_bytes(n);
   static DeviceAttr attr;
   cudaError_t e = attr.ensure(smem, [](size_t b) {
-    cudaError_t r = cudaFuncSetAttribute(dm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t r = cudaFuncSetAttribute(dm_kernel<RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)b);
     if (r == cudaSuccess)   // several CTAs per SM need the full shared-memory carveout
-      r = cudaFuncSetAttribute(dm_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+      r = cudaFuncSetAttribute(dm_kernel<RPL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
     return r;
   });
   if (e != cudaSuccess) return e;
-  dm_kernel<<<2 * nw, DM_THREADS, smem, st>>>(W, tw, N, n, Gc, Wd, info, want_gc, save_old);
+  dm_kernel<RPL><<<2 * nw, DM_THREADS, smem, st>>>(W, tw, N, n, Gc, Wd, info, want_gc, save_old);
   return cudaGetLastError();
+}
+
+cudaError_t launch_dm(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc, z_t* Wd,
+                      int* info, int want_gc, int save_old, cudaStream_t st) {
+  return n <= 32 ? launch_dm_rpl<1>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st)
+                 : launch_dm_rpl<2>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st);
 }
 
 // ============================================================ sigma

@@ -29,6 +29,7 @@
 
 #include "afq_kernels.h"
 #include "afq_mixed.h"
+#include "gj.cuh"
 #include "tc_gemm.cuh"
 
 namespace afq {
@@ -545,112 +546,35 @@ lu_inv_kernel(const float2* __restrict__ T1, int n, Op Tinv, z_t* __restrict__ W
   }
 }
 
-// The same Gauss-Jordan (in-place exchange form, implicit izamax pivoting) with the matrix
-// in shared memory: 128 threads per matrix (warps on rows, lanes on columns), two
-// barriers per pivot (the searching warp also scales the pivot row); small register
-// footprint, so five matrices share an SM.
+// The same Gauss-Jordan with the matrix in shared memory (gj.cuh), 128 threads per matrix.
+// 2048 matrices of 48 x 48: 0.56 -> 0.43 ms, 2048 of 64 x 64 1.31 -> 0.79 ms (a pivot at a time
+// before); what remains is the panel's chain, 1240 clocks per pivot at four matrices per SM.
 constexpr int LUS_THREADS = 128;
-size_t lus_smem_bytes(int n) { return sizeof(z_t) * ((size_t)n * (n + 1) + 2 * n); }
+size_t lus_smem_bytes(int n) { return sizeof(z_t) * (size_t)n * (n + 1); }
 
-__global__ void __launch_bounds__(LUS_THREADS)
+template <int RPL>
+__global__ void __launch_bounds__(LUS_THREADS, 4)
 lu_smem_kernel(const float2* __restrict__ T1, int n, Op Tinv, z_t* __restrict__ Wd,
                int* __restrict__ info, int want_inv, int save_old) {
   extern __shared__ __align__(16) unsigned char lus_raw[];
-  __shared__ int s_p, pivrow[64], invp[64], used[64];
-  __shared__ z_t s_pv;
-  const int q = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int NWARP = LUS_THREADS / 32;
+  __shared__ GjState gj;
+  const int q = blockIdx.x, tid = threadIdx.x;
   const int ld = n + 1, nn = n * n;
   z_t* T = reinterpret_cast<z_t*>(lus_raw);
-  z_t* pcol = T + n * ld;
-  z_t* prow = pcol + n;
   const float2* src = T1 + (long long)q * nn;
   for (int e = tid; e < nn; e += LUS_THREADS) {
     const float2 v = src[e];
     T[(e / n) * ld + e % n] = zmk(v.x, v.y);
   }
-  for (int i = tid; i < 64; i += LUS_THREADS) used[i] = 0;
-  __syncthreads();
-  z_t det = zmk(1.0, 0.0);
-  int sing = 0;
-  for (int j = 0; j < n; j++) {
-    if (warp == 0) {   // pivot: max |re| + |im| of column j over the unused rows
-      double best = -1.0;
-      int bi = n;
-      for (int i = lane; i < n; i += 32) {
-        if (used[i]) continue;
-        const double v = zabs1(T[i * ld + j]);
-        if (v > best) { best = v; bi = i; }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (lane == 0) {
-        s_p = best > 0.0 ? bi : -1;
-        if (bi < n) {
-          s_pv = T[bi * ld + j];
-          used[bi] = 1;
-          pivrow[j] = bi;
-        }
-      }
-    }
-    if (warp == 0) {   // the scaled pivot row, prepared by the searching warp
-      __syncwarp();
-      const int pp = s_p;
-      if (pp >= 0) {
-        const z_t inv = zrecip(T[pp * ld + j]);
-        for (int c = lane; c < n; c += 32) prow[c] = (c == j) ? inv : zmul(T[pp * ld + c], inv);
-      }
-    }
-    __syncthreads();
-    const int p = s_p;
-    if (p < 0) { sing = 1; break; }   // uniform across the CTA
-    if (tid == 0) det = zmul(det, s_pv);
-    // lanes own columns lane and lane + 32 (n <= 64): the pivot row's values stay in
-    // registers across the rows; a row's factor is its own column-j entry, read before
-    // any lane of the warp writes the row; four rows per warp in flight
-    const bool c0 = lane < n, c1 = lane + 32 < n;
-    const z_t pr0 = c0 ? prow[lane] : zmk(0, 0), pr1 = c1 ? prow[lane + 32] : zmk(0, 0);
-#pragma unroll 4
-    for (int i = warp; i < n; i += NWARP) {
-      z_t* Ti = T + i * ld;
-      if (i == p) {
-        if (c0) Ti[lane] = pr0;
-        if (c1) Ti[lane + 32] = pr1;
-        continue;
-      }
-      const z_t f = Ti[j];
-      const z_t b0 = (c0 && lane != j) ? Ti[lane] : zmk(0, 0);
-      const z_t b1 = (c1 && lane + 32 != j) ? Ti[lane + 32] : zmk(0, 0);
-      __syncwarp();
-      if (c0)
-        Ti[lane] = zmk(fma(-f.x, pr0.x, fma(f.y, pr0.y, b0.x)), fma(-f.x, pr0.y, fma(-f.y, pr0.x, b0.y)));
-      if (c1)
-        Ti[lane + 32] =
-            zmk(fma(-f.x, pr1.x, fma(f.y, pr1.y, b1.x)), fma(-f.x, pr1.y, fma(-f.y, pr1.x, b1.y)));
-    }
-    __syncthreads();
-  }
-  if (sing) det = zmk(0, 0);
-  if (tid == 0 && !sing) {
-    int inv_cnt = 0;
-    for (int a = 0; a < n; a++)
-      for (int b = a + 1; b < n; b++) inv_cnt += pivrow[a] > pivrow[b];
-    if (inv_cnt & 1) det = zmk(-det.x, -det.y);
-    for (int a = 0; a < n; a++) invp[pivrow[a]] = a;
-  }
-  __syncthreads();
+  gj_run<RPL, LUS_THREADS / 32>(T, ld, n, want_inv, 1, gj);
+  const int sing = gj.sing;
   if (want_inv) {
     const long long base = (long long)q * 2 * n * 2 * n;
-    for (int e = tid; e < nn; e += LUS_THREADS) {
-      const int i = e / n, c = e % n;
-      const int ra = sing ? i : invp[i], cb = sing ? c : pivrow[c];
-      const z_t y = sing ? zmk(0, 0) : T[i * ld + c];
-      put2(Tinv, base + (2LL * ra) * 2 * n + 2 * cb, (float)y.x, (float)-y.y);
-      put2(Tinv, base + (2LL * ra + 1) * 2 * n + 2 * cb, (float)y.y, (float)y.x);
+    for (int e = tid; e < nn; e += LUS_THREADS) {   // row a of T1^-1, lanes along b
+      const int a = e / n, b = e % n;
+      const z_t y = sing ? zmk(0, 0) : T[gj.pivrow[a] * ld + gj.invp[b]];
+      put2(Tinv, base + (2LL * a) * 2 * n + 2 * b, (float)y.x, (float)-y.y);
+      put2(Tinv, base + (2LL * a + 1) * 2 * n + 2 * b, (float)y.y, (float)y.x);
     }
   }
   if (tid == 0) {
@@ -660,28 +584,35 @@ lu_smem_kernel(const float2* __restrict__ T1, int n, Op Tinv, z_t* __restrict__ 
       if (sp == 0) d[5] = d[4];
       d[6 + sp] = d[2 + sp];
     }
-    d[2 + sp] = det;
+    d[2 + sp] = gj.det;
     info[q] = sing;
   }
+}
+
+template <int RPL>
+cudaError_t launch_lu_smem(const float2* T1, int n, int nmat, Op Tinv, z_t* Wd, int* info,
+                           int want_inv, int save_old, cudaStream_t st) {
+  const size_t smem = lus_smem_bytes(n);
+  static DeviceAttr attr;   // and the full shared-memory carveout: several matrices per SM
+  cudaError_t e = attr.ensure(smem, [](size_t b) {
+    cudaError_t r = cudaFuncSetAttribute(lu_smem_kernel<RPL>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(lu_smem_kernel<RPL>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
+    return r;
+  });
+  if (e != cudaSuccess) return e;
+  lu_smem_kernel<RPL><<<nmat, LUS_THREADS, smem, st>>>(T1, n, Tinv, Wd, info, want_inv, save_old);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_lu(const float2* T1, int n, int nmat, Op Tinv, z_t* Wd, int* info, int want_inv,
                       int save_old, cudaStream_t st) {
   static const bool regs = getenv("AFQ_LU_REGISTERS") != nullptr;
   if (!regs && n <= 64) {   // shared-memory form (default)
-    const size_t smem = lus_smem_bytes(n);
-    static DeviceAttr attr;   // and the full shared-memory carveout: five matrices per SM
-    cudaError_t e = attr.ensure(smem, [](size_t b) {
-      cudaError_t r = cudaFuncSetAttribute(lu_smem_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
-      if (r == cudaSuccess)
-        r = cudaFuncSetAttribute(lu_smem_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-      return r;
-    });
-    if (e != cudaSuccess) return e;
-    lu_smem_kernel<<<nmat, LUS_THREADS, smem, st>>>(T1, n, Tinv, Wd, info, want_inv, save_old);
-    return cudaGetLastError();
+    return n <= 32 ? launch_lu_smem<1>(T1, n, nmat, Tinv, Wd, info, want_inv, save_old, st)
+                   : launch_lu_smem<2>(T1, n, nmat, Tinv, Wd, info, want_inv, save_old, st);
   }
   // 16 x 16 threads per matrix: few registers per thread, many warps per SM
   if (n <= 16)
