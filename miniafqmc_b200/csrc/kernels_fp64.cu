@@ -5,6 +5,7 @@
 //   tw  [N][2n]       trial, same interleave
 //   Gc  [nw][2][n][N] per-walker compact density matrices (linear index s*n*N + a*N + k)
 //   vHS [nw][N][N], vbias / X / xraw [nchol][nw] (reference layout)
+#include <cooperative_groups.h>
 #include <cstdlib>
 
 #include "afq_kernels.h"
@@ -180,20 +181,27 @@ cudaError_t launch_dm(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc
 
 // ============================================================ sigma
 // X = x + i vbias, hybridW[w] = -sum_c i vb (x + i/2 vb)  (miniafqmc_base.cpp:281-289).
-// Block (32 walkers) x (32 groups of Cholesky rows); fixed-order reduction over groups.
-__global__ void __launch_bounds__(1024)
+// A cluster of 8 CTAs per 32 walkers (lanes), a CTA's 32 warps and the cluster's CTAs on
+// Cholesky rows; the groups' sums meet in the first CTA in a fixed order.  The field's normals
+// cost two FP64 logarithm / sine evaluations' latency per row and warp: one CTA per 32
+// walkers took 20 us at 256 rows and 90 us at 1536.
+constexpr int kSigmaCluster = 8;
+__global__ void __cluster_dims__(kSigmaCluster, 1, 1) __launch_bounds__(1024)
 sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restrict__ xraw,
              z_t* __restrict__ hybridW, int nchol, int nw, const DevScalars* __restrict__ sc,
              int use_xraw) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
   __shared__ z_t red[32][33];
-  const int lane = threadIdx.x, g = threadIdx.y;
-  const int w = blockIdx.x * 32 + lane;
+  __shared__ z_t part[32];
+  const int lane = threadIdx.x, g = threadIdx.y, rank = blockIdx.x % kSigmaCluster;
+  const int w = blockIdx.x / kSigmaCluster * 32 + lane;
   const unsigned long long seed = sc->seed, step = sc->step;
   const long long nwg = sc->nwalk_global > 0 ? sc->nwalk_global : nw;
   const long long woff = sc->walker_offset;
   z_t hw = zmk(0, 0);
   if (w < nw) {
-    for (int c = g; c < nchol; c += 32) {
+    for (int c = rank * 32 + g; c < nchol; c += 32 * kSigmaCluster) {
       long long e = (long long)c * nw + w;
       double x;
       if (use_xraw) {
@@ -215,17 +223,24 @@ sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restr
   }
   red[g][lane] = hw;
   __syncthreads();
-  if (g == 0 && w < nw) {
+  if (g == 0) {
     z_t s = zmk(0, 0);
     for (int q = 0; q < 32; q++) s = zadd(s, red[q][lane]);
+    part[lane] = s;
+  }
+  cl.sync();
+  if (rank == 0 && g == 0 && w < nw) {
+    z_t s = zmk(0, 0);
+    for (int q = 0; q < kSigmaCluster; q++) s = zadd(s, cl.map_shared_rank(part, q)[lane]);
     hybridW[w] = s;
   }
+  cl.sync();   // every CTA's sums stay until the first has read them
 }
 
 cudaError_t launch_sigma(const z_t* vbias, z_t* X, double* xraw, z_t* hybridW, int nchol,
                          int nw, const DevScalars* sc, int use_xraw, cudaStream_t st) {
-  sigma_kernel<<<(nw + 31) / 32, dim3(32, 32), 0, st>>>(vbias, X, xraw, hybridW, nchol, nw, sc,
-                                                         use_xraw);
+  sigma_kernel<<<(nw + 31) / 32 * kSigmaCluster, dim3(32, 32), 0, st>>>(vbias, X, xraw, hybridW,
+                                                                       nchol, nw, sc, use_xraw);
   return cudaGetLastError();
 }
 
