@@ -795,6 +795,134 @@ cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStr
   return cudaGetLastError();
 }
 
+// ============================================================ small propagation chain
+// W_w <- P exp(i V_w) P W_w for a small orbital count in ONE launch: a CTA per (walker, eight
+// columns) keeps P, then V, then P in shared memory, the Taylor terms' columns beside it and
+// their sum in registers.  The eight products as launches of their own cost 8.5 us each at 64
+// orbitals and 16 walkers (latency: 64-step K chains on a few SMs); sums run over k in the
+// same order, so the walkers are the same bit for bit.  512 threads: 64 rows x 8 columns (one
+// warp issues an FP64 multiply-add only every ten clocks, so four warps per scheduler), rows
+// i and i + 64 in one pass.
+constexpr int PS_COLS = 8, PS_THREADS = 512, PS_ROWS = PS_THREADS / PS_COLS;
+constexpr int kPropSmallMaxN = 112;
+
+size_t prop_small_smem(int N) { return sizeof(z_t) * ((size_t)N * (N + 1) + 2 * (size_t)N * PS_COLS); }
+
+__global__ void __launch_bounds__(PS_THREADS)
+prop_small_kernel(const z_t* __restrict__ P, const z_t* __restrict__ V, z_t* __restrict__ W,
+                  int N, int n2, int order) {
+  extern __shared__ __align__(16) unsigned char ps_smem[];
+  z_t* M = reinterpret_cast<z_t*>(ps_smem);   // [N][N + 1]
+  z_t* T = M + N * (N + 1);                   // [N][8], two buffers
+  z_t* U = T + N * PS_COLS;
+  const int tid = threadIdx.x, jl = tid % PS_COLS, i0 = tid / PS_COLS;
+  const int j = blockIdx.x * PS_COLS + jl;
+  z_t* Ww = W + (long long)blockIdx.y * N * n2;
+  const z_t* Vw = V + (long long)blockIdx.y * N * N;
+  auto load = [&](const z_t* src) {
+    const int dr = PS_THREADS / N, dc = PS_THREADS - dr * N;
+    for (int r = tid / N, c = tid - tid / N * N; r < N;) {
+      cp_async16(M + r * (N + 1) + c, src + r * N + c, 16);
+      r += dr;
+      if ((c += dc) >= N) {
+        c -= N;
+        r++;
+      }
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+  };
+  const bool two = i0 + PS_ROWS < N, one = i0 < N;
+  const z_t* M0 = M + (one ? i0 : 0) * (N + 1);
+  const z_t* M1 = M + (two ? i0 + PS_ROWS : 0) * (N + 1);
+  z_t acc[2], S[2];
+  auto product = [&](const z_t* B) {
+    acc[0] = acc[1] = zmk(0, 0);
+    if (N <= PS_ROWS) {
+#pragma unroll 8
+      for (int k = 0; k < N; k++) zfma(acc[0], M0[k], B[k * PS_COLS + jl]);
+    } else {
+#pragma unroll 4
+      for (int k = 0; k < N; k++) {
+        const z_t b = B[k * PS_COLS + jl];
+        zfma(acc[0], M0[k], b);
+        zfma(acc[1], M1[k], b);
+      }
+    }
+  };
+  auto put = [&](z_t* B, const z_t (&v)[2]) {
+    if (one) B[i0 * PS_COLS + jl] = v[0];
+    if (two) B[(i0 + PS_ROWS) * PS_COLS + jl] = v[1];
+  };
+  const z_t zero = zmk(0, 0);
+  {
+    const z_t w0[2] = {one && j < n2 ? Ww[(long long)i0 * n2 + j] : zero,
+                       two && j < n2 ? Ww[(long long)(i0 + PS_ROWS) * n2 + j] : zero};
+    put(T, w0);
+  }
+  load(P);
+  product(T);
+  S[0] = acc[0];
+  S[1] = acc[1];
+  put(U, S);
+  if (order > 0) {
+    __syncthreads();   // every row of P is read
+    load(Vw);
+  }
+  z_t *cur = U, *nxt = T;
+  for (int k = 1; k <= order; k++) {   // T = (i / k) V T; S += T
+    product(cur);
+    const z_t f = zmk(0.0, 1.0 / (double)k);
+    const z_t t[2] = {zmul(f, acc[0]), zmul(f, acc[1])};
+    S[0] = zadd(S[0], t[0]);
+    S[1] = zadd(S[1], t[1]);
+    if (k < order)
+      put(nxt, t);
+    else
+      put(nxt, S);
+    __syncthreads();
+    z_t* x = cur;
+    cur = nxt;
+    nxt = x;
+  }
+  if (order > 0)
+    load(P);
+  else
+    __syncthreads();
+  product(cur);
+  if (j < n2) {
+    if (one) Ww[(long long)i0 * n2 + j] = acc[0];
+    if (two) Ww[(long long)(i0 + PS_ROWS) * n2 + j] = acc[1];
+  }
+}
+
+// Up to 1.2e8 real operations per product, where the separate products are latency bound:
+// 64 orbitals, 16 walkers (1.7e7) 70 -> 36 us, 100 orbitals, 20 walkers of 30+30 electrons
+// (9.6e7) 150 -> 127 us; past it the tiled products win (64 orbitals, 250 walkers, 2.6e8: 165
+// against 207 us).
+bool prop_small_fits(int N, int n2, int nw) {
+  return N <= kPropSmallMaxN && nw <= 65535 && 8.0 * N * N * (double)n2 * nw <= 1.2e8;
+}
+
+cudaError_t launch_prop_small(const z_t* P, const z_t* V, z_t* W, int N, int n2, int nw, int order,
+                              cudaStream_t st) {
+  const size_t smem = prop_small_smem(N);
+  static DeviceAttr attr;
+  cudaError_t e = attr.ensure(smem, [](size_t b) {
+    cudaError_t r = cudaFuncSetAttribute(prop_small_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(prop_small_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
+    return r;
+  });
+  if (e != cudaSuccess) return e;
+  prop_small_kernel<<<dim3((n2 + PS_COLS - 1) / PS_COLS, nw), PS_THREADS, smem, st>>>(P, V, W, N, n2,
+                                                                                      order);
+  return cudaGetLastError();
+}
+
 // ============================================================ walker layout
 // Both layouts hold runs of n entries (orbital row i, spin s): one warp per device row,
 // 16-byte entries, coalesced on both sides.
