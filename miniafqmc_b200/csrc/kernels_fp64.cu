@@ -33,6 +33,8 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
 dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
           z_t* __restrict__ Gc, z_t* __restrict__ Wd, int* __restrict__ info, int want_gc,
           int save_old) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char dm_smem[];
   const int w = blockIdx.x >> 1, s = blockIdx.x & 1;
   const int ldT = n + 1;
@@ -169,7 +171,7 @@ cudaError_t launch_dm_rpl(const z_t* W, const z_t* tw, int N, int n, int nw, z_t
     return r;
   });
   if (e != cudaSuccess) return e;
-  dm_kernel<RPL><<<2 * nw, DM_THREADS, smem, st>>>(W, tw, N, n, Gc, Wd, info, want_gc, save_old);
+  pdl_launch(dm_kernel<RPL>, 2 * nw, DM_THREADS, smem, st, W, tw, N, n, Gc, Wd, info, want_gc, save_old);
   return cudaGetLastError();
 }
 
@@ -190,6 +192,8 @@ __global__ void __cluster_dims__(kSigmaCluster, 1, 1) __launch_bounds__(1024)
 sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restrict__ xraw,
              z_t* __restrict__ hybridW, int nchol, int nw, const DevScalars* __restrict__ sc,
              int use_xraw) {
+  pdl_trigger();
+  pdl_wait();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ z_t red[32][33];
@@ -239,7 +243,7 @@ sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restr
 
 cudaError_t launch_sigma(const z_t* vbias, z_t* X, double* xraw, z_t* hybridW, int nchol,
                          int nw, const DevScalars* sc, int use_xraw, cudaStream_t st) {
-  sigma_kernel<<<(nw + 31) / 32 * kSigmaCluster, dim3(32, 32), 0, st>>>(vbias, X, xraw, hybridW,
+  pdl_launch(sigma_kernel, (nw + 31) / 32 * kSigmaCluster, dim3(32, 32), 0, st, vbias, X, xraw, hybridW,
                                                                        nchol, nw, sc, use_xraw);
   return cudaGetLastError();
 }
@@ -257,6 +261,8 @@ csr_walker_kernel(const int* __restrict__ rowIndex, const int* __restrict__ cols
                   const z_t* __restrict__ zvals, const double* __restrict__ rvals,
                   const z_t* __restrict__ B, int nrows, int nw, z_t* __restrict__ out,
                   long long out_ld) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int WALK = 32 * WPL;
   __shared__ z_t tile[ROWS][WALK + 1];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -316,10 +322,10 @@ cudaError_t csr_walker_launch(const int* rowIndex, const int* cols, const z_t* z
                               long long out_ld, cudaStream_t st) {
   dim3 grid((nrows + ROWS - 1) / ROWS, (nw + 32 * WPL - 1) / (32 * WPL));
   if (rvals)
-    csr_walker_kernel<true, ROWS, WPL><<<grid, ROWS * 32, 0, st>>>(rowIndex, cols, nullptr, rvals,
+    pdl_launch(csr_walker_kernel<true, ROWS, WPL>, grid, ROWS * 32, 0, st, rowIndex, cols, nullptr, rvals,
                                                                    B, nrows, nw, out, out_ld);
   else
-    csr_walker_kernel<false, ROWS, WPL><<<grid, ROWS * 32, 0, st>>>(rowIndex, cols, zvals, nullptr,
+    pdl_launch(csr_walker_kernel<false, ROWS, WPL>, grid, ROWS * 32, 0, st, rowIndex, cols, zvals, nullptr,
                                                                     B, nrows, nw, out, out_ld);
   return cudaGetLastError();
 }
@@ -387,6 +393,8 @@ cudaError_t launch_csr_gather(const int* rowIndex, const int* cols, const z_t* v
 __global__ void __launch_bounds__(1024)
 weights_kernel(z_t* __restrict__ Wd, const z_t* __restrict__ hybridW, int nw, double dt,
                DevScalars* __restrict__ sc, int update_eshift) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t red[32];
   const double eshift = sc->eshift;
   double sum = 0.0;
@@ -413,7 +421,7 @@ weights_kernel(z_t* __restrict__ Wd, const z_t* __restrict__ hybridW, int nw, do
 
 cudaError_t launch_weights(z_t* Wd, const z_t* hybridW, int nw, double dt, DevScalars* sc,
                            int update_eshift, cudaStream_t st) {
-  weights_kernel<<<1, 1024, 0, st>>>(Wd, hybridW, nw, dt, sc, update_eshift);
+  pdl_launch(weights_kernel, 1, 1024, 0, st, Wd, hybridW, nw, dt, sc, update_eshift);
   return cudaGetLastError();
 }
 
@@ -469,6 +477,8 @@ constexpr int QR_THREADS = 256;
 
 __global__ void __launch_bounds__(QR_THREADS)
 ortho_kernel(z_t* __restrict__ W, int N, int n) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t tau_s[64];
   __shared__ z_t sdot[4][65];
   __shared__ z_t red[QR_THREADS / 32];
@@ -596,7 +606,7 @@ ortho_kernel(z_t* __restrict__ W, int N, int n) {
 }
 
 cudaError_t launch_ortho(z_t* W, int N, int n, int nw, cudaStream_t st) {
-  ortho_kernel<<<2 * nw, QR_THREADS, 0, st>>>(W, N, n);
+  pdl_launch(ortho_kernel, 2 * nw, QR_THREADS, 0, st, W, N, n);
   return cudaGetLastError();
 }
 
@@ -619,6 +629,8 @@ size_t cholqr_smem_bytes(int n) {
 
 __global__ void __launch_bounds__(256)
 ortho_cholqr_kernel(z_t* __restrict__ W, int N, int n, int* __restrict__ info, int two_pass) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char cq_smem[];
   const int w = blockIdx.x >> 1, s = blockIdx.x & 1;
   const int ld = n + 1;
@@ -791,7 +803,7 @@ cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStr
     const char* e = getenv("AFQ_CHOLQR_PASSES");
     return e && atoi(e) == 2 ? 1 : 0;
   }();
-  ortho_cholqr_kernel<<<2 * nw, 256, smem, st>>>(W, N, n, info, two_pass);
+  pdl_launch(ortho_cholqr_kernel, 2 * nw, 256, smem, st, W, N, n, info, two_pass);
   return cudaGetLastError();
 }
 
@@ -811,6 +823,8 @@ size_t prop_small_smem(int N) { return sizeof(z_t) * ((size_t)N * (N + 1) + 2 * 
 __global__ void __launch_bounds__(PS_THREADS)
 prop_small_kernel(const z_t* __restrict__ P, const z_t* __restrict__ V, z_t* __restrict__ W,
                   int N, int n2, int order) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char ps_smem[];
   z_t* M = reinterpret_cast<z_t*>(ps_smem);   // [N][N + 1]
   z_t* T = M + N * (N + 1);                   // [N][8], two buffers
@@ -918,7 +932,7 @@ cudaError_t launch_prop_small(const z_t* P, const z_t* V, z_t* W, int N, int n2,
     return r;
   });
   if (e != cudaSuccess) return e;
-  prop_small_kernel<<<dim3((n2 + PS_COLS - 1) / PS_COLS, nw), PS_THREADS, smem, st>>>(P, V, W, N, n2,
+  pdl_launch(prop_small_kernel, dim3((n2 + PS_COLS - 1) / PS_COLS, nw), PS_THREADS, smem, st, P, V, W, N, n2,
                                                                                       order);
   return cudaGetLastError();
 }
@@ -1075,6 +1089,8 @@ energy_reduce_kernel(const z_t* __restrict__ Gc, const z_t* __restrict__ haj, in
                      const z_t* __restrict__ Gcloc, const z_t* __restrict__ cv, int nchol,
                      const z_t* __restrict__ Kpart, int nblk, int nw, int mode,
                      z_t* __restrict__ Wd, double* __restrict__ parts) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t red[8];
   const int w = blockIdx.x;
   const z_t* g = Gc + (long long)w * nak;
@@ -1117,7 +1133,7 @@ energy_reduce_kernel(const z_t* __restrict__ Gc, const z_t* __restrict__ haj, in
 cudaError_t launch_energy_reduce(const z_t* Gc, const z_t* haj, int nak, const z_t* Gcloc,
                                  const z_t* cv, int nchol, const z_t* Kpart, int nblk, int nw,
                                  int mode, z_t* Wd, double* parts, cudaStream_t st) {
-  energy_reduce_kernel<<<nw, 256, 0, st>>>(Gc, haj, nak, Gcloc, cv, nchol, Kpart, nblk, nw, mode,
+  pdl_launch(energy_reduce_kernel, nw, 256, 0, st, Gc, haj, nak, Gcloc, cv, nchol, Kpart, nblk, nw, mode,
                                            Wd, parts);
   return cudaGetLastError();
 }
@@ -1125,6 +1141,8 @@ cudaError_t launch_energy_reduce(const z_t* Gc, const z_t* haj, int nak, const z
 // sum Re(eloc) Re(w) and sum Re(w) (afqmc_sys.hpp:127-132), fixed-order reduction.
 __global__ void __launch_bounds__(1024)
 eav_kernel(const z_t* __restrict__ Wd, int nw, DevScalars* __restrict__ sc) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t red[32];
   double a = 0.0, b = 0.0;
   for (int w = threadIdx.x; w < nw; w += blockDim.x) {
@@ -1140,7 +1158,7 @@ eav_kernel(const z_t* __restrict__ Wd, int nw, DevScalars* __restrict__ sc) {
 }
 
 cudaError_t launch_eav(const z_t* Wd, int nw, DevScalars* sc, cudaStream_t st) {
-  eav_kernel<<<1, 1024, 0, st>>>(Wd, nw, sc);
+  pdl_launch(eav_kernel, 1, 1024, 0, st, Wd, nw, sc);
   return cudaGetLastError();
 }
 

@@ -320,6 +320,8 @@ __global__ void pack_sym_kernel(Op Sd, int N, int Kv, const int* __restrict__ pa
 // X [nc][nw] -> Xf rows (w, re|im): real Spvn: (Re X[:,w]) and (Im X[:,w]);
 // complex Spvn: (Re, -Im) and (Im, Re) interleaved along c.
 __global__ void pack_x_kernel(const z_t* __restrict__ X, int nc, int nw, int Kv, int real, Op dst) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t t[32][33];
   const int c0 = blockIdx.x * 32, w0 = blockIdx.y * 32;
   for (int i = threadIdx.y; i < 32; i += blockDim.y) {
@@ -344,6 +346,8 @@ __global__ void pack_x_kernel(const z_t* __restrict__ X, int nc, int nw, int Kv,
 // W [nw][N][2n] -> B form F [nw][4n][2N]: row j: (Re W[:,j], -Im W[:,j]); row 2n+j: (Im, Re)
 // both == 2: real-A form instead, row j = Re W[:, j], row n2 + j = Im W[:, j] (K = N).
 __global__ void pack_w_kernel(const z_t* __restrict__ W, int N, int n2, Op dst, int both = 1) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t t[32][33];
   const int w = blockIdx.z, k0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   const z_t* Ww = W + (long long)w * N * n2;
@@ -380,6 +384,8 @@ __global__ void pack_trial_kernel(const z_t* __restrict__ tw, int N, int n2, Op 
 }
 // W [nw][N][n2] -> bf16 hi/lo in the same layout ((re, im) pairs): A operand of Gc.
 __global__ void pack_wn_kernel(const z_t* __restrict__ W, long long count, Op dst) {
+  pdl_trigger();
+  pdl_wait();
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < count;
        e += (long long)gridDim.x * blockDim.x) {
     const z_t v = W[e];
@@ -556,6 +562,8 @@ template <int RPL>
 __global__ void __launch_bounds__(LUS_THREADS, 4)
 lu_smem_kernel(const float2* __restrict__ T1, int n, Op Tinv, z_t* __restrict__ Wd,
                int* __restrict__ info, int want_inv, int save_old) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char lus_raw[];
   __shared__ GjState gj;
   const int q = blockIdx.x, tid = threadIdx.x;
@@ -603,7 +611,7 @@ cudaError_t launch_lu_smem(const float2* T1, int n, int nmat, Op Tinv, z_t* Wd, 
     return r;
   });
   if (e != cudaSuccess) return e;
-  lu_smem_kernel<RPL><<<nmat, LUS_THREADS, smem, st>>>(T1, n, Tinv, Wd, info, want_inv, save_old);
+  pdl_launch(lu_smem_kernel<RPL>, nmat, LUS_THREADS, smem, st, T1, n, Tinv, Wd, info, want_inv, save_old);
   return cudaGetLastError();
 }
 
@@ -636,6 +644,8 @@ cudaError_t launch_lu(const float2* T1, int n, int nmat, Op Tinv, z_t* Wd, int* 
 // wscale (optional): per-walker factor applied before the conversion (fp16 operands).
 __global__ void pack_gc_kernel(const z_t* __restrict__ Gc, int nw, int n, int N, Op Gb, Op Gx,
                                int nwx = 0, int real = 0, const float* __restrict__ wscale = nullptr) {
+  pdl_trigger();
+  pdl_wait();
   const long long NAK = 2LL * n * N, tot = (long long)nw * NAK;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
        e += (long long)gridDim.x * blockDim.x) {
@@ -674,6 +684,8 @@ __global__ void pack_gc_kernel(const z_t* __restrict__ Gc, int nw, int n, int N,
 __global__ void reduce_part_kernel(const float* __restrict__ part, int splits, int M, int nw,
                                    z_t* __restrict__ out, float ascale = 1.0f,
                                    const float* __restrict__ wscale = nullptr) {
+  pdl_trigger();
+  pdl_wait();
   const long long tot = (long long)M * nw, sz = (long long)M * 2 * nw;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < tot;
        e += (long long)gridDim.x * blockDim.x) {
@@ -1835,7 +1847,7 @@ static cudaError_t vhs_product(MixedState* m, cudaStream_t st) {
 
 cudaError_t mixed_vhs_pack(MixedState* m, const z_t* X, cudaStream_t st) {
   const int nc = m->nc, nw = m->nw;
-  pack_x_kernel<<<dim3((nc + 31) / 32, (nw + 31) / 32), dim3(32, 8), 0, st>>>(X, nc, nw, m->Kv,
+  pdl_launch(pack_x_kernel, dim3((nc + 31) / 32, (nw + 31) / 32), dim3(32, 8), 0, st, X, nc, nw, m->Kv,
                                                                              m->s_real, m->Xf);
   return cudaGetLastError();
 }
@@ -1874,7 +1886,7 @@ static cudaError_t propagate_chain(MixedState* m, z_t* W, int wave, bool timing,
   if (!timing) m->packed = false;
   cudaError_t e;
   if (!from_f2 && !timing) {
-    pack_w_kernel<<<dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st>>>(
+    pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, 
         W, N, n2, m->F[0], pr ? 2 : 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -1943,7 +1955,7 @@ cudaError_t mixed_propagate(MixedState* m, z_t* W, const z_t*, cudaStream_t st) 
   m->packed = false;
   cudaError_t e;
   if (!from_f2) {
-    pack_w_kernel<<<dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st>>>(
+    pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, 
         W, N, n2, m->F[0], pr ? 2 : 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -2115,7 +2127,7 @@ cudaError_t mixed_vhs_multi(MixedState* const* ms, int n, cudaStream_t st) {
 cudaError_t mixed_prop_pack(MixedState* m, const z_t* W, cudaStream_t st) {
   if (m->packed) return cudaSuccess;   // the P W operand is in F2
   const bool pr = m->preal && m->in.order >= 1;
-  pack_w_kernel<<<dim3((m->N + 31) / 32, (2 * m->n + 31) / 32, m->nw), dim3(32, 8), 0, st>>>(
+  pdl_launch(pack_w_kernel, dim3((m->N + 31) / 32, (2 * m->n + 31) / 32, m->nw), dim3(32, 8), 0, st, 
       W, m->N, 2 * m->n, m->F[0], pr ? 2 : 1);
   return cudaGetLastError();
 }
@@ -2187,8 +2199,8 @@ cudaError_t mixed_repack(MixedState* m, const z_t* W, cudaStream_t st) {
   if (n2 % 32 || !m->Wn.hi) return cudaSuccess;   // no fused path: the consumers pack
   const bool pr = m->preal && m->in.order >= 1;
   const dim3 grid((N + 31) / 32, (n2 + 31) / 32, nw), blk(32, 8);
-  pack_w_kernel<<<grid, blk, 0, st>>>(W, N, n2, m->F2, pr ? 2 : 1);
-  pack_w_kernel<<<grid, blk, 0, st>>>(W, N, n2, m->F[0], 0);
+  pdl_launch(pack_w_kernel, grid, blk, 0, st, W, N, n2, m->F2, pr ? 2 : 1);
+  pdl_launch(pack_w_kernel, grid, blk, 0, st, W, N, n2, m->F[0], 0);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
     m->packed = true;
@@ -2223,7 +2235,7 @@ static cudaError_t splitk_product(MixedState* m, const tc::Maps& mp, int prec, f
   }
   if (e != cudaSuccess) return e;
   const bool f16 = prec == PREC_SPLIT16;
-  reduce_part_kernel<<<grid_for((long long)nc * nw), 256, 0, st>>>(
+  pdl_launch(reduce_part_kernel, grid_for((long long)nc * nw), 256, 0, st, 
       m->part, m->splits, nc, nw, out, f16 ? ascale : 1.0f, f16 ? m->wscale : nullptr);
   return cudaGetLastError();
 }
@@ -2231,7 +2243,7 @@ static cudaError_t splitk_product(MixedState* m, const tc::Maps& mp, int prec, f
 // Gb of every walker (per-walker scales first when the G products run fp16 split)
 static cudaError_t pack_gb(MixedState* m, const z_t* Gc, cudaStream_t st) {
   if (m->Gb.f16) gc_scale_kernel<<<m->nw, 256, 0, st>>>(Gc, m->NAK, m->wscale);
-  pack_gc_kernel<<<grid_for((long long)m->nw * m->NAK), 256, 0, st>>>(
+  pdl_launch(pack_gc_kernel, grid_for((long long)m->nw * m->NAK), 256, 0, st, 
       Gc, m->nw, m->n, m->N, m->Gb, Op{}, 0, m->greal, m->Gb.f16 ? m->wscale : nullptr);
   return cudaGetLastError();
 }
@@ -2332,7 +2344,7 @@ cudaError_t mixed_exchange(MixedState* m, const z_t* Gc, int nsub, z_t* Kpart, i
   if (!m->in.Lh || nsub > m->nw) return cudaErrorInvalidValue;
   const bool f16 = m->Gx.f16;
   if (f16) gc_scale_kernel<<<nsub, 256, 0, st>>>(Gc, m->NAK, m->wscale);
-  pack_gc_kernel<<<grid_for((long long)nsub * m->NAK), 256, 0, st>>>(
+  pdl_launch(pack_gc_kernel, grid_for((long long)nsub * m->NAK), 256, 0, st, 
       Gc, nsub, m->n, m->N, Op{}, m->Gx, m->nw, m->greal, f16 ? m->wscale : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -2366,7 +2378,7 @@ cudaError_t mixed_exchange_lowp(MixedState* m, const z_t* Gc, int nsub, z_t* Kpa
                                 cudaStream_t st) {
   if (!m->in.Lh || nsub > m->nw) return cudaErrorInvalidValue;
   if (m->Gx.f16 || m->prec_ek != PREC_SPLIT) return cudaErrorNotSupported;
-  pack_gc_kernel<<<grid_for((long long)nsub * m->NAK), 256, 0, st>>>(
+  pdl_launch(pack_gc_kernel, grid_for((long long)nsub * m->NAK), 256, 0, st, 
       Gc, nsub, m->n, m->N, Op{}, m->Gx, m->nw, m->greal, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -2404,7 +2416,7 @@ cudaError_t mixed_dm(MixedState* m, const z_t* W, z_t* Gc, z_t* Wd, int* info, i
     // T1 (conjugated) of both spins: one 128-row tile per walker; its A operand is packed
     // unless the walkers' packed forms are current
     if (!m->packed) {
-      pack_w_kernel<<<dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st>>>(W, N, n2,
+      pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, W, N, n2,
                                                                                    m->F[0], 0);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -2417,7 +2429,7 @@ cudaError_t mixed_dm(MixedState* m, const z_t* W, z_t* Gc, z_t* Wd, int* info, i
         !want_gc)
       return e;
   }
-  pack_wn_kernel<<<grid_for((long long)nw * N * n2), 256, 0, st>>>(W, (long long)nw * N * n2, m->Wn);
+  pdl_launch(pack_wn_kernel, grid_for((long long)nw * N * n2), 256, 0, st, W, (long long)nw * N * n2, m->Wn);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   for (int sp = 0; sp < 2; sp++) {
     tc::GemmShape g{N, 2 * n, 2 * n, nw, 128, (N + 127) / 128, true, true, 0};

@@ -227,6 +227,8 @@ AFQ_D const z_t* src_row(const RowSrc& src, int r, bool dbl) {
 template <int MODE>
 __global__ void __launch_bounds__(256)
 slice_kernel(RowSrc src, int nrows, int K, Slices s) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
   const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= nrows) return;
@@ -246,6 +248,8 @@ constexpr int kSliceCluster = 8;
 template <int MODE>
 __global__ void __cluster_dims__(kSliceCluster, 1, 1) __launch_bounds__(256)
 slice_cluster_kernel(RowSrc src, int K, Slices s) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
   constexpr bool PAIR = MODE == kPairs || MODE == kSplitCx;   // two digits per entry
   namespace cg = cooperative_groups;
@@ -290,9 +294,9 @@ template <int MODE>
 cudaError_t slice_rows(const RowSrc& src, int nrows, int K, const Slices& s, cudaStream_t st) {
   if (nrows <= 0) return cudaSuccess;
   if (K > 1024)
-    slice_cluster_kernel<MODE><<<nrows * kSliceCluster, 256, 0, st>>>(src, K, s);
+    pdl_launch(slice_cluster_kernel<MODE>, nrows * kSliceCluster, 256, 0, st, src, K, s);
   else
-    slice_kernel<MODE><<<(nrows + 7) / 8, 256, 0, st>>>(src, nrows, K, s);
+    pdl_launch(slice_kernel<MODE>, (nrows + 7) / 8, 256, 0, st, src, nrows, K, s);
   return cudaGetLastError();
 }
 
@@ -303,6 +307,8 @@ template <bool TWO>
 __global__ void __launch_bounds__(256)
 slice_found_kernel(RowSrc src, int nrows, int K, Slices s, const int* __restrict__ cplx,
                    int nslab_real) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= nrows) return;
   const z_t* p = src.row(r);
@@ -326,6 +332,8 @@ slice_found_kernel(RowSrc src, int nrows, int K, Slices s, const int* __restrict
 template <bool REALA>
 __global__ void __cluster_dims__(kSliceCluster, 1, 1) __launch_bounds__(256)
 slice_x_kernel(const z_t* __restrict__ X, int nc, int nw, Slices s) {
+  pdl_trigger();
+  pdl_wait();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ unsigned long long red[2][8][32], mx[2][32];
@@ -400,6 +408,8 @@ slice_x_kernel(const z_t* __restrict__ X, int nc, int nw, Slices s) {
 // W [nw][N][n2] -> Wt [nw][n2][N]
 __global__ void __launch_bounds__(256)
 transpose_kernel(const z_t* __restrict__ W, int N, int n2, z_t* __restrict__ Wt) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t t[32][33];
   const int w = blockIdx.z, k0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   const z_t* src = W + (long long)w * N * n2;
@@ -524,6 +534,8 @@ struct EpiW {
 __global__ void __launch_bounds__(256)
 part_sum_kernel(const double* __restrict__ part, long long ld, long long sz, int splits, int rows,
                 int nw, z_t* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const long long tot = (long long)rows * nw;
   for (long long e = blockIdx.x * 256LL + threadIdx.x; e < tot; e += gridDim.x * 256LL) {
     const long long r = e / nw, w = e - r * nw;
@@ -542,6 +554,8 @@ constexpr int kTraceThreads = 128;
 __global__ void __launch_bounds__(kTraceThreads)
 trace_kernel(const z_t* __restrict__ T, int n, long long ld, int row0, int c_first,
              z_t* __restrict__ Kpart, int nblk, int w_first, int s) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char tr_smem[];
   z_t* t = reinterpret_cast<z_t*>(tr_smem);   // [n][n + 1]
   __shared__ z_t red[kTraceThreads / 32];
@@ -730,6 +744,8 @@ cudaError_t trace_attr(int n, size_t* smem) {
 __global__ void __launch_bounds__(128)
 ek_sum_kernel(const z_t* __restrict__ part, int count, const int* __restrict__ err,
               z_t* __restrict__ ek) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ z_t red[4];
   const int w = blockIdx.x;
   z_t s = zmk(0, 0);
@@ -808,22 +824,22 @@ cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc
     const long long ld = (2LL * w * n + 3) / 4 * 4;
     for (int s = 0; s < 2; s++) {
       const RowSrc gs{Gc + w0 * NAK + (long long)s * n * N, n, NAK, N};
-      slice_found_kernel<true><<<(w * n + 7) / 8, 256, 0, st>>>(gs, w * n, N, g, cplx, nslab_real);
+      pdl_launch(slice_found_kernel<true>, (w * n + 7) / 8, 256, 0, st, gs, w * n, N, g, cplx, nslab_real);
       for (int c0 = 0; c0 < nc; c0 += cc) {
         const int c = std::min(cc, nc - c0);
         a.rows = c * n;
         const RowSrc as{Lh + c0 * NAK + (long long)s * n * N, n, NAK, N};
-        slice_found_kernel<false><<<(c * n + 7) / 8, 256, 0, st>>>(as, c * n, N, a, cplx,
+        pdl_launch(slice_found_kernel<false>, (c * n + 7) / 8, 256, 0, st, as, c * n, N, a, cplx,
                                                                   nslab_real);
         oz::Gemm gm{&a, &g, c * n, 2 * w * n, 1};
         gm.cplx = cplx;
         gm.nslab_real = nslab_real;
         if ((e = oz::launch<7>(gm, EpiRows{b.T, ld, c * n}, err, st)) != cudaSuccess) return e;
-        trace_kernel<<<dim3(c, w), kTraceThreads, smem, st>>>(
+        pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st, 
             reinterpret_cast<const z_t*>(b.T), n, ld / 2, 0, c0, b.part, nc, 0, s);
       }
     }
-    ek_sum_kernel<<<w, 128, 0, st>>>(b.part, 2 * nc, err, ek + w0);
+    pdl_launch(ek_sum_kernel, w, 128, 0, st, b.part, 2 * nc, err, ek + w0);
   }
   return cudaGetLastError();
 }
@@ -884,7 +900,7 @@ cudaError_t oz_gsite(OzState* o, int site, const z_t* Gc, z_t* out, cudaStream_t
   e = oz::launch<7>(gm, EpiPart{o->part, o->part_ld, sz, g.rows}, o->err, st);
   if (e != cudaSuccess) return e;
   const long long tot = (long long)g.rows * nw;
-  part_sum_kernel<<<(unsigned)std::min<long long>((tot + 255) / 256, 148 * 16), 256, 0, st>>>(
+  pdl_launch(part_sum_kernel, (unsigned)std::min<long long>((tot + 255) / 256, 148 * 16), 256, 0, st, 
       o->part, o->part_ld, sz, g.splits, g.rows, nw, out);
   return cudaGetLastError();
 }
@@ -895,9 +911,9 @@ cudaError_t oz_vhs(OzState* o, const z_t* X, z_t* vHS, cudaStream_t st) {
   const int nw = o->in.nw, nc = o->in.nchol;
   const int grid = (nw + 31) / 32 * kSliceCluster;
   if (o->sreal)
-    slice_x_kernel<true><<<grid, 256, 0, st>>>(X, nc, nw, o->xb);
+    pdl_launch(slice_x_kernel<true>, grid, 256, 0, st, X, nc, nw, o->xb);
   else
-    slice_x_kernel<false><<<grid, 256, 0, st>>>(X, nc, nw, o->xb);
+    pdl_launch(slice_x_kernel<false>, grid, 256, 0, st, X, nc, nw, o->xb);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const long long N2 = (long long)o->in.N * o->in.N;
@@ -911,7 +927,7 @@ int oz_propagate_launches(const OzState* o) { return 1 + 1 + 2 * (2 + o->in.orde
 
 cudaError_t oz_propagate(OzState* o, z_t* W, const z_t* vHS, z_t* S, z_t* T, cudaStream_t st) {
   const int N = o->in.N, n2 = 2 * o->in.n, nw = o->in.nw, order = o->in.order;
-  transpose_kernel<<<dim3((N + 31) / 32, (n2 + 31) / 32, nw), 256, 0, st>>>(W, N, n2, T);
+  pdl_launch(transpose_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), 256, 0, st, W, N, n2, T);
   cudaError_t e = cudaGetLastError();
   auto pslice = [&](const z_t* src) {   // walker columns as the B operand of Propg1
     const RowSrc rs{src, 1, N, 0};
@@ -962,7 +978,7 @@ cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nb
         const long long ld = (2LL * w * n + 3) / 4 * 4;
         EpiRows epi{o->T, ld, row0 + c * n};
         if ((e = oz::launch<7>(g, epi, o->err, st)) != cudaSuccess) break;
-        trace_kernel<<<dim3(c, w), kTraceThreads, smem, st>>>(
+        pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st, 
             reinterpret_cast<const z_t*>(o->T), n, ld / 2, row0, c0, Kpart, nblk, w0, s);
         e = cudaGetLastError();
       }

@@ -237,6 +237,8 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
   const int total = job.sched.total();
   const int nslab = job.cplx && *job.cplx == 0 ? job.nslab_real : job.nslab;
   auto slabs = [&](int z, int& s0) {
@@ -392,8 +394,7 @@ cudaError_t launch(const Gemm& g, const Epi& epi, int* err, cudaStream_t st) {
   j.nslab_real = g.nslab_real;
   const int total = j.sched.total();
   const int grid = total < tc::sm_count() ? total : tc::sm_count();
-  kern<<<grid, kThreads, kSmem, st>>>(j, epi, err);
-  return cudaGetLastError();
+  return pdl_launch(kern, grid, kThreads, kSmem, st, j, epi, err);
 }
 
 }  // namespace oz

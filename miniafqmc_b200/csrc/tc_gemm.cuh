@@ -332,6 +332,8 @@ AFQ_D void gemm_tile(const Maps& maps, int mt, int nt, int m0, int n0, int batch
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 4 && lane == 0) {
     // ---- TMA producer
@@ -699,6 +701,8 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
   const int total = job.tile0[job.np];
   auto where = [&](int t, int& p, int& z, int& mt, int& nt) {
     if constexpr (CHAIN)
@@ -1050,9 +1054,8 @@ cudaError_t launch(const Maps& maps, const GemmShape& g, const Epi& epi, int* er
   const int ns = g.n_step > 0 ? g.n_step : BN;
   const unsigned ntiles = (g.N + ns - 1) / ns;
   dim3 grid(g.m_fast ? g.m_tiles : ntiles, g.m_fast ? ntiles : g.m_tiles, g.batch);
-  kern<<<grid, 192, C::SMEM, st>>>(maps, g.K, g.m_step, ns, g.a_batched, g.b_batched, g.k_split,
-                                    g.m_fast ? 1 : 0, g.z0, epi, err);
-  return cudaGetLastError();
+  return pdl_launch(kern, grid, 192, C::SMEM, st, maps, g.K, g.m_step, ns, g.a_batched, g.b_batched,
+                    g.k_split, g.m_fast ? 1 : 0, g.z0, epi, err);
 }
 
 // One launch over the work list of job.np problems (job.tile0 filled by the caller: the
@@ -1124,8 +1127,7 @@ cudaError_t launch_persistent(const Maps& maps, const GemmShape& g, const Epi& e
   const int total = job.tile0[1];
   if (total <= 0) return cudaSuccess;
   const int grid = total < sm_count() ? total : sm_count();
-  kern<<<grid, P::THREADS, P::SMEM, st>>>(job, err);
-  return cudaGetLastError();
+  return pdl_launch(kern, grid, P::THREADS, P::SMEM, st, job, err);
 }
 
 // Chain launch: the persistent kernel over a dependency-ordered tile list (PJob chain
