@@ -28,7 +28,10 @@ size_t dm_smem_bytes(int n) {
   return sizeof(z_t) * (n * ldT + buf);
 }
 
-template <int RPL>
+// R = ceil(n / 16): the register blocks are R x R (a runtime bound left 16 predicated blocks of
+// multiply-adds to issue for any n; 1024 walkers of 48+48 electrons at 384 orbitals 2.50 ->
+// 2.28 ms, 16 of 16+16 at 64 orbitals 31 -> 23 us).
+template <int R>
 __global__ void __launch_bounds__(DM_THREADS, 2)
 dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
           z_t* __restrict__ Gc, z_t* __restrict__ Wd, int* __restrict__ info, int want_gc,
@@ -49,14 +52,13 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
   // ---- phase 1: T1 = W_s^T tw_s; thread (ta, tb) of a 16 x 16 grid owns rows
   // a = ta + 16i and columns b = tb + 16j (i, j < R = ceil(n/16)), a register block that
   // reuses each shared-memory operand R times
-  const int R = (n + 15) / 16;
   const int ta = tid / 16, tb = tid % 16;
   {
-    z_t acc[4][4];
+    z_t acc[R][R];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < R; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = zmk(0, 0);
+      for (int j = 0; j < R; j++) acc[i][j] = zmk(0, 0);
     for (int k0 = 0; k0 < N; k0 += DM_KC) {
       const int kc = min(DM_KC, N - k0);
       for (int e = tid; e < kc * n; e += nt) {
@@ -66,41 +68,41 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
       }
       __syncthreads();
       for (int kk = 0; kk < kc; kk++) {
-        z_t av[4], bv[4];
+        z_t av[R], bv[R];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < R; i++) {
           const int a = ta + 16 * i, b = tb + 16 * i;
-          av[i] = (i < R && a < n) ? buf[kk * n + a] : zmk(0, 0);
-          bv[i] = (i < R && b < n) ? buf[DM_KC * n + kk * n + b] : zmk(0, 0);
+          av[i] = (a < n) ? buf[kk * n + a] : zmk(0, 0);
+          bv[i] = (b < n) ? buf[DM_KC * n + kk * n + b] : zmk(0, 0);
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < R; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (i < R && j < R) zfma(acc[i][j], av[i], bv[j]);
+          for (int j = 0; j < R; j++)
+            zfma(acc[i][j], av[i], bv[j]);
       }
       __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < R; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
+      for (int j = 0; j < R; j++) {
         const int a = ta + 16 * i, b = tb + 16 * j;
-        if (i < R && j < R && a < n && b < n) T[a * ldT + b] = acc[i][j];
+        if (a < n && b < n) T[a * ldT + b] = acc[i][j];
       }
   }
 
   // ---- phase 2: pivoted elimination
-  gj_run<RPL, DM_THREADS / 32>(T, ldT, n, want_gc, 0, gj);
+  gj_run<(R > 2 ? 2 : 1), DM_THREADS / 32>(T, ldT, n, want_gc, 0, gj);
   const int sing = gj.sing;
   const z_t det = gj.det;
 
   // ---- phase 3: Gc_s = T1^-1 W_s^T, T1^-1[a][b] = T[pivrow[a]][invp[b]]
   if (want_gc) {
     z_t* Gout = Gc + ((long long)w * 2 + s) * n * N;
-    const z_t* Ta[4];
+    const z_t* Ta[R];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < R; i++) {
       const int a = ta + 16 * i;
       Ta[i] = T + ((!sing && a < n) ? gj.pivrow[a] * ldT : 0);
     }
@@ -115,33 +117,30 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
         buf[b * (KC3 + 1) + kk] = Ws[(long long)(k0 + kk) * ldw + b];
       }
       __syncthreads();
-      z_t acc[4][4];
+      z_t acc[R][4];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < R; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[i][j] = zmk(0, 0);
       if (!sing)
         for (int b = 0; b < n; b++) {
-          z_t tv[4], wv[4];
+          z_t tv[R], wv[4];
           const int ib = gj.invp[b];
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int a = ta + 16 * i;
-            tv[i] = (i < R && a < n) ? Ta[i][ib] : zmk(0, 0);
-            wv[i] = buf[b * (KC3 + 1) + tk + 16 * i];
-          }
+          for (int i = 0; i < R; i++) tv[i] = ta + 16 * i < n ? Ta[i][ib] : zmk(0, 0);
 #pragma unroll
-          for (int i = 0; i < 4; i++)
+          for (int j = 0; j < 4; j++) wv[j] = buf[b * (KC3 + 1) + tk + 16 * j];
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-              if (i < R) zfma(acc[i][j], tv[i], wv[j]);
+          for (int i = 0; i < R; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) zfma(acc[i][j], tv[i], wv[j]);
         }
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < R; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const int a = ta + 16 * i, kk = tk + 16 * j;
-          if (i < R && a < n && kk < kc) Gout[(long long)a * N + k0 + kk] = acc[i][j];
+          if (a < n && kk < kc) Gout[(long long)a * N + k0 + kk] = acc[i][j];
         }
       __syncthreads();
     }
@@ -157,28 +156,33 @@ dm_kernel(const z_t* __restrict__ W, const z_t* __restrict__ tw, int N, int n,
   }
 }
 
-template <int RPL>
-cudaError_t launch_dm_rpl(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc, z_t* Wd,
+template <int R>
+cudaError_t launch_dm_r(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc, z_t* Wd,
                           int* info, int want_gc, int save_old, cudaStream_t st) {
   size_t smem = dm_smem_bytes(n);
   static DeviceAttr attr;
   cudaError_t e = attr.ensure(smem, [](size_t b) {
-    cudaError_t r = cudaFuncSetAttribute(dm_kernel<RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t r = cudaFuncSetAttribute(dm_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)b);
     if (r == cudaSuccess)   // several CTAs per SM need the full shared-memory carveout
-      r = cudaFuncSetAttribute(dm_kernel<RPL>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      r = cudaFuncSetAttribute(dm_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
     return r;
   });
   if (e != cudaSuccess) return e;
-  pdl_launch(dm_kernel<RPL>, 2 * nw, DM_THREADS, smem, st, W, tw, N, n, Gc, Wd, info, want_gc, save_old);
+  pdl_launch(dm_kernel<R>, 2 * nw, DM_THREADS, smem, st, W, tw, N, n, Gc, Wd, info, want_gc, save_old);
   return cudaGetLastError();
 }
 
 cudaError_t launch_dm(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc, z_t* Wd,
                       int* info, int want_gc, int save_old, cudaStream_t st) {
-  return n <= 32 ? launch_dm_rpl<1>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st)
-                 : launch_dm_rpl<2>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st);
+  switch ((n + 15) / 16) {
+    case 1: return launch_dm_r<1>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st);
+    case 2: return launch_dm_r<2>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st);
+    case 3: return launch_dm_r<3>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st);
+    case 4: return launch_dm_r<4>(W, tw, N, n, nw, Gc, Wd, info, want_gc, save_old, st);
+  }
+  return cudaErrorInvalidValue;   // the register blocks cover n <= 64
 }
 
 // ============================================================ sigma
@@ -627,6 +631,7 @@ size_t cholqr_smem_bytes(int n) {
   return sizeof(z_t) * ((size_t)2 * n * (n + 1) + (size_t)CQ_KC * (n + 1));
 }
 
+template <int R>   // ceil(n / 16): the register blocks in use
 __global__ void __launch_bounds__(256)
 ortho_cholqr_kernel(z_t* __restrict__ W, int N, int n, int* __restrict__ info, int two_pass) {
   pdl_trigger();
@@ -642,18 +647,18 @@ ortho_cholqr_kernel(z_t* __restrict__ W, int N, int n, int* __restrict__ info, i
   const long long ldw = 2 * n;
   z_t* B = W + (long long)w * N * ldw + s * n;
   const int tid = threadIdx.x, nt = blockDim.x;
-  const int R = (n + 15) / 16, ta = tid / 16, tb = tid % 16;   // n <= 64, 256 threads
+  const int ta = tid / 16, tb = tid % 16;   // n <= 64, 256 threads
   if (tid == 0) s_bad = 0;
   for (int pass = 0; pass < 2; pass++) {
     // ---- Gram matrix G[a][b] = sum_k conj(B[k][a]) B[k][b]; thread (ta, tb) of a 16 x 16
     // grid owns a = ta + 16i, b = tb + 16j (i, j < R = ceil(n/16)): R^2 products per 2R
     // shared-memory reads
     {
-      z_t acc[4][4];
+      z_t acc[R][R];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = zmk(0, 0);
+        for (int j = 0; j < R; j++) acc[i][j] = zmk(0, 0);
       for (int k0 = 0; k0 < N; k0 += CQ_KC) {
         const int kc = min(CQ_KC, N - k0);
         for (int e = tid; e < kc * n; e += nt) {
@@ -662,28 +667,28 @@ ortho_cholqr_kernel(z_t* __restrict__ W, int N, int n, int* __restrict__ info, i
         }
         __syncthreads();
         for (int kk = 0; kk < kc; kk++) {
-          z_t av[4], bv[4];
+          z_t av[R], bv[R];
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
+          for (int i = 0; i < R; i++) {
             const int a = ta + 16 * i, b = tb + 16 * i;
-            av[i] = (i < R && a < n) ? buf[kk * ld + a] : zmk(0, 0);
-            bv[i] = (i < R && b < n) ? buf[kk * ld + b] : zmk(0, 0);
+            av[i] = (a < n) ? buf[kk * ld + a] : zmk(0, 0);
+            bv[i] = (b < n) ? buf[kk * ld + b] : zmk(0, 0);
           }
           // blocks i > j hold only a > b: the lower triangle, which nothing reads
 #pragma unroll
-          for (int i = 0; i < 4; i++)
+          for (int i = 0; i < R; i++)
 #pragma unroll
-            for (int j = i; j < 4; j++)
-              if (i < R && j < R) zfma_conj(acc[i][j], av[i], bv[j]);
+            for (int j = i; j < R; j++)
+              zfma_conj(acc[i][j], av[i], bv[j]);
         }
         __syncthreads();
       }
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = i; j < 4; j++) {
+        for (int j = i; j < R; j++) {
           const int a = ta + 16 * i, b = tb + 16 * j;
-          if (i < R && j < R && a < n && b < n) G[a * ld + b] = acc[i][j];
+          if (a < n && b < n) G[a * ld + b] = acc[i][j];
         }
     }
     __syncthreads();
@@ -745,39 +750,38 @@ ortho_cholqr_kernel(z_t* __restrict__ W, int N, int n, int* __restrict__ info, i
         buf[kk * ld + a] = B[(long long)(k0 + kk) * ldw + a];
       }
       __syncthreads();
-      z_t acc[2][4];
+      z_t acc[2][R];
 #pragma unroll
       for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = zmk(0, 0);
+        for (int j = 0; j < R; j++) acc[i][j] = zmk(0, 0);
       // R^-1 is upper triangular: rows a in [16r, 16r + 16) reach columns b = tb + 16j
       // only for j >= r
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        if (r >= R) break;
+      for (int r = 0; r < R; r++) {
         const int a1 = min(16 * r + 16, n);
         for (int a = 16 * r; a < a1; a++) {
-          z_t bv[2], rv[4];
+          z_t bv[2], rv[R];
 #pragma unroll
           for (int i = 0; i < 2; i++) bv[i] = buf[(ta + 16 * i) * ld + a];
 #pragma unroll
-          for (int j = r; j < 4; j++) {
+          for (int j = r; j < R; j++) {
             const int b = tb + 16 * j;
-            rv[j] = (j < R && b < n) ? Ri[a * ld + b] : zmk(0, 0);
+            rv[j] = (b < n) ? Ri[a * ld + b] : zmk(0, 0);
           }
 #pragma unroll
           for (int i = 0; i < 2; i++)
 #pragma unroll
-            for (int j = r; j < 4; j++)
-              if (j < R) zfma(acc[i][j], bv[i], rv[j]);
+            for (int j = r; j < R; j++)
+              zfma(acc[i][j], bv[i], rv[j]);
         }
       }
 #pragma unroll
       for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < R; j++) {
           const int kk = ta + 16 * i, b = tb + 16 * j;
-          if (j < R && kk < kc && b < n) B[(long long)(k0 + kk) * ldw + b] = acc[i][j];
+          if (kk < kc && b < n) B[(long long)(k0 + kk) * ldw + b] = acc[i][j];
         }
       __syncthreads();
     }
@@ -786,15 +790,15 @@ ortho_cholqr_kernel(z_t* __restrict__ W, int N, int n, int* __restrict__ info, i
   if (tid == 0) info[w * 2 + s] |= s_bad ? 2 : 0;
 }
 
-cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStream_t st) {
-  if (n > 64) return cudaErrorInvalidValue;   // the register tiles cover n <= 64
+template <int R>
+cudaError_t launch_cholqr_r(z_t* W, int N, int n, int nw, int* info, cudaStream_t st) {
   size_t smem = cholqr_smem_bytes(n);
   static DeviceAttr attr;
   cudaError_t e = attr.ensure(smem, [](size_t b) {
-    cudaError_t r = cudaFuncSetAttribute(ortho_cholqr_kernel,
+    cudaError_t r = cudaFuncSetAttribute(ortho_cholqr_kernel<R>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
     if (r == cudaSuccess)
-      r = cudaFuncSetAttribute(ortho_cholqr_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+      r = cudaFuncSetAttribute(ortho_cholqr_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
     return r;
   });
@@ -803,8 +807,18 @@ cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStr
     const char* e = getenv("AFQ_CHOLQR_PASSES");
     return e && atoi(e) == 2 ? 1 : 0;
   }();
-  pdl_launch(ortho_cholqr_kernel, 2 * nw, 256, smem, st, W, N, n, info, two_pass);
+  pdl_launch(ortho_cholqr_kernel<R>, 2 * nw, 256, smem, st, W, N, n, info, two_pass);
   return cudaGetLastError();
+}
+
+cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStream_t st) {
+  switch ((n + 15) / 16) {
+    case 1: return launch_cholqr_r<1>(W, N, n, nw, info, st);
+    case 2: return launch_cholqr_r<2>(W, N, n, nw, info, st);
+    case 3: return launch_cholqr_r<3>(W, N, n, nw, info, st);
+    case 4: return launch_cholqr_r<4>(W, N, n, nw, info, st);
+  }
+  return cudaErrorInvalidValue;   // the register tiles cover n <= 64
 }
 
 // ============================================================ small propagation chain
