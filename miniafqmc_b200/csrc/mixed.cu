@@ -171,6 +171,7 @@ struct MixedState {
   int chain_wave = 0;
   float chain_ms[6] = {};
   int splits0 = 1, part_cap = 1;
+  int part_bn = 128;   // columns of a vbias / Coulomb tile (128 or 256)
 };
 
 namespace {
@@ -895,6 +896,13 @@ struct EpiPart {
   AFQ_D void operator()(int z, int, int m, int n0, const float* v) const {
     if (m >= M) return;
     float* row = part + z * sz + (long long)m * Ncol;
+    if (Ncol % 4 == 0) {   // 16-byte aligned groups, whole or past the end
+#pragma unroll
+      for (int i = 0; i < 32; i += 4)
+        if (n0 + i < Ncol)
+          *reinterpret_cast<float4*>(row + n0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < 32; i++)
       if (n0 + i < Ncol) row[n0 + i] = v[i];
@@ -1374,7 +1382,9 @@ int promote_kb(int which) {
   static const KB kb = [] {   // initialised once, thread-safe
     // C4 (NMO 384, 48+48 electrons, nchol 1536, 1024 walkers), same walkers as the FP64
     // form: E_J error 2e-6 Ha with part=2; E_K -1.4e-5 Ha with ex=1 (5.9 ms per 128-walker
-    // subset), -2.7e-5 Ha with ex=2 (4.7 ms), -9.1e-5 Ha without promotion (4.4 ms)
+    // subset), -2.7e-5 Ha with ex=2 (4.7 ms), -9.1e-5 Ha without promotion (4.4 ms).  These
+    // times predate the epilogue's register split (768 vectors x 256 walkers at ex=2 5.25 ->
+    // 4.21 ms)
     KB r{{2, 2}};
     if (const char* env = getenv("AFQ_PROMOTE")) {
       const std::string s(env);
@@ -1634,7 +1644,16 @@ cudaError_t mixed_create(const MixedInit* init, MixedState** out, std::string* m
   // split K of the vbias / Coulomb products so the grid covers the GPU (about four tiles
   // per SM); the tuner also tries half and twice as many slices
   {
-    const int tiles = ((nc + 127) / 128) * ((2 * nw + 127) / 128);
+    // Tile width.  The product is bound by shared memory: per 128-byte K slab a 128-column
+    // tile's MMAs read 96 KB and its fills write 64 KB for 768 tensor clocks (1280 clocks at
+    // 128 bytes a clock), a 256-column tile 144 + 96 KB for 1536 (1920).  1536 vectors x 1024
+    // walkers of 48+48 electrons 0.68 -> 0.47 ms, 1024 x 512 of 64+64 0.23 -> 0.185, 800 x 256
+    // of 40+40 (14 tiles) vbias stage 31 -> 28 us.  With fewer tiles the slices run out (384
+    // vectors x 128 walkers 6.6 -> 8.0 us), and with 262 columns half of the second tile is
+    // padding (54 -> 77 us).
+    const int mt = (nc + 127) / 128, w128 = (2 * nw + 127) / 128, w256 = (2 * nw + 255) / 256;
+    m->part_bn = mt * w256 >= 13 && 16 * w256 <= 9 * w128 ? 256 : 128;
+    const int tiles = mt * ((2 * nw + m->part_bn - 1) / m->part_bn);
     set_splits(m, std::max(1, std::min(16, (int)((4 * 148 + tiles - 1) / tiles))));
     m->splits0 = m->splits;
     const int ks = m->ksplit;
@@ -1737,10 +1756,10 @@ cudaError_t mixed_create(const MixedInit* init, MixedState** out, std::string* m
   const uint64_t Kg = m->greal ? NAK : 2 * NAK;   // K of the vbias / Coulomb products
   const uint64_t Kx = m->greal ? N : 2 * N;       // K of the exchange product
   ok &= map2(m->m_vbias, m->SpT, Kg, nc, 1, Kg, 0, m->Gb, Kg, 2 * nw, 1, Kg, 0,
-             128);
+             m->part_bn);
   if (init->Lh) {
     ok &= map2(m->m_ej, m->LhJ, Kg, nc, 1, Kg, 0, m->Gb, Kg, 2 * nw, 1, Kg, 0,
-               128);
+               m->part_bn);
     m->ex_Gn = 128 / n;
     m->ex_Gw = std::max(1, 256 / (2 * n));
     while (m->ex_Gw > 1 && !pick_bn(m->ex_Gw * 2 * n)) m->ex_Gw--;
@@ -2228,10 +2247,10 @@ static cudaError_t splitk_product(MixedState* m, const tc::Maps& mp, int prec, f
   const int pk = promote_kb(PROMOTE_PART);
   if (pk && m->tune[TS_PART] == 2) return cudaErrorInvalidValue;   // promotion: persistent only
   switch (pk) {   // chained K slabs in TMEM (0: whole slice)
-    case 1: e = run_bn(128, prec, mp, g, EpiPartPromoted<1>{ep}, m->err, st); break;
-    case 2: e = run_bn(128, prec, mp, g, EpiPartPromoted<2>{ep}, m->err, st); break;
-    case 4: e = run_bn(128, prec, mp, g, EpiPartPromoted<4>{ep}, m->err, st); break;
-    default: e = run_bn(128, prec, mp, g, ep, m->err, st, m->tune[TS_PART]);
+    case 1: e = run_bn(m->part_bn, prec, mp, g, EpiPartPromoted<1>{ep}, m->err, st); break;
+    case 2: e = run_bn(m->part_bn, prec, mp, g, EpiPartPromoted<2>{ep}, m->err, st); break;
+    case 4: e = run_bn(m->part_bn, prec, mp, g, EpiPartPromoted<4>{ep}, m->err, st); break;
+    default: e = run_bn(m->part_bn, prec, mp, g, ep, m->err, st, m->tune[TS_PART]);
   }
   if (e != cudaSuccess) return e;
   const bool f16 = prec == PREC_SPLIT16;
