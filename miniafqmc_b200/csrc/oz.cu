@@ -677,8 +677,9 @@ cudaError_t create_gsites(OzState* o, cudaStream_t st) {
 
 // vHS as a dense product.  The CSR kernel does nnz x nw real (complex) multiply-adds at about
 // 2.9e12 (1.4e12) a second (C4's 45.3 M nonzeros x 128 walkers: 3.89 ms; 0.42 M x 256: 90
-// us), a tile slab here takes about 0.55 us of one SM plus 2 us per tile and 15 us of
-// launches: the smaller of the two estimates.
+// us), a tile slab here takes about 1.0 us of one SM under load plus 2 us per tile and 15 us
+// of launches (C4 x 128 walkers: 32 tiles of 24 slabs per SM, 0.93 ms): the smaller of the
+// two estimates.
 cudaError_t create_vhs(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;
   const long long N2 = (long long)in.N * in.N;

@@ -5,8 +5,11 @@
 //   B_KMAJ: B(k,n) = B[b*sB + n*ldb + k]   else B(k,n) = B[b*sB + k*ldb + n]
 //   B_REAL: B holds real doubles (ZGemmDesc::Br), each multiply-add a real x complex one
 //
-// sm_100a has no FP64 tensor-core kind for tcgen05 and its FP64 FMA rate equals its
-// FP64 MMA rate, so the FP64 form is a register-tiled CUDA-core GEMM: a BM x BN tile per
+// Products large enough for the digit splitting of oz.cu run on the int8 tensor cores; this
+// kernel keeps the smaller ones, those whose digits do not fit the device memory, sites
+// without a digit form and the K beyond its int32 sums.  sm_100a has no FP64 tensor-core kind
+// for tcgen05 and its FP64 FMA rate equals its FP64 MMA rate, so it is a register-tiled
+// CUDA-core GEMM: a BM x BN tile per
 // CTA, TM x TN complex accumulators per thread, BK-deep k slabs double-buffered in
 // shared memory with cp.async.  A and B slabs are stored [k][m] / [k][n] so the inner
 // loop reads one A broadcast and TN consecutive B values per k.

@@ -6,11 +6,17 @@ c N n eps cond(W) of each other."""
 import numpy as np
 import pytest
 
-from conftest import tiny_system
+from miniafqmc_b200.synthetic import Config, make_system
 
 pytestmark = pytest.mark.gpu
 
 EPS = 2.0 ** -53
+
+
+def system(nmo, nel, cplx):
+    """Without Vakbl: (nmo nel)^2 entries per spin."""
+    return make_system(Config(nmo, nel, 8, 0.3, 7, dt=0.01, nwalk=3, complex_trial=cplx,
+                              complex_chol=cplx), build_vakbl=False)
 
 
 @pytest.mark.parametrize("nmo,nel", [(1, 1), (5, 5), (40, 15), (40, 16), (300, 17), (33, 32),
@@ -18,7 +24,7 @@ EPS = 2.0 ** -53
 def test_householder_matches_lapack(nmo, nel):
     from miniafqmc_b200.afqmc import AfqmcSys
     nw = 3
-    s = tiny_system(nmo=nmo, nel=nel, nchol=4)
+    s = system(nmo, nel, True)
     rng = np.random.default_rng(nmo + nel)
     W = rng.normal(size=(nw, 2, nmo, nel)) + 1j * rng.normal(size=(nw, 2, nmo, nel))
     W[1, 0] = np.triu(W[1, 0])                       # nothing below the diagonal
@@ -40,7 +46,7 @@ def test_householder_matches_lapack(nmo, nel):
 def test_cholqr_spans_the_same_space(nmo, nel):
     from miniafqmc_b200.afqmc import AfqmcSys, AFQ_PREC_MIXED
     nw = 3
-    s = tiny_system(complex_trial=False, complex_chol=False, nmo=nmo, nel=nel, nchol=8)
+    s = system(nmo, nel, False)
     rng = np.random.default_rng(nmo + nel)
     W, Wd = s.initial_walkers(nw)
     W = W + 0.1 / np.sqrt(nmo) * (rng.normal(size=W.shape) + 1j * rng.normal(size=W.shape))
