@@ -1167,30 +1167,69 @@ struct EpiExchange {
   float ascale;           // scale of the Lh operand (1 for bf16)
   const float* wscale;    // per-walker scale of the G operand (null for bf16)
   AFQ_D void tile(int s, int mt, int nt, float* t, int ld, int tid) const {
+    // Thread (cv, a) sums T[a][b] T[b][a] over the b = a + d (mod n) of half the circle, each
+    // pair once with weight two; products and sums in FP64.  With all n^2 pairs dealt to the
+    // lanes of the walker's warp by an integer division each, one chain of multiply-adds a
+    // lane, the trace outlasted the MMAs six times (616 vectors x 131 walkers of 28+28
+    // electrons at 184 orbitals 1.24 -> 0.97 ms; what is left is one tile at a time per SM).
+    constexpr int kBatch = 8;   // walkers between barriers
+    __shared__ double red[kBatch][4][2];
     const int lane = tid & 31, warp = tid >> 5;
-    for (int wl = warp; wl < Gw; wl += 4) {
-      const int w = nt * Gw + wl;
-      double sr = 0.0, si = 0.0;
-      for (int cv = 0; cv < Gn; cv++) {
-        if (mt * Gn + cv >= nc) break;
-        const float* rows = t + (long long)cv * n * ld + wl * 2 * n;
-        for (int q = lane; q < n * n; q += 32) {
-          const int a = q / n, b = q % n;
-          const double ar = rows[a * ld + b], ai = rows[a * ld + n + b];
-          const double br = rows[b * ld + a], bi = rows[b * ld + n + a];
-          sr += ar * br - ai * bi;
-          si += ar * bi + ai * br;
+    const int ncv = min(Gn, nc - mt * Gn);
+    const int cv = tid / n, a = tid - cv * n;
+    for (int w0 = 0; w0 < Gw; w0 += kBatch) {
+      const int nb = min(kBatch, Gw - w0);
+      for (int wl = 0; wl < nb; wl++) {
+        double sr = 0.0, si = 0.0;
+        if (tid < ncv * n) {
+          const float* blk = t + (long long)cv * n * ld + (w0 + wl) * 2 * n;
+          const float* own = blk + a * ld;   // T[a][.]
+          const float* col = blk + a;        // T[.][a]
+          double pr = 0.0, pi = 0.0;
+          int b = a;
+#pragma unroll 4
+          for (int d = 1; d <= (n - 1) / 2; d++) {
+            b = b + 1 == n ? 0 : b + 1;
+            const double ar = own[b], ai = own[n + b];
+            const double br = col[b * ld], bi = col[b * ld + n];
+            sr = fma(ar, br, sr);
+            pr = fma(ai, bi, pr);
+            si = fma(ar, bi, si);
+            pi = fma(ai, br, pi);
+          }
+          if (n % 2 == 0 && a < n / 2) {     // the opposite point, once per pair
+            b = a + n / 2;
+            const double ar = own[b], ai = own[n + b];
+            const double br = col[b * ld], bi = col[b * ld + n];
+            sr = fma(ar, br, sr);
+            pr = fma(ai, bi, pr);
+            si = fma(ar, bi, si);
+            pi = fma(ai, br, pi);
+          }
+          const double dr = own[a], di = own[n + a];
+          sr = 2.0 * (sr - pr) + (dr * dr - di * di);
+          si = 2.0 * (si + pi) + 2.0 * dr * di;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          sr += __shfl_xor_sync(0xffffffffu, sr, o);
+          si += __shfl_xor_sync(0xffffffffu, si, o);
+        }
+        if (lane == 0) {
+          red[wl][warp][0] = sr;
+          red[wl][warp][1] = si;
         }
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sr += __shfl_xor_sync(0xffffffffu, sr, o);
-        si += __shfl_xor_sync(0xffffffffu, si, o);
-      }
-      if (lane == 0 && w < nw) {
+      tc::epi_bar();
+      const int w = nt * Gw + w0 + tid;
+      if (tid < nb && w < nw) {
+        const double (*r)[2] = red[tid];
         const double u = 1.0 / ((double)ascale * (wscale ? (double)wscale[w] : 1.0));
-        Kpart[((long long)w * 2 + s) * nblk + mt] = zmk(sr * u * u, si * u * u);
+        Kpart[((long long)w * 2 + s) * nblk + mt] =
+            zmk((((r[0][0] + r[1][0]) + r[2][0]) + r[3][0]) * u * u,
+                (((r[0][1] + r[1][1]) + r[2][1]) + r[3][1]) * u * u);
       }
+      if (w0 + kBatch < Gw) tc::epi_bar();   // red is rewritten
     }
   }
 };

@@ -14,7 +14,12 @@ pytestmark = pytest.mark.gpu
 
 # 2n = 24, 32, 64 and 128: 10, 8, 4 and 2 Cholesky vectors per tile
 @pytest.mark.parametrize("nmo,nel,nchol,nw", [(16, 12, 16, 5), (32, 16, 600, 9), (32, 16, 592, 3),
-                                              (32, 32, 608, 4), (64, 64, 304, 3)])
+                                              (32, 32, 608, 4), (64, 64, 304, 3),
+                                              # other widths, per-tile kernel: walkers in
+                                              # batches of eight, half circles of pairs
+                                              (32, 4, 80, 37), (40, 8, 40, 17), (40, 20, 32, 7),
+                                              (56, 28, 16, 10), (64, 36, 8, 5), (48, 44, 8, 3),
+                                              (64, 60, 8, 3)])
 def test_exchange_covers_every_block(nmo, nel, nchol, nw):
     from miniafqmc_b200.afqmc import AfqmcSys, AFQ_PREC_MIXED
     s = tiny_system(complex_trial=False, complex_chol=False, nmo=nmo, nel=nel, nchol=nchol)
