@@ -685,6 +685,7 @@ ortho_smem_kernel(z_t* __restrict__ W, int N, int n) {
     }
     __syncthreads();
   }
+  __syncthreads();   // an identity reflector leaves its turn early: tau_s[n - 1] may just be written
 
   // Q = H(1) ... H(n) applied to the first n columns of the identity (zung2r)
   for (int i = n - 1; i >= 0; i--) {
