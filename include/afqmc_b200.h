@@ -279,6 +279,13 @@ afq_status afq_get_tuning(afq_handle* h, int* choice, double* ms);
  * mixed form.  ms[6]: the best milliseconds of the CSR product and of the dense product
  * per operand (0 when not timed).  With AFQ_TUNE=0 the rule is dense at >= 25% density. */
 afq_status afq_get_sparse_paths(afq_handle* h, int* path, double* ms);
+/* FP64 form: which products run as digit products on the int8 tensor cores (operands
+ * written as signed 8-bit digits; AFQ_PREC_FP64 above), 0s for the mixed form.  on[6]:
+ * vbias, Coulomb vector, Vakbl G, vHS, propagation chain, exchange.  A product that is off
+ * runs on the FP64 pipe as afq_get_sparse_paths and afq_get_tuning describe.  Decided at
+ * set-up from the sizes and the free device memory; AFQ_FP64_DIGITS=0 in the environment
+ * of afq_set_hamiltonian switches all of them off. */
+afq_status afq_get_digit_products(afq_handle* h, int* on);
 /* Mixed form: launch schedule the set-up tuner picked (no reference counterpart); 0s for
  * the FP64 form.
  * sched[0]: walkers per group of the propagation chain.  The chain's products (P W, the

@@ -37,6 +37,7 @@ EXPORTS = [
     "afq_batch_create", "afq_batch_destroy", "afq_batch_substep", "afq_batch_synchronize",
     "afq_get_tuning", "afq_halfrotate", "afq_population_control",
     "afq_mixed_density_matrix_full", "afq_vbias_full", "afq_get_sparse_paths",
+    "afq_get_digit_products",
     "afq_set_tc_wait_limit", "afq_substep_begin", "afq_substep_end", "afq_batch_substeps",
     "afq_copy_walkers", "afq_get_schedule", "afq_batch_set_fused",
 ]
@@ -99,7 +100,7 @@ def signatures() -> dict:
         "afq_halfrotate": ([I, P, I, I, I, P, D, D, P, P, P, P, P], I),
         "afq_population_control": ([P, U64, U64], I),
         "afq_mixed_density_matrix_full": ([P], I), "afq_vbias_full": ([P], I),
-        "afq_get_sparse_paths": ([P, P, P], I),
+        "afq_get_sparse_paths": ([P, P, P], I), "afq_get_digit_products": ([P, P], I),
         "afq_set_tc_wait_limit": ([I, ctypes.c_longlong], I),
         "afq_substep_begin": ([P, U64, U64, P], I), "afq_substep_end": ([P, U64, I], I),
         "afq_batch_substeps": ([P, P, U64, I, I], I),
@@ -363,6 +364,15 @@ class AfqmcSys:
         return {k: {"path": names[int(p[i])], "ms": [round(float(t[2 * i]), 4),
                                                       round(float(t[2 * i + 1]), 4)]}
                 for i, k in enumerate(self.SPARSE_OPERANDS)}
+
+    DIGIT_PRODUCTS = ["vbias", "coulomb", "vakbl", "vHS", "propagate", "exchange"]
+
+    def digit_products(self) -> dict:
+        """FP64 form: per product whether it runs as a digit product on the int8 tensor
+        cores (False: on the FP64 pipe)."""
+        on = np.zeros(6, np.int32)
+        self._check(self.lib.afq_get_digit_products(self.h, _p(on)))
+        return {k: bool(v) for k, v in zip(self.DIGIT_PRODUCTS, on)}
 
     def substep(self, seed: int, step_tot: int, northo: int, graph: bool = True):
         """One substep of the driver loop (miniafqmc_base.cpp:251-337)."""

@@ -1033,7 +1033,8 @@ afq_status afq_set_hamiltonian(afq_handle* h, const afq_csr_z* Spvn, const afq_c
   if (!h->mixed) {
     afq::OzInit oi{N, n, nc, h->nw, h->d.taylor_order, h->Lh, h->spT_dense, h->vk_dense,
                    h->sp_dense, h->sp_dense_r, (long long)Spvn->rowIndex[N * N], h->P};
-    AFQ_CUDA(h, afq::oz_create(oi, &h->oz, h->st));
+    const char* digits = getenv("AFQ_FP64_DIGITS");
+    if (!digits || atoi(digits) != 0) AFQ_CUDA(h, afq::oz_create(oi, &h->oz, h->st));
     if (afq::oz_has_exchange(h->oz, h->nw)) {   // one partial sum per Cholesky vector
       if (nc > h->nblk) AFQ_CUDA(h, dalloc(h, &h->Kpart, (size_t)h->nw * 2 * nc));
       h->nblk = nc;
@@ -1814,6 +1815,15 @@ afq_status afq_get_sparse_paths(afq_handle* h, int* path, double* ms) {
       ms[2 * i + 1] = h->sp_ms[i][1];
     }
   }
+  return AFQ_OK;
+}
+
+afq_status afq_get_digit_products(afq_handle* h, int* on) {
+  if (!h || !on) return AFQ_ERR_ARG;
+  for (int i = 0; i < afq::OZ_NG; i++) on[i] = afq::oz_has_gsite(h->oz, i);
+  on[3] = afq::oz_has_vhs(h->oz);
+  on[4] = afq::oz_has_propagate(h->oz);
+  on[5] = afq::oz_has_exchange(h->oz, h->nw);
   return AFQ_OK;
 }
 
