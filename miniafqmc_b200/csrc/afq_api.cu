@@ -1860,7 +1860,13 @@ afq_status afq_synchronize(afq_handle* h) {
   if (h->cv) AFQ_CUDA(h, afq::cv_sync(h->cv));   // the estimator's online training
   if (h->mixed || h->oz) {
     int flags = 0;
-    AFQ_CUDA(h, h->mixed ? afq::mixed_error(h->mixed, &flags) : afq::oz_error(h->oz, &flags));
+    if (h->mixed) {
+      AFQ_CUDA(h, afq::mixed_error(h->mixed, &flags));
+    } else {
+      int* pinned = reinterpret_cast<int*>(h->h_sc);
+      AFQ_CUDA(h, afq::oz_error(h->oz, pinned, h->st));
+      flags = *pinned;
+    }
     if (flags) return fail(h, AFQ_ERR_CUDA, "tensor-core pipeline wait timed out (flags " +
                                                 std::to_string(flags) + ")");
   }

@@ -59,8 +59,10 @@ struct OzBuffers {
 bool oz_exchange_buffers_fit(const OzBuffers& b, int N, int n, int nc, int nw);
 cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc, int N, int n,
                                 int nc, int nw, z_t* ek, cudaStream_t st);
-// Timeout flags raised by the kernels (0 when clean), and the bound of their waits.
-cudaError_t oz_error(OzState* o, int* flags);
+// Timeout flags raised by the kernels (0 when clean), read into pinned memory on the handle's
+// stream (a copy on the legacy stream would wait for the work of the caller's blocking streams),
+// and the bound of their waits.
+cudaError_t oz_error(OzState* o, int* flags, cudaStream_t st);
 cudaError_t oz_set_wait_clocks(long long clocks);
 
 }  // namespace afq

@@ -988,10 +988,10 @@ cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nb
   return e;
 }
 
-cudaError_t oz_error(OzState* o, int* flags) {
-  *flags = 0;
-  cudaError_t e = cudaMemcpy(flags, o->err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && *flags) e = cudaMemset(o->err, 0, sizeof(int));
+cudaError_t oz_error(OzState* o, int* flags, cudaStream_t st) {
+  cudaError_t e = cudaMemcpyAsync(flags, o->err, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && *flags) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
   return e;
 }
 
