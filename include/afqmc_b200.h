@@ -40,7 +40,13 @@ typedef enum {
 } afq_status;
 
 typedef enum {
-  AFQ_PREC_FP64 = 0,        /* every contraction in FP64 (the plain form)                */
+  AFQ_PREC_FP64 = 0,        /* every contraction in FP64 (the plain form).  Large ones run as
+                               digit products: operand rows in fixed point, 55 bits below
+                               the row's largest entry, products of 8-bit digits summed
+                               exactly; a walker's result then agrees with an FP64
+                               product's in its norm (not entry by entry), and a result
+                               that digits do not hold is computed on the FP64 pipe
+                               (afq_get_digit_products)                               */
   AFQ_PREC_MIXED = 1        /* tensor-core contractions, FP64 LU/QR/weights              */
 } afq_precision;
 
@@ -284,8 +290,10 @@ afq_status afq_get_sparse_paths(afq_handle* h, int* path, double* ms);
  * vbias, Coulomb vector, Vakbl G, vHS, propagation chain, exchange.  A product that is off
  * runs on the FP64 pipe as afq_get_sparse_paths and afq_get_tuning describe.  Decided at
  * set-up from the sizes and the free device memory; AFQ_FP64_DIGITS=0 in the environment
- * of afq_set_hamiltonian switches all of them off. */
-afq_status afq_get_digit_products(afq_handle* h, int* on);
+ * of afq_set_hamiltonian switches all of them off.  redone[6] (may be NULL; synchronises):
+ * the walkers so far whose result the digits did not hold and the FP64 pipe computed (a
+ * product of all walkers counts each). */
+afq_status afq_get_digit_products(afq_handle* h, int* on, long long* redone);
 /* Mixed form: launch schedule the set-up tuner picked (no reference counterpart); 0s for
  * the FP64 form.
  * sched[0]: walkers per group of the propagation chain.  The chain's products (P W, the
@@ -327,7 +335,7 @@ afq_status afq_copy_out(afq_handle* h, int which, void* host);
  * other pointers are rejected with AFQ_ERR_ARG before any device work.
  * Asynchronous on `stream` (a cudaStream_t, NULL for the default stream).  The partial
  * sums live in one file-scope device array of 2^18 complex values, operand digits and a
- * chunk of the products in a second one (4 and 79 MiB, held from the first call on a GPU
+ * chunk of the products in a second one (4 and 81 MiB, held from the first call on a GPU
  * until exit): calls with 2 * nwalk * ceil(nchol / (96 /
  * naea)) above that, or with ceil(nwalk / (96 / naea)) above 65535, are rejected with
  * AFQ_ERR_UNSUPPORTED (split the walkers into batches); naea must be <= 96.  The first

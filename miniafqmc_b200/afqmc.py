@@ -100,7 +100,7 @@ def signatures() -> dict:
         "afq_halfrotate": ([I, P, I, I, I, P, D, D, P, P, P, P, P], I),
         "afq_population_control": ([P, U64, U64], I),
         "afq_mixed_density_matrix_full": ([P], I), "afq_vbias_full": ([P], I),
-        "afq_get_sparse_paths": ([P, P, P], I), "afq_get_digit_products": ([P, P], I),
+        "afq_get_sparse_paths": ([P, P, P], I), "afq_get_digit_products": ([P, P, P], I),
         "afq_set_tc_wait_limit": ([I, ctypes.c_longlong], I),
         "afq_substep_begin": ([P, U64, U64, P], I), "afq_substep_end": ([P, U64, I], I),
         "afq_batch_substeps": ([P, P, U64, I, I], I),
@@ -371,8 +371,15 @@ class AfqmcSys:
         """FP64 form: per product whether it runs as a digit product on the int8 tensor
         cores (False: on the FP64 pipe)."""
         on = np.zeros(6, np.int32)
-        self._check(self.lib.afq_get_digit_products(self.h, _p(on)))
+        self._check(self.lib.afq_get_digit_products(self.h, _p(on), None))
         return {k: bool(v) for k, v in zip(self.DIGIT_PRODUCTS, on)}
+
+    def digit_products_redone(self) -> dict:
+        """Per product the walkers so far whose result the digits did not hold (entries
+        spread too far, infinities) and the FP64 pipe computed."""
+        on, redone = np.zeros(6, np.int32), np.zeros(6, np.int64)
+        self._check(self.lib.afq_get_digit_products(self.h, _p(on), _p(redone)))
+        return {k: int(v) for k, v in zip(self.DIGIT_PRODUCTS, redone)}
 
     def substep(self, seed: int, step_tot: int, northo: int, graph: bool = True):
         """One substep of the driver loop (miniafqmc_base.cpp:251-337)."""

@@ -342,15 +342,20 @@ cudaError_t body_dm(afq_handle* h, int want_gc, int save_old) {
 
 cudaError_t body_vbias(afq_handle* h) {
   if (h->mixed) return afq::mixed_vbias(h->mixed, h->Gc, h->vbias, h->st);
-  if (afq::oz_has_gsite(h->oz, afq::OZ_VBIAS))
-    return afq::oz_gsite(h->oz, afq::OZ_VBIAS, h->Gc, h->vbias, h->st);
+  OzGate gate;   // after a digit product: the FP64 pipe's form only where that does not hold
+  if (afq::oz_has_gsite(h->oz, afq::OZ_VBIAS)) {
+    const cudaError_t e = afq::oz_gsite(h->oz, afq::OZ_VBIAS, h->Gc, h->vbias, h->st);
+    if (e != cudaSuccess) return e;
+    gate = afq::oz_gate(h->oz, afq::OZ_VBIAS);
+  }
   if (h->spT_dense) {
     ZGemmDesc g{h->nc, h->nw, (int)h->NAK, h->spT_dense, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
+    g.gate = gate;
     EpiStore e{h->vbias, h->nw, 0, zmk(0, 0), 0};
     return zgemm_launch<true, true>(g, 1, e, h->st, h->f64cfg[afq_handle::F64_VBIAS]);
   }
   return launch_csr_gather(h->spT_ri, h->spT_ci, h->spT_v, h->Gc, h->NAK, h->nc, h->nw, h->vbias,
-                           h->st);
+                           h->st, gate);
 }
 
 cudaError_t body_sigma(afq_handle* h, int use_xraw) {
@@ -361,9 +366,10 @@ cudaError_t body_sigma(afq_handle* h, int use_xraw) {
 // vHS^T [w][ik] = sum_c X[c][w] Spvn[ik][c] with the dense Spvn: one ZGEMM of M = nw,
 // N = NMO^2, K = nchol writing each walker's matrix row by row (real x complex
 // multiply-adds when Spvn is real).
-cudaError_t dense_vhs(afq_handle* h, int cfg) {
+cudaError_t dense_vhs(afq_handle* h, int cfg, const OzGate& gate = OzGate()) {
   const long long NN = (long long)h->N * h->N;
-  ZGemmDesc g{h->nw, (int)NN, h->nc, h->X, h->nw, 0, h->sp_dense, h->nc, 0, zmk(1, 0)};
+  ZGemmDesc g{h->nw, (int)NN, h->nc, h->X, h->nw, 0, h->sp_dense, h->nc, 0, zmk(1, 0),
+              nullptr, gate};
   EpiStore ep{h->vHS, NN, 0, zmk(0, 0), 0};
   if (h->sp_dense_r) {
     g.Br = h->sp_dense_r;
@@ -374,18 +380,23 @@ cudaError_t dense_vhs(afq_handle* h, int cfg) {
 
 cudaError_t body_vhs(afq_handle* h) {
   if (h->mixed) return afq::mixed_vhs(h->mixed, h->X, h->vHS, h->st);
-  if (afq::oz_has_vhs(h->oz)) return afq::oz_vhs(h->oz, h->X, h->vHS, h->st);
-  if (h->sp_dense || h->sp_dense_r) return dense_vhs(h, h->vhsd_cfg);
+  OzGate gate;
+  if (afq::oz_has_vhs(h->oz)) {
+    const cudaError_t e = afq::oz_vhs(h->oz, h->X, h->vHS, h->st);
+    if (e != cudaSuccess) return e;
+    gate = afq::oz_gate(h->oz, afq::OZ_VHS);
+  }
+  if (h->sp_dense || h->sp_dense_r) return dense_vhs(h, h->vhsd_cfg, gate);
   return afq::launch_csr_walker(h->sp_ri, h->sp_ci, h->sp_v, h->sp_rv, h->X, h->N * h->N, h->nw,
                                 h->vHS, (long long)h->N * h->N, h->st,
-                                h->f64cfg[afq_handle::F64_VHS]);
+                                h->f64cfg[afq_handle::F64_VHS], gate);
 }
 
 cudaError_t body_propagate(afq_handle* h) {
   h->dm_cache = false;
   if (h->mixed) return afq::mixed_propagate(h->mixed, h->W, h->vHS, h->st);
   if (afq::oz_has_propagate(h->oz))
-    return afq::oz_propagate(h->oz, h->W, h->vHS, h->S, h->T1, h->st);
+    return afq::oz_propagate(h->oz, h->P, h->W, h->vHS, h->S, h->T1, h->T2, h->st);
   const int N = h->N, n2 = 2 * h->n, nw = h->nw;
   if (afq::prop_small_fits(N, n2, nw))
     return afq::launch_prop_small(h->P, h->vHS, h->W, N, n2, nw, h->d.taylor_order, h->st);
@@ -430,9 +441,14 @@ cudaError_t body_ortho(afq_handle* h) {
 
 // The Coulomb vector of every walker, cvec [nchol][nw] (FP64 form).
 cudaError_t fp64_coulomb(afq_handle* h, int cfg) {
-  if (afq::oz_has_gsite(h->oz, afq::OZ_COULOMB))
-    return afq::oz_gsite(h->oz, afq::OZ_COULOMB, h->Gc, h->cvec, h->st);
-  ZGemmDesc g{h->nc, h->nw, (int)h->NAK, h->Lh, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
+  OzGate gate;
+  if (afq::oz_has_gsite(h->oz, afq::OZ_COULOMB)) {
+    const cudaError_t e = afq::oz_gsite(h->oz, afq::OZ_COULOMB, h->Gc, h->cvec, h->st);
+    if (e != cudaSuccess) return e;
+    gate = afq::oz_gate(h->oz, afq::OZ_COULOMB);
+  }
+  ZGemmDesc g{h->nc, h->nw, (int)h->NAK, h->Lh, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0), nullptr,
+              gate};
   EpiStore ep{h->cvec, h->nw, 0, zmk(0, 0), 0};
   return zgemm_launch<true, true>(g, 1, ep, h->st, cfg);
 }
@@ -440,27 +456,36 @@ cudaError_t fp64_coulomb(afq_handle* h, int cfg) {
 // FP64 exchange partial sums of m walkers: int8 tensor cores where set up, else the FP64
 // pipe (h->nblk follows the choice).
 cudaError_t fp64_exchange(afq_handle* h, const z_t* G, int m, z_t* Kpart) {
-  if (afq::oz_has_exchange(h->oz, m)) return afq::oz_exchange(h->oz, G, m, Kpart, h->nblk, h->st);
+  const int* gate = nullptr;
+  if (afq::oz_has_exchange(h->oz, m)) {
+    const cudaError_t e = afq::oz_exchange(h->oz, G, m, Kpart, h->nblk, h->st);
+    if (e != cudaSuccess) return e;
+    gate = afq::oz_exchange_gate(h->oz);
+  }
   int nb = 0;
-  return afq::launch_exchange(h->Lh, G, h->N, h->n, h->nc, m, Kpart, &nb, h->st);
+  return afq::launch_exchange(h->Lh, G, h->N, h->n, h->nc, m, Kpart, &nb, h->st, gate, h->nblk);
 }
 
 cudaError_t body_energy(afq_handle* h, int mode) {
   cudaError_t e;
   const int nak = (int)h->NAK;
   if (mode == AFQ_ENERGY_VAKBL) {
+    OzGate gate;
     if (afq::oz_has_gsite(h->oz, afq::OZ_VAKBL)) {
       if ((e = afq::oz_gsite(h->oz, afq::OZ_VAKBL, h->Gc, h->Gcloc, h->st)) != cudaSuccess)
         return e;
-    } else if (h->vk_dense) {
-      ZGemmDesc g{nak, h->nw, nak, h->vk_dense, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0)};
+      gate = afq::oz_gate(h->oz, afq::OZ_VAKBL);
+    }
+    if (h->vk_dense) {
+      ZGemmDesc g{nak, h->nw, nak, h->vk_dense, h->NAK, 0, h->Gc, h->NAK, 0, zmk(1, 0), nullptr,
+                  gate};
       EpiStore ep{h->Gcloc, h->nw, 0, zmk(0, 0), 0};
       if ((e = zgemm_launch<true, true>(g, 1, ep, h->st, h->f64cfg[afq_handle::F64_VAKBL])) !=
           cudaSuccess)
         return e;
     } else {
       if ((e = launch_csr_gather(h->vk_ri, h->vk_ci, h->vk_v, h->Gc, h->NAK, nak, h->nw, h->Gcloc,
-                                 h->st)) != cudaSuccess)
+                                 h->st, gate)) != cudaSuccess)
         return e;
     }
     if ((e = afq::launch_energy_reduce(h->Gc, h->haj, nak, h->Gcloc, nullptr, 0, nullptr, 0, h->nw,
@@ -490,14 +515,14 @@ cudaError_t st_dm(afq_handle* h, int want_gc, int save_old) {
 }
 cudaError_t st_vbias(afq_handle* h) {
   int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VBIAS)
-           : afq::oz_has_gsite(h->oz, afq::OZ_VBIAS) ? afq::oz_gsite_launches(h->oz, afq::OZ_VBIAS) : 1;
+           : afq::oz_has_gsite(h->oz, afq::OZ_VBIAS) ? afq::oz_gsite_launches() + 1 : 1;
   return staged(h, AFQ_STAGE_VBIAS, nl, [&] { return body_vbias(h); });
 }
 cudaError_t st_sigma(afq_handle* h, int use_xraw) {
   return staged(h, AFQ_STAGE_SIGMA, 1, [&] { return body_sigma(h, use_xraw); });
 }
 cudaError_t st_vhs(afq_handle* h) {
-  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VHS) : afq::oz_has_vhs(h->oz) ? 2 : 1;
+  int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_VHS) : afq::oz_has_vhs(h->oz) ? 3 : 1;
   return staged(h, AFQ_STAGE_VHS, nl, [&] { return body_vhs(h); });
 }
 cudaError_t st_propagate(afq_handle* h) {
@@ -515,10 +540,10 @@ cudaError_t st_ortho(afq_handle* h) {
 }
 cudaError_t st_energy(afq_handle* h, int mode) {
   const int site = mode == AFQ_ENERGY_VAKBL ? afq::OZ_VAKBL : afq::OZ_COULOMB;
-  int nl = 2 + (afq::oz_has_gsite(h->oz, site) ? afq::oz_gsite_launches(h->oz, site) : 1);
+  int nl = 2 + (afq::oz_has_gsite(h->oz, site) ? afq::oz_gsite_launches() + 1 : 1);
   if (mode != AFQ_ENERGY_VAKBL)
     nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_ENERGY) + 2
-                  : nl + (afq::oz_has_exchange(h->oz, h->nw) ? afq::oz_exchange_launches(h->oz, h->nw) : 1);
+                  : nl + (afq::oz_has_exchange(h->oz, h->nw) ? afq::oz_exchange_launches(h->oz, h->nw) + 1 : 1);
   return staged(h, AFQ_STAGE_ENERGY, nl, [&] { return body_energy(h, mode); });
 }
 
@@ -1818,12 +1843,21 @@ afq_status afq_get_sparse_paths(afq_handle* h, int* path, double* ms) {
   return AFQ_OK;
 }
 
-afq_status afq_get_digit_products(afq_handle* h, int* on) {
+afq_status afq_get_digit_products(afq_handle* h, int* on, long long* redone) {
   if (!h || !on) return AFQ_ERR_ARG;
   for (int i = 0; i < afq::OZ_NG; i++) on[i] = afq::oz_has_gsite(h->oz, i);
   on[3] = afq::oz_has_vhs(h->oz);
   on[4] = afq::oz_has_propagate(h->oz);
   on[5] = afq::oz_has_exchange(h->oz, h->nw);
+  if (redone) {
+    unsigned long long n[afq::OZ_NPRODUCTS] = {};
+    if (h->oz) {
+      cudaSetDevice(h->d.device);
+      AFQ_CUDA(h, cudaStreamSynchronize(h->st));
+      AFQ_CUDA(h, afq::oz_redone(h->oz, n));
+    }
+    for (int i = 0; i < afq::OZ_NPRODUCTS; i++) redone[i] = (long long)n[i];
+  }
   return AFQ_OK;
 }
 

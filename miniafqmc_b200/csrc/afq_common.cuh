@@ -69,6 +69,30 @@ inline cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t 
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// Launch of the FP64 pipe's form of a product after its digit form (oz_gemm.cuh): the kernel
+// returns at once when every mark of the digit form's columns is set and no wait timed out,
+// which is all but always.  Read by each CTA itself (32 bytes per 16 walkers): a launch of its
+// own for the verdict cost 3 us.  The default opens.
+struct OzGate {
+  const uint4* ok = nullptr;    // n16 groups of 16 marks
+  int n16 = 0;
+  const int* err = nullptr;
+  unsigned long long* redone = nullptr;   // += walkers by an open gate
+  int walkers = 0;
+};
+AFQ_D bool oz_gate_open(const OzGate& g) {
+  if (!g.ok) return true;
+  bool bad = *g.err != 0;
+  for (int i = threadIdx.x; i < g.n16; i += blockDim.x) {
+    const uint4 v = g.ok[i];
+    bad |= (v.x & v.y & v.z & v.w) != 0x01010101u;
+  }
+  bad = __syncthreads_or(bad);
+  if (bad && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+    *g.redone += g.walkers;
+  return bad;
+}
+
 AFQ_HD z_t zmk(double r, double i) { return make_double2(r, i); }
 AFQ_HD z_t zadd(z_t a, z_t b) { return make_double2(a.x + b.x, a.y + b.y); }
 AFQ_HD z_t zsub(z_t a, z_t b) { return make_double2(a.x - b.x, a.y - b.y); }

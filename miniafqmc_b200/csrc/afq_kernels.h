@@ -16,10 +16,12 @@ cudaError_t launch_sigma(const z_t* vbias, z_t* X, double* xraw, z_t* hybridW, i
 constexpr int kCsrWalkerCfgs = 7;
 cudaError_t launch_csr_walker(const int* rowIndex, const int* cols, const z_t* zvals,
                               const double* rvals, const z_t* B, int nrows, int nw, z_t* out,
-                              long long out_ld, cudaStream_t st, int cfg = 0);
+                              long long out_ld, cudaStream_t st, int cfg = 0,
+                              const OzGate& gate = OzGate());
 const char* csr_walker_cfg_name(int cfg);
 cudaError_t launch_csr_gather(const int* rowIndex, const int* cols, const z_t* vals, const z_t* G,
-                              long long ldg, int nrows, int nw, z_t* out, cudaStream_t st);
+                              long long ldg, int nrows, int nw, z_t* out, cudaStream_t st,
+                              const OzGate& gate = OzGate());
 cudaError_t launch_weights(z_t* Wd, const z_t* hybridW, int nw, double dt, DevScalars* sc,
                            int update_eshift, cudaStream_t st);
 cudaError_t launch_set_scalars(DevScalars* sc, unsigned long long seed, unsigned long long step,
@@ -37,8 +39,11 @@ cudaError_t launch_prop_small(const z_t* P, const z_t* V, z_t* W, int N, int n2,
 cudaError_t launch_walker_layout(const z_t* src, z_t* dst, int N, int n, int nw, int to_ref,
                                  cudaStream_t st);
 size_t exch_smem_bytes();
+// Partial sums per (walker, spin, block of Cholesky vectors), Kpart[nw][2][stride] (0: *nblk_out,
+// the blocks; zeros past them).  gate [nw]: only walkers with a non-zero entry.
 cudaError_t launch_exchange(const z_t* Lh, const z_t* Gc, int N, int n, int nchol, int nw,
-                            z_t* Kpart, int* nblk_out, cudaStream_t st);
+                            z_t* Kpart, int* nblk_out, cudaStream_t st, const int* gate = nullptr,
+                            int stride = 0);
 cudaError_t launch_energy_reduce(const z_t* Gc, const z_t* haj, int nak, const z_t* Gcloc,
                                  const z_t* cv, int nchol, const z_t* Kpart, int nblk, int nw,
                                  int mode, z_t* Wd, double* parts, cudaStream_t st);

@@ -259,79 +259,91 @@ cudaError_t launch_sigma(const z_t* vbias, z_t* X, double* xraw, z_t* hybridW, i
 // stages its [rows x walkers] results in shared memory and writes them walker-major.
 // ROWS warps (rows) per CTA, WPL walkers per lane (CTA covers 32 WPL walkers); the set-up
 // tuner picks the shape (every shape sums each output in CSR order: same results).
-template <bool REALV, int ROWS, int WPL>
+// GATED: the form after a digit product, a few CTAs that loop over the rows (one CTA per row
+// group took 50 us to return at once at 384 orbitals; the loop costs the plain form 7 of 91 us
+// at 128 orbitals, 256 walkers).
+template <bool REALV, int ROWS, int WPL, bool GATED>
 __global__ void __launch_bounds__(ROWS * 32)
 csr_walker_kernel(const int* __restrict__ rowIndex, const int* __restrict__ cols,
                   const z_t* __restrict__ zvals, const double* __restrict__ rvals,
                   const z_t* __restrict__ B, int nrows, int nw, z_t* __restrict__ out,
-                  long long out_ld) {
+                  long long out_ld, OzGate gate) {
   pdl_trigger();
   pdl_wait();
+  if (GATED && !oz_gate_open(gate)) return;
   constexpr int WALK = 32 * WPL;
   __shared__ z_t tile[ROWS][WALK + 1];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * ROWS, r = r0 + wy;
   const int w0 = blockIdx.y * WALK;
-  z_t acc[WPL];
+  for (int r0 = blockIdx.x * ROWS; r0 < nrows; r0 += gridDim.x * ROWS) {
+    const int r = r0 + wy;
+    z_t acc[WPL];
 #pragma unroll
-  for (int j = 0; j < WPL; j++) acc[j] = zmk(0, 0);
-  if (r < nrows) {
-    const int beg = rowIndex[r], end = rowIndex[r + 1];
-    for (int p0 = beg; p0 < end; p0 += 32) {
-      const int cnt = min(32, end - p0);
-      int myc = 0;
-      z_t myv = zmk(0, 0);
-      double myr = 0.0;
-      if (lane < cnt) {
-        myc = cols[p0 + lane];
-        if (REALV) myr = rvals[p0 + lane];
-        else myv = zvals[p0 + lane];
-      }
-      for (int q = 0; q < cnt; q++) {
-        const int c = __shfl_sync(0xffffffffu, myc, q);
-        const z_t* br = B + (long long)c * nw;
-        if (REALV) {
-          const double v = __shfl_sync(0xffffffffu, myr, q);
+    for (int j = 0; j < WPL; j++) acc[j] = zmk(0, 0);
+    if (r < nrows) {
+      const int beg = rowIndex[r], end = rowIndex[r + 1];
+      for (int p0 = beg; p0 < end; p0 += 32) {
+        const int cnt = min(32, end - p0);
+        int myc = 0;
+        z_t myv = zmk(0, 0);
+        double myr = 0.0;
+        if (lane < cnt) {
+          myc = cols[p0 + lane];
+          if (REALV) myr = rvals[p0 + lane];
+          else myv = zvals[p0 + lane];
+        }
+        for (int q = 0; q < cnt; q++) {
+          const int c = __shfl_sync(0xffffffffu, myc, q);
+          const z_t* br = B + (long long)c * nw;
+          if (REALV) {
+            const double v = __shfl_sync(0xffffffffu, myr, q);
 #pragma unroll
-          for (int j = 0; j < WPL; j++) {
-            const int w = w0 + 32 * j + lane;
-            if (w < nw) zfma_r(acc[j], v, br[w]);
-          }
-        } else {
-          z_t v;
-          v.x = __shfl_sync(0xffffffffu, myv.x, q);
-          v.y = __shfl_sync(0xffffffffu, myv.y, q);
+            for (int j = 0; j < WPL; j++) {
+              const int w = w0 + 32 * j + lane;
+              if (w < nw) zfma_r(acc[j], v, br[w]);
+            }
+          } else {
+            z_t v;
+            v.x = __shfl_sync(0xffffffffu, myv.x, q);
+            v.y = __shfl_sync(0xffffffffu, myv.y, q);
 #pragma unroll
-          for (int j = 0; j < WPL; j++) {
-            const int w = w0 + 32 * j + lane;
-            if (w < nw) zfma(acc[j], v, br[w]);
+            for (int j = 0; j < WPL; j++) {
+              const int w = w0 + 32 * j + lane;
+              if (w < nw) zfma(acc[j], v, br[w]);
+            }
           }
         }
       }
     }
-  }
 #pragma unroll
-  for (int j = 0; j < WPL; j++) tile[wy][32 * j + lane] = acc[j];
-  __syncthreads();
-  for (int e = threadIdx.x; e < ROWS * WALK; e += ROWS * 32) {
-    const int wl = e / ROWS, rr = e % ROWS;
-    const int w = w0 + wl, rw = r0 + rr;
-    if (w < nw && rw < nrows) out[(long long)w * out_ld + rw] = tile[rr][wl];
+    for (int j = 0; j < WPL; j++) tile[wy][32 * j + lane] = acc[j];
+    __syncthreads();
+    for (int e = threadIdx.x; e < ROWS * WALK; e += ROWS * 32) {
+      const int wl = e / ROWS, rr = e % ROWS;
+      const int w = w0 + wl, rw = r0 + rr;
+      if (w < nw && rw < nrows) out[(long long)w * out_ld + rw] = tile[rr][wl];
+    }
+    if constexpr (!GATED) break;
+    __syncthreads();   // the next rows reuse the tile
   }
 }
 
 template <int ROWS, int WPL>
 cudaError_t csr_walker_launch(const int* rowIndex, const int* cols, const z_t* zvals,
                               const double* rvals, const z_t* B, int nrows, int nw, z_t* out,
-                              long long out_ld, cudaStream_t st) {
+                              long long out_ld, cudaStream_t st, const OzGate& gate) {
   dim3 grid((nrows + ROWS - 1) / ROWS, (nw + 32 * WPL - 1) / (32 * WPL));
-  if (rvals)
-    pdl_launch(csr_walker_kernel<true, ROWS, WPL>, grid, ROWS * 32, 0, st, rowIndex, cols, nullptr, rvals,
-                                                                   B, nrows, nw, out, out_ld);
-  else
-    pdl_launch(csr_walker_kernel<false, ROWS, WPL>, grid, ROWS * 32, 0, st, rowIndex, cols, zvals, nullptr,
-                                                                    B, nrows, nw, out, out_ld);
-  return cudaGetLastError();
+  if (gate.ok) {
+    grid.x = std::min(grid.x, 8u * 148u);
+    return rvals ? pdl_launch(csr_walker_kernel<true, ROWS, WPL, true>, grid, ROWS * 32, 0, st,
+                              rowIndex, cols, nullptr, rvals, B, nrows, nw, out, out_ld, gate)
+                 : pdl_launch(csr_walker_kernel<false, ROWS, WPL, true>, grid, ROWS * 32, 0, st,
+                              rowIndex, cols, zvals, nullptr, B, nrows, nw, out, out_ld, gate);
+  }
+  return rvals ? pdl_launch(csr_walker_kernel<true, ROWS, WPL, false>, grid, ROWS * 32, 0, st,
+                            rowIndex, cols, nullptr, rvals, B, nrows, nw, out, out_ld, gate)
+               : pdl_launch(csr_walker_kernel<false, ROWS, WPL, false>, grid, ROWS * 32, 0, st,
+                            rowIndex, cols, zvals, nullptr, B, nrows, nw, out, out_ld, gate);
 }
 
 const char* csr_walker_cfg_name(int cfg) {
@@ -343,15 +355,15 @@ const char* csr_walker_cfg_name(int cfg) {
 // cfg: 0 built-in (16 rows x 2 walkers per lane), 1..kCsrWalkerCfgs the shapes above
 cudaError_t launch_csr_walker(const int* rowIndex, const int* cols, const z_t* zvals,
                               const double* rvals, const z_t* B, int nrows, int nw, z_t* out,
-                              long long out_ld, cudaStream_t st, int cfg) {
+                              long long out_ld, cudaStream_t st, int cfg, const OzGate& gate) {
   switch (cfg) {
-    case 2: return csr_walker_launch<8, 2>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
-    case 3: return csr_walker_launch<4, 2>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
-    case 4: return csr_walker_launch<16, 1>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
-    case 5: return csr_walker_launch<8, 4>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
-    case 6: return csr_walker_launch<4, 4>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
-    case 7: return csr_walker_launch<32, 1>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
-    default: return csr_walker_launch<16, 2>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st);
+    case 2: return csr_walker_launch<8, 2>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
+    case 3: return csr_walker_launch<4, 2>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
+    case 4: return csr_walker_launch<16, 1>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
+    case 5: return csr_walker_launch<8, 4>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
+    case 6: return csr_walker_launch<4, 4>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
+    case 7: return csr_walker_launch<32, 1>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
+    default: return csr_walker_launch<16, 2>(rowIndex, cols, zvals, rvals, B, nrows, nw, out, out_ld, st, gate);
   }
 }
 
@@ -361,7 +373,10 @@ cudaError_t launch_csr_walker(const int* rowIndex, const int* cols, const z_t* z
 __global__ void __launch_bounds__(256)
 csr_gather_kernel(const int* __restrict__ rowIndex, const int* __restrict__ cols,
                   const z_t* __restrict__ vals, const z_t* __restrict__ G, long long ldg,
-                  int nrows, int nw, z_t* __restrict__ out) {
+                  int nrows, int nw, z_t* __restrict__ out, OzGate gate) {
+  pdl_trigger();
+  pdl_wait();
+  if (!oz_gate_open(gate)) return;
   const int lane = threadIdx.x & 31;
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= nrows) return;
@@ -387,9 +402,10 @@ csr_gather_kernel(const int* __restrict__ rowIndex, const int* __restrict__ cols
 }
 
 cudaError_t launch_csr_gather(const int* rowIndex, const int* cols, const z_t* vals, const z_t* G,
-                              long long ldg, int nrows, int nw, z_t* out, cudaStream_t st) {
-  csr_gather_kernel<<<(nrows + 7) / 8, 256, 0, st>>>(rowIndex, cols, vals, G, ldg, nrows, nw, out);
-  return cudaGetLastError();
+                              long long ldg, int nrows, int nw, z_t* out, cudaStream_t st,
+                              const OzGate& gate) {
+  return pdl_launch(csr_gather_kernel, (nrows + 7) / 8, 256, 0, st, rowIndex, cols, vals, G, ldg,
+                    nrows, nw, out, gate);
 }
 
 // ============================================================ weights
@@ -1114,93 +1130,109 @@ size_t exch_smem_bytes() {
 
 __global__ void __launch_bounds__(EX_THREADS)
 exchange_kernel(const z_t* __restrict__ Lh, const z_t* __restrict__ Gc, int N, int n, int nchol,
-                int nw, int Gn, int Gw, z_t* __restrict__ Kpart, int nblk) {
+                int nw, int Gn, int Gw, z_t* __restrict__ Kpart, int nblk,
+                const int* __restrict__ gate) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char ex_smem[];
   z_t* As = reinterpret_cast<z_t*>(ex_smem);          // [2][BK][T+1]
   z_t* Bs = As + 2 * EX_BK * (EX_T + 1);
   const int s = blockIdx.z;
-  const int c0 = blockIdx.x * Gn, w0 = blockIdx.y * Gw;
+  const int c0 = blockIdx.x * Gn;
   const long long NAK = 2LL * n * N;
   const int Mr = Gn * n, Nc = Gw * n;
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
 
-  auto load = [&](int stage, int k0) {
-    z_t* as = As + stage * EX_BK * (EX_T + 1);
-    z_t* bs = Bs + stage * EX_BK * (EX_T + 1);
-    for (int e = tid; e < EX_T * EX_BK; e += EX_THREADS) {
-      int m = e / EX_BK, k = e % EX_BK, gk = k0 + k;
-      int cv = m / n, a = m % n;
-      const z_t* src = Lh;
-      int bytes = 0;
-      if (m < Mr && c0 + cv < nchol && gk < N) {
-        src = Lh + (long long)(c0 + cv) * NAK + (long long)s * n * N + (long long)a * N + gk;
-        bytes = 16;
-      }
-      cp_async16(as + k * (EX_T + 1) + m, src, bytes);
-      const z_t* srcb = Gc;
-      int bb = 0;
-      if (m < Nc && w0 + m / n < nw && gk < N) {
-        int wl = m / n, b = m % n;
-        srcb = Gc + (long long)(w0 + wl) * NAK + (long long)s * n * N + (long long)b * N + gk;
-        bb = 16;
-      }
-      cp_async16(bs + k * (EX_T + 1) + m, srcb, bb);
+  for (int w0 = blockIdx.y * Gw; w0 < nw; w0 += gridDim.y * Gw) {
+    if (gate) {   // uniform
+      bool any = false;
+      for (int w = w0; w < min(nw, w0 + Gw); w++) any |= gate[w] != 0;
+      if (!any) continue;
     }
-    cp_async_commit();
-  };
+    auto load = [&](int stage, int k0) {
+      z_t* as = As + stage * EX_BK * (EX_T + 1);
+      z_t* bs = Bs + stage * EX_BK * (EX_T + 1);
+      for (int e = tid; e < EX_T * EX_BK; e += EX_THREADS) {
+        int m = e / EX_BK, k = e % EX_BK, gk = k0 + k;
+        int cv = m / n, a = m % n;
+        const z_t* src = Lh;
+        int bytes = 0;
+        if (m < Mr && c0 + cv < nchol && gk < N) {
+          src = Lh + (long long)(c0 + cv) * NAK + (long long)s * n * N + (long long)a * N + gk;
+          bytes = 16;
+        }
+        cp_async16(as + k * (EX_T + 1) + m, src, bytes);
+        const z_t* srcb = Gc;
+        int bb = 0;
+        if (m < Nc && w0 + m / n < nw && gk < N) {
+          int wl = m / n, b = m % n;
+          srcb = Gc + (long long)(w0 + wl) * NAK + (long long)s * n * N + (long long)b * N + gk;
+          bb = 16;
+        }
+        cp_async16(bs + k * (EX_T + 1) + m, srcb, bb);
+      }
+      cp_async_commit();
+    };
 
-  z_t acc[EX_TM][EX_TN];
+    z_t acc[EX_TM][EX_TN];
 #pragma unroll
-  for (int i = 0; i < EX_TM; i++)
+    for (int i = 0; i < EX_TM; i++)
 #pragma unroll
-    for (int j = 0; j < EX_TN; j++) acc[i][j] = zmk(0, 0);
-  const int nk = (N + EX_BK - 1) / EX_BK;
-  load(0, 0);
-  for (int kt = 0; kt < nk; kt++) {
-    if (kt + 1 < nk) {
-      load((kt + 1) & 1, (kt + 1) * EX_BK);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    const z_t* as = As + (kt & 1) * EX_BK * (EX_T + 1);
-    const z_t* bs = Bs + (kt & 1) * EX_BK * (EX_T + 1);
-#pragma unroll 4
-    for (int kk = 0; kk < EX_BK; kk++) {
-      z_t a[EX_TM], b[EX_TN];
-#pragma unroll
-      for (int i = 0; i < EX_TM; i++) a[i] = as[kk * (EX_T + 1) + ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < EX_TN; j++) b[j] = bs[kk * (EX_T + 1) + tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < EX_TM; i++)
-#pragma unroll
-        for (int j = 0; j < EX_TN; j++) zfma(acc[i][j], a[i], b[j]);
-    }
-    __syncthreads();
-  }
-  z_t* Ts = reinterpret_cast<z_t*>(ex_smem);             // [T][T+1], reuses the slabs
-#pragma unroll
-  for (int i = 0; i < EX_TM; i++)
-#pragma unroll
-    for (int j = 0; j < EX_TN; j++) Ts[(ty + 16 * i) * (EX_T + 1) + tx + 16 * j] = acc[i][j];
-  __syncthreads();
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int wl = warp; wl < Gw; wl += EX_THREADS / 32) {
-    z_t sum = zmk(0, 0);
-    for (int cv = 0; cv < Gn; cv++)
-      for (int t = lane; t < n * n; t += 32) {
-        int a = t / n, b = t % n;
-        zfma(sum, Ts[(cv * n + a) * (EX_T + 1) + wl * n + b], Ts[(cv * n + b) * (EX_T + 1) + wl * n + a]);
+      for (int j = 0; j < EX_TN; j++) acc[i][j] = zmk(0, 0);
+    const int nk = (N + EX_BK - 1) / EX_BK;
+    load(0, 0);
+    for (int kt = 0; kt < nk; kt++) {
+      if (kt + 1 < nk) {
+        load((kt + 1) & 1, (kt + 1) * EX_BK);
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
       }
-    sum = warp_zsum(sum);
-    if (lane == 0 && w0 + wl < nw) Kpart[((long long)(w0 + wl) * 2 + s) * nblk + blockIdx.x] = sum;
+      __syncthreads();
+      const z_t* as = As + (kt & 1) * EX_BK * (EX_T + 1);
+      const z_t* bs = Bs + (kt & 1) * EX_BK * (EX_T + 1);
+#pragma unroll 4
+      for (int kk = 0; kk < EX_BK; kk++) {
+        z_t a[EX_TM], b[EX_TN];
+#pragma unroll
+        for (int i = 0; i < EX_TM; i++) a[i] = as[kk * (EX_T + 1) + ty + 16 * i];
+#pragma unroll
+        for (int j = 0; j < EX_TN; j++) b[j] = bs[kk * (EX_T + 1) + tx + 16 * j];
+#pragma unroll
+        for (int i = 0; i < EX_TM; i++)
+#pragma unroll
+          for (int j = 0; j < EX_TN; j++) zfma(acc[i][j], a[i], b[j]);
+      }
+      __syncthreads();
+    }
+    z_t* Ts = reinterpret_cast<z_t*>(ex_smem);             // [T][T+1], reuses the slabs
+#pragma unroll
+    for (int i = 0; i < EX_TM; i++)
+#pragma unroll
+      for (int j = 0; j < EX_TN; j++) Ts[(ty + 16 * i) * (EX_T + 1) + tx + 16 * j] = acc[i][j];
+    __syncthreads();
+    const int lane = tid & 31, warp = tid >> 5;
+    for (int wl = warp; wl < Gw; wl += EX_THREADS / 32) {
+      z_t sum = zmk(0, 0);
+      for (int cv = 0; cv < Gn; cv++)
+        for (int t = lane; t < n * n; t += 32) {
+          int a = t / n, b = t % n;
+          zfma(sum, Ts[(cv * n + a) * (EX_T + 1) + wl * n + b], Ts[(cv * n + b) * (EX_T + 1) + wl * n + a]);
+        }
+      sum = warp_zsum(sum);
+      if (w0 + wl < nw && (!gate || gate[w0 + wl])) {   // zeros past the Cholesky blocks, where nblk is a finer blocking's
+        z_t* k = Kpart + ((long long)(w0 + wl) * 2 + s) * nblk;
+        for (int q = blockIdx.x + lane * gridDim.x; q < nblk; q += 32 * gridDim.x)
+          k[q] = lane == 0 && q == blockIdx.x ? sum : zmk(0, 0);
+      }
+    }
+    __syncthreads();   // the next walkers' slabs reuse the tile
   }
 }
 
 cudaError_t launch_exchange(const z_t* Lh, const z_t* Gc, int N, int n, int nchol, int nw,
-                            z_t* Kpart, int* nblk_out, cudaStream_t st) {
+                            z_t* Kpart, int* nblk_out, cudaStream_t st, const int* gate,
+                            int stride) {
   if (n > EX_T) return cudaErrorInvalidValue;
   const int Gn = EX_T / n, Gw = EX_T / n;
   const int nblk = (nchol + Gn - 1) / Gn;
@@ -1213,9 +1245,10 @@ cudaError_t launch_exchange(const z_t* Lh, const z_t* Gc, int N, int n, int ncho
                                 (int)b);
   });
   if (e != cudaSuccess) return e;
-  dim3 grid(nblk, (nw + Gw - 1) / Gw, 2);
-  exchange_kernel<<<grid, EX_THREADS, smem, st>>>(Lh, Gc, N, n, nchol, nw, Gn, Gw, Kpart, nblk);
-  return cudaGetLastError();
+  // a gated launch mostly does nothing: few CTAs, each looping over the walker groups
+  dim3 grid(nblk, std::min((nw + Gw - 1) / Gw, gate ? 4 : 65535), 2);
+  return pdl_launch(exchange_kernel, grid, EX_THREADS, smem, st, Lh, Gc, N, n, nchol, nw, Gn, Gw,
+                    Kpart, stride ? stride : nblk, gate);
 }
 
 // ============================================================ energy reductions

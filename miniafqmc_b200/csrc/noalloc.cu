@@ -21,7 +21,7 @@ constexpr long long kMaxExchangePartials = 1LL << 18;
 static __device__ __align__(256) z_t g_exchange_scratch[kMaxExchangePartials];
 
 // Chunks of the digit products (oz.cu): 48 MiB of T (five waves of 64 KB output tiles), 24
-// MiB of G digits and 6 MiB of Lh digits with their row scales, loaded with this file's
+// MiB of G digits and 6 MiB of Lh digits with their row scales and norms, loaded with this file's
 // kernels by the first call on a device.  With 40 and 20 MiB, 96 walkers at 200 orbitals
 // split into two uneven chunks: 10.8 against 7.0 ms (28.0 ms on the FP64 pipe).
 constexpr size_t kTBytes = 48u << 20, kGBytes = 24u << 20, kABytes = 6u << 20;
@@ -29,8 +29,10 @@ constexpr int kGRows = 16384, kARows = 4096;
 struct Scratch {
   double T[kTBytes / 8];
   int8_t g[kGBytes], a[kABytes];
-  double g_scale[kGRows], a_scale[kARows];
+  double g_scale[2 * kGRows], a_scale[kARows];
   int flags[8];
+  double norms[kMaxExchangePartials], sa2[2];
+  int gate[kMaxExchangePartials / 2];
 };
 static __device__ __align__(256) Scratch g_oz_scratch;
 
@@ -41,9 +43,11 @@ Scratch* g_oz_addr[kMaxDevices] = {};
 
 // EK[w] = 1/2 sum over spins and Cholesky blocks of the partials, in a fixed order.
 __global__ void __launch_bounds__(128)
-exchange_finish_kernel(const z_t* __restrict__ part, int nblk, z_t* __restrict__ ek) {
-  __shared__ z_t red[4];
+exchange_finish_kernel(const z_t* __restrict__ part, int nblk, z_t* __restrict__ ek,
+                       const int* __restrict__ gate) {
   const int w = blockIdx.x;
+  if (gate && gate[w] == 0) return;
+  __shared__ z_t red[4];
   z_t s = zmk(0, 0);
   for (int q = threadIdx.x; q < 2 * nblk; q += blockDim.x)
     s = zadd(s, part[(long long)w * 2 * nblk + q]);
@@ -92,19 +96,22 @@ extern "C" afq_status afq_exchange_energy_noalloc(const double* Lh, const double
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const afq::OzBuffers b{oz->a, oz->g, kABytes, kGBytes, oz->a_scale, oz->g_scale, kARows, kGRows,
-                         oz->T, kTBytes, scratch, kMaxExchangePartials, oz->flags};
-  if (afq::oz_exchange_buffers_fit(b, nmo, naea, nchol, nwalk))
-    return afq::oz_exchange_buffers(b, reinterpret_cast<const z_t*>(Lh),
-                                    reinterpret_cast<const z_t*>(Gc), nmo, naea, nchol, nwalk,
-                                    reinterpret_cast<z_t*>(ek), st) == cudaSuccess
-               ? AFQ_OK
-               : AFQ_ERR_CUDA;
-  // the array keeps the previous call's contents: clear the part this call reads
-  if (cudaMemsetAsync(scratch, 0, sizeof(z_t) * used, st) != cudaSuccess) return AFQ_ERR_CUDA;
+                         oz->T, kTBytes, scratch, oz->norms, kMaxExchangePartials, oz->flags,
+                         oz->sa2, oz->gate};
+  const int* gate = nullptr;   // after the digit products: only what they leave to the FP64 pipe
+  if (afq::oz_exchange_buffers_fit(b, nmo, naea, nchol, nwalk)) {
+    if (afq::oz_exchange_buffers(b, reinterpret_cast<const z_t*>(Lh),
+                                 reinterpret_cast<const z_t*>(Gc), nmo, naea, nchol, nwalk,
+                                 reinterpret_cast<z_t*>(ek), st) != cudaSuccess)
+      return AFQ_ERR_CUDA;
+    gate = oz->gate;
+  } else if (cudaMemsetAsync(scratch, 0, sizeof(z_t) * used, st) != cudaSuccess) {
+    return AFQ_ERR_CUDA;   // the array keeps the previous call's contents
+  }
   int nb = 0;
   if (afq::launch_exchange(reinterpret_cast<const z_t*>(Lh), reinterpret_cast<const z_t*>(Gc), nmo,
-                           naea, nchol, nwalk, scratch, &nb, st) != cudaSuccess)
+                           naea, nchol, nwalk, scratch, &nb, st, gate) != cudaSuccess)
     return AFQ_ERR_CUDA;
-  exchange_finish_kernel<<<nwalk, 128, 0, st>>>(scratch, nb, reinterpret_cast<z_t*>(ek));
+  exchange_finish_kernel<<<nwalk, 128, 0, st>>>(scratch, nb, reinterpret_cast<z_t*>(ek), gate);
   return cudaGetLastError() == cudaSuccess ? AFQ_OK : AFQ_ERR_CUDA;
 }

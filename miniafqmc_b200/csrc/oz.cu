@@ -20,11 +20,17 @@ struct OzState {
   size_t block_left = 0;
   size_t free_left = 0;     // device memory not yet planned for
   int* err = nullptr;
+  // per product (OzProduct) the walkers whose result the digits did not hold; per walker
+  // whether the last exchange's did not, and whether the propagation's did not on the way
+  unsigned long long* redone = nullptr;
+  int *ex_gate = nullptr, *prop_bad = nullptr;
   // exchange: rows (c, a) of Lh per spin, columns (w, b, re | im) of G, T = Lh_c Gc_w^T of a
   // chunk of Cholesky vectors and walkers
   bool lreal = false;
   Slices lx[2], gx;
   double* T = nullptr;
+  double* norms = nullptr;  // half of |T|^2 per partial sum
+  double *sa2 = nullptr, *sb = nullptr;   // exchange_holds: of lx, of gx per spin
   int ex_w = 0, ex_c = 0;   // walkers and Cholesky vectors per chunk
   bool exchange = false;
   // products with G: static operand rows, G rows (w, re | im) shared by the sites, partial
@@ -73,14 +79,29 @@ cudaError_t oz_alloc(OzState* o, T** p, size_t count) {
   return e;
 }
 
-// Slices of `batch` x `rows` rows of K digits-worth of entries, in tiles of `tile` rows.
-cudaError_t alloc_slices(OzState* o, Slices* s, int tile, int rows, int batch, int K) {
+// Slices of `batch` x `rows` rows of K digits-worth of entries, in tiles of `tile` rows;
+// checked (Slices::top, Slices::ok) when `st` is given.
+struct Checked {
+  cudaStream_t st;
+};
+constexpr size_t ok_bytes(size_t rows) { return (rows + 15) / 16 * 16; }
+cudaError_t alloc_slices(OzState* o, Slices* s, int tile, int rows, int batch, int K,
+                         const Checked* checked = nullptr) {
   s->tile = tile;
   s->rows = rows;
   s->batch = batch;
   s->nslab = (K + oz::kSlab - 1) / oz::kSlab;
   cudaError_t e = oz_alloc(o, &s->d, s->bytes());
   if (e == cudaSuccess) e = oz_alloc(o, &s->scale, (size_t)rows * batch);
+  if (!checked || e != cudaSuccess) return e;
+  if (tile == oz::kBM) {
+    e = oz_alloc(o, &s->top, batch);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->top, 0, sizeof(double) * batch, checked->st);
+  } else {
+    const size_t bytes = ok_bytes((size_t)rows * batch);
+    e = oz_alloc(o, &s->ok, bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->ok, 1, bytes, checked->st);
+  }
   return e;
 }
 
@@ -106,7 +127,8 @@ AFQ_D RowScale row_scale(unsigned long long maxbits) {
   if (maxbits == 0) return r;
   const double mx = __longlong_as_double((long long)maxbits);
   int e;
-  if (maxbits >= 0x7FE0000000000000ull) {   // inf, nan, or 2^e beyond the range
+  // inf, nan, or a scale whose products could leave the range (2^900, 2^-900)
+  if (maxbits >= 0x7830000000000000ull || maxbits < 0x07B0000000000000ull) {
     r.scale = __longlong_as_double(0x7ff8000000000000LL);
     return r;
   }
@@ -210,11 +232,37 @@ AFQ_D void row_max(const z_t* __restrict__ p, int k0, int k1, int t, int nt,
     m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
   }
 }
+// The check of a product whose result columns are sliced as the next one's operand (rows of
+// `per` a batch): column r, whose largest entry is factor^-1 times the product's, against
+// kFloor x (largest A scale) x (its own B scale old[2r], old[2r + 1]); bad [batch].
+struct RowCheck {
+  const double* top = nullptr;
+  int batched = 0, per = 1;
+  const double* old = nullptr;
+  double factor = 1.0;
+  int* bad = nullptr;
+};
+AFQ_D void check_row(const RowCheck& c, int r, unsigned long long maxbits) {
+  if (!c.top) return;
+  const int z = r / c.per;
+  const double lim = oz::kFloor * c.top[c.batched ? z : 0] * fmax(c.old[2 * r], c.old[2 * r + 1]);
+  if (!(c.factor * __longlong_as_double((long long)maxbits) >= lim)) c.bad[z] = 1;   // NaN: bad
+}
+// The row's scale and its mark: a zero row is ok as it is.
+AFQ_D void put_scale(const Slices& s, long long i, double scale) {
+  if (s.ok) {
+    s.ok[i] = scale == 0.0;
+  }
+  s.scale[i] = scale;
+}
 template <int MODE>
 AFQ_D void put_scales(const Slices& s, int rb, int r0, const RowScale& s0, const RowScale& s1) {
-  double* sc = s.scale + (long long)rb * s.rows + r0;
-  sc[0] = s0.scale;
-  if constexpr (MODE == kSplitRe || MODE == kSplitCx) sc[1] = s1.scale;
+  const long long i = (long long)rb * s.rows + r0;
+  put_scale(s, i, s0.scale);
+  if constexpr (MODE == kSplitRe || MODE == kSplitCx) put_scale(s, i + 1, s1.scale);
+  if (s.top)   // non-negative scales (and NaN above them) order like their bits
+    atomicMax(reinterpret_cast<unsigned long long*>(s.top + rb),
+              (unsigned long long)__double_as_longlong(s0.scale));
 }
 AFQ_D const z_t* src_row(const RowSrc& src, int r, bool dbl) {
   if (!dbl) return src.row(r);
@@ -226,7 +274,7 @@ AFQ_D const z_t* src_row(const RowSrc& src, int r, bool dbl) {
 // L2).  Memory bound: 16 bytes read per complex entry, 14 (28 for kSplitCx) written.
 template <int MODE>
 __global__ void __launch_bounds__(256)
-slice_kernel(RowSrc src, int nrows, int K, Slices s) {
+slice_kernel(RowSrc src, int nrows, int K, Slices s, RowCheck chk) {
   pdl_trigger();
   pdl_wait();
   constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
@@ -235,6 +283,7 @@ slice_kernel(RowSrc src, int nrows, int K, Slices s) {
   const z_t* p = src_row(src, r, MODE == kDouble);
   unsigned long long m0, m1;
   row_max<MODE>(p, 0, K, lane, 32, m0, m1);
+  if (lane == 0) check_row(chk, r, max(m0, m1));
   if constexpr (MODE == kPairs || MODE == kSplitCx) m0 = m1 = max(m0, m1);
   const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
   const int rb = r / s.per_batch(TWO), r0 = (r - rb * s.per_batch(TWO)) * (TWO ? 2 : 1);
@@ -247,7 +296,7 @@ slice_kernel(RowSrc src, int nrows, int K, Slices s) {
 constexpr int kSliceCluster = 8;
 template <int MODE>
 __global__ void __cluster_dims__(kSliceCluster, 1, 1) __launch_bounds__(256)
-slice_cluster_kernel(RowSrc src, int K, Slices s) {
+slice_cluster_kernel(RowSrc src, int K, Slices s, RowCheck chk) {
   pdl_trigger();
   pdl_wait();
   constexpr bool TWO = MODE == kSplitRe || MODE == kSplitCx;
@@ -281,6 +330,7 @@ slice_cluster_kernel(RowSrc src, int K, Slices s) {
     m1 = max(m1, o[1]);
   }
   cl.sync();   // every CTA's shared memory stays until all have read it
+  if (part == 0 && threadIdx.x == 0) check_row(chk, r, max(m0, m1));
   if constexpr (PAIR) m0 = m1 = max(m0, m1);
   const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
   const int rb = r / s.per_batch(TWO), r0 = (r - rb * s.per_batch(TWO)) * (TWO ? 2 : 1);
@@ -291,13 +341,12 @@ slice_cluster_kernel(RowSrc src, int K, Slices s) {
 // Slices nrows source rows of K entries into `s` (its first rows).  Rows above 1024 entries
 // get a cluster each (16 rows of 2048 entries at one warp a row would fill two SMs).
 template <int MODE>
-cudaError_t slice_rows(const RowSrc& src, int nrows, int K, const Slices& s, cudaStream_t st) {
+cudaError_t slice_rows(const RowSrc& src, int nrows, int K, const Slices& s, cudaStream_t st,
+                       const RowCheck& chk = RowCheck()) {
   if (nrows <= 0) return cudaSuccess;
   if (K > 1024)
-    pdl_launch(slice_cluster_kernel<MODE>, nrows * kSliceCluster, 256, 0, st, src, K, s);
-  else
-    pdl_launch(slice_kernel<MODE>, (nrows + 7) / 8, 256, 0, st, src, nrows, K, s);
-  return cudaGetLastError();
+    return pdl_launch(slice_cluster_kernel<MODE>, nrows * kSliceCluster, 256, 0, st, src, K, s, chk);
+  return pdl_launch(slice_kernel<MODE>, (nrows + 7) / 8, 256, 0, st, src, nrows, K, s, chk);
 }
 
 // Rows of an A operand (TWO = false: one row of reals, or of pairs) or of a B operand (re and
@@ -367,8 +416,8 @@ slice_x_kernel(const z_t* __restrict__ X, int nc, int nw, Slices s) {
   if (!REALA) m0 = m1 = max(m0, m1);
   const RowScale s0 = row_scale(m0), s1 = row_scale(m1);
   if (part == 0 && wy == 0) {
-    s.scale[2 * w] = s0.scale;
-    s.scale[2 * w + 1] = s1.scale;
+    put_scale(s, 2 * w, s0.scale);
+    put_scale(s, 2 * w + 1, s1.scale);
   }
   const int plane = s.tile * oz::kSlab, Kp = s.nslab * oz::kSlab;
   constexpr int NE = REALA ? 16 : 8;   // source entries per 16 digits
@@ -405,11 +454,16 @@ slice_x_kernel(const z_t* __restrict__ X, int nc, int nw, Slices s) {
   }
 }
 
-// W [nw][N][n2] -> Wt [nw][n2][N]
+// W [nw][N][n2] -> Wt [nw][n2][N]; clears top [nw] and bad [nw].
 __global__ void __launch_bounds__(256)
-transpose_kernel(const z_t* __restrict__ W, int N, int n2, z_t* __restrict__ Wt) {
+transpose_kernel(const z_t* __restrict__ W, int N, int n2, z_t* __restrict__ Wt, double* top,
+                 int* bad) {
   pdl_trigger();
   pdl_wait();
+  if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) {
+    top[blockIdx.z] = 0.0;
+    bad[blockIdx.z] = 0;
+  }
   __shared__ z_t t[32][33];
   const int w = blockIdx.z, k0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   const z_t* src = W + (long long)w * N * n2;
@@ -530,35 +584,113 @@ struct EpiW {
       if (j0 + i / 2 < n2) oz::store4(p + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
   }
 };
-// out[r][w] = sum over the K splits of the partial products, in order.
+// out[r][w] = sum over the K splits of the partial products, in order; marks of B's rows
+// (w, re | im) as in oz_gemm_kernel.  `lanes` (a power of two up to 32) walkers by 256 / lanes
+// rows per CTA and pass, so that a thread keeps its walker and a CTA writes each mark once: all
+// CTAs write the same few lines, and one store per element made 1536 x 128 sums take 165 us
+// longer.
 __global__ void __launch_bounds__(256)
 part_sum_kernel(const double* __restrict__ part, long long ld, long long sz, int splits, int rows,
-                int nw, z_t* __restrict__ out) {
+                int nw, int lanes, z_t* __restrict__ out, const double* __restrict__ top,
+                Slices b) {
   pdl_trigger();
   pdl_wait();
-  const long long tot = (long long)rows * nw;
-  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < tot; e += gridDim.x * 256LL) {
-    const long long r = e / nw, w = e - r * nw;
-    const z_t* p = reinterpret_cast<const z_t*>(part + r * ld) + w;
-    z_t t = p[0];
-    for (int q = 1; q < splits; q++) t = zadd(t, p[q * (sz / 2)]);
-    out[e] = t;
+  __shared__ unsigned char mark[64];
+  if (threadIdx.x < 64) mark[threadIdx.x] = 0;
+  __syncthreads();
+  const int wl = threadIdx.x % lanes, w0 = blockIdx.y * lanes, w = w0 + wl, rpb = 256 / lanes;
+  if (w < nw) {
+    const double lim = oz::kFloor * *top;
+    const double lre = lim * b.scale[2 * w], lim_im = lim * b.scale[2 * w + 1];
+    bool re = false, im = false;   // NaN marks nothing
+    for (int r = blockIdx.x * rpb + threadIdx.x / lanes; r < rows; r += gridDim.x * rpb) {
+      const z_t* p = reinterpret_cast<const z_t*>(part + r * ld) + w;
+      z_t t = p[0];
+      for (int q = 1; q < splits; q++) t = zadd(t, p[q * (sz / 2)]);
+      out[(long long)r * nw + w] = t;
+      re |= fabs(t.x) >= lre;
+      im |= fabs(t.y) >= lim_im;
+    }
+    if (re) mark[2 * wl] = 1;
+    if (im) mark[2 * wl + 1] = 1;
   }
+  __syncthreads();
+  const int i = threadIdx.x;
+  if (i < 2 * lanes && mark[i] && 2 * w0 + i < 2 * nw) b.ok[2 * w0 + i] = 1;
+}
+
+// W_w <- P (sum_k (i V_w)^k / k!) P W_w on the FP64 pipe for the walkers whose columns miss a
+// mark (ok [nw][2 n2], of the last product; bad: of those before) or when a wait timed out: a CTA per (walker, eight columns), a row per thread and pass, terms and sum in
+// the scratch S, T [nw][n2][N] (columns contiguous), from Wt, the walkers as they were.  Sums
+// over k in order.  All but always it reads 2 n2 marks and returns.
+constexpr int kRedoCols = 8;
+__global__ void __launch_bounds__(256)
+prop_redo_kernel(const z_t* __restrict__ P, const z_t* __restrict__ V, const z_t* __restrict__ Wt,
+                 z_t* S, z_t* T, z_t* __restrict__ W, int N, int n2, int order,
+                 const unsigned char* __restrict__ ok, const int* __restrict__ bad,
+                 const int* __restrict__ err, unsigned long long* redone) {
+  pdl_trigger();
+  pdl_wait();
+  const int w = blockIdx.y, tid = threadIdx.x, j0 = blockIdx.x * kRedoCols;
+  bool redo = *err != 0 || bad[w];
+  for (int i = tid; i < 2 * n2; i += 256) redo |= !ok[(long long)w * 2 * n2 + i];
+  if (!__syncthreads_or(redo)) return;
+  if (tid == 0 && blockIdx.x == 0) atomicAdd(redone, 1ull);
+  const int cols = min(kRedoCols, n2 - j0);
+  const long long c0 = ((long long)w * n2 + j0) * N;
+  z_t *s = S + c0, *t = T + c0;
+  // rows i, i + 256, ... of M times the columns B (visible to the CTA), handed to put(i, j, v)
+  auto product = [&](const z_t* M, const z_t* B, auto put) {
+    for (int i = tid; i < N; i += 256) {
+      z_t acc[kRedoCols];
+#pragma unroll
+      for (int j = 0; j < kRedoCols; j++) acc[j] = zmk(0, 0);
+      const z_t* m = M + (long long)i * N;
+      for (int k = 0; k < N; k++)
+#pragma unroll
+        for (int j = 0; j < kRedoCols; j++)
+          if (j < cols) zfma(acc[j], m[k], B[(long long)j * N + k]);
+#pragma unroll
+      for (int j = 0; j < kRedoCols; j++)
+        if (j < cols) put(i, j, acc[j]);
+    }
+    __syncthreads();
+  };
+  const z_t* Vw = V + (long long)w * N * N;
+  product(P, Wt + c0, [&](int i, int j, z_t v) { s[(long long)j * N + i] = v; });
+  // a term replaces the last one once every row is formed: until then it waits in W's columns
+  z_t* Ww = W + (long long)w * N * n2 + j0;
+  for (int k = 1; k <= order; k++) {
+    const z_t f = zmk(0.0, 1.0 / (double)k);
+    product(Vw, k == 1 ? s : t, [&](int i, int j, z_t v) { Ww[(long long)i * n2 + j] = zmul(f, v); });
+    for (int i = tid; i < N; i += 256)
+      for (int j = 0; j < cols; j++) {
+        const z_t v = Ww[(long long)i * n2 + j];
+        const long long o = (long long)j * N + i;
+        t[o] = v;
+        s[o] = zadd(s[o], v);
+      }
+    __syncthreads();
+  }
+  product(P, s, [&](int i, int j, z_t v) { Ww[(long long)i * n2 + j] = v; });
 }
 
 // Kpart[w][s][c] = tr(T T), T the n x n block of (c, w) in the chunk's product (rows
 // row0 + c n + a, columns w n + b).  One CTA per block, which passes through shared memory
 // by asynchronous copies: few registers and 16 n (n + 1) bytes a CTA keep several CTAs per
 // SM, whose copies overlap the others' sums (the block is fresh in L2).
+// norms[w][s][c] = half of |T|^2: the real parts of even columns and the imaginary parts of odd
+// ones (one multiply-add an entry beside the trace's four; FP64 sets the kernel's pace).
 constexpr int kTraceThreads = 128;
 __global__ void __launch_bounds__(kTraceThreads)
 trace_kernel(const z_t* __restrict__ T, int n, long long ld, int row0, int c_first,
-             z_t* __restrict__ Kpart, int nblk, int w_first, int s) {
+             z_t* __restrict__ Kpart, int nblk, int w_first, int s, double* __restrict__ norms) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) unsigned char tr_smem[];
   z_t* t = reinterpret_cast<z_t*>(tr_smem);   // [n][n + 1]
-  __shared__ z_t red[kTraceThreads / 32];
+  static_assert(kTraceThreads == 128, "four partial sums");
+  __shared__ double red[4][3];
   const int c = blockIdx.x, w = blockIdx.y, tid = threadIdx.x;
   const z_t* src = T + (row0 + (long long)c * n) * ld + (long long)w * n;
   // entry (a, b), stepping kTraceThreads entries at a time
@@ -573,19 +705,85 @@ trace_kernel(const z_t* __restrict__ T, int n, long long ld, int row0, int c_fir
     }
   }
   cp_async_commit();
+  const int lane = tid & 31, warp = tid >> 5;
   cp_async_wait<0>();
   __syncthreads();
   z_t sum = zmk(0, 0);
+  double f2 = 0.0;
   for (int a = a0, b = b0; a < n;) {
-    zfma(sum, t[a * (n + 1) + b], t[b * (n + 1) + a]);
+    const z_t x = t[a * (n + 1) + b];
+    zfma(sum, x, t[b * (n + 1) + a]);
+    const double h = b & 1 ? x.y : x.x;
+    f2 = fma(h, h, f2);
     a += da;
     if ((b += db) >= n) {
       b -= n;
       a++;
     }
   }
-  sum = block_zsum(sum, red);
-  if (tid == 0) Kpart[((long long)(w_first + w) * 2 + s) * nblk + c_first + c] = sum;
+  sum = warp_zsum(sum);
+  f2 = warp_sum(f2);
+  if (lane == 0) {
+    red[warp][0] = sum.x;
+    red[warp][1] = sum.y;
+    red[warp][2] = f2;
+  }
+  __syncthreads();
+  if (tid < 3) {
+    const double r = (red[0][tid] + red[2][tid]) + (red[1][tid] + red[3][tid]);
+    const long long o = ((long long)(w_first + w) * 2 + s) * nblk + c_first + c;
+    if (tid < 2)
+      reinterpret_cast<double*>(Kpart + o)[tid] = r;
+    else
+      norms[o] = r;
+  }
+}
+
+// Whether the digits hold a walker's exchange energy (one CTA of 128 threads): the error of an
+// entry of T is about 2^-56 sqrt(K) of its row's times its column's scale, so where the walker's
+// sum of |T|^2 (norms [2 nchol], halves) reaches kFloor^2 of the sum of those products squared,
+// the energy has 2^-49 sqrt(K) of the former.  sa2 [2]: sum of the squares of all row scales;
+// sb + s stride: the walker's 2n column scales, per spin.
+AFQ_D bool exchange_holds(const double* __restrict__ norms, int count, const double* sa2,
+                          const double* __restrict__ sb, long long stride, int n, z_t* red) {
+  z_t q = zmk(0, 0);
+  for (int i = threadIdx.x; i < count; i += 128) q.x += norms[i];
+  for (int i = threadIdx.x; i < 4 * n; i += 128) {
+    const int s = i >= 2 * n;
+    const double b = sb[s * stride + i - s * 2 * n];
+    q.y = fma(b * b, sa2[s], q.y);
+  }
+  q = block_zsum(q, red);
+  return 2.0 * q.x >= oz::kFloor * oz::kFloor * q.y;   // false for NaN
+}
+__global__ void __launch_bounds__(128)
+exchange_verdict_kernel(const double* __restrict__ norms, int count, const double* sa2,
+                        const double* __restrict__ sb, long long stride, int n,
+                        const int* __restrict__ err, int* __restrict__ gate,
+                        unsigned long long* redone) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ z_t red[4];
+  const int w = blockIdx.x;
+  const bool ok = exchange_holds(norms + (long long)w * count, count, sa2, sb + 2LL * w * n, stride,
+                                 n, red) && *err == 0;
+  if (threadIdx.x == 0) {
+    gate[w] = !ok;
+    if (!ok) atomicAdd(redone, 1ull);
+  }
+}
+// sa2[s] += sum of the squares of `count` scales of spin s (blockIdx.x, one CTA each).
+__global__ void __launch_bounds__(1024)
+scale_norm_kernel(const double* __restrict__ s0, const double* __restrict__ s1, int count,
+                  double* sa2) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ z_t red[32];
+  const double* p = blockIdx.x ? s1 : s0;
+  z_t q = zmk(0, 0);
+  for (int i = threadIdx.x; i < count; i += 1024) q.x = fma(p[i], p[i], q.x);
+  q = block_zsum(q, red);
+  if (threadIdx.x == 0) sa2[blockIdx.x] += q.x;
 }
 
 }  // namespace
@@ -617,7 +815,10 @@ cudaError_t create_exchange(OzState* o, cudaStream_t st) {
   if (o->ex_c < nc && whole * per_c <= cap + cap / 4)
     o->ex_c = (int)((cap + cap / 4) / per_c / whole) * whole;
   const size_t tb = per_c * o->ex_c + 256LL * 16 * (o->ex_w + 1) * n;   // whole row tiles
-  if (!fits(o, e, 2 * slice_bytes((long long)nc * n, K) + slice_bytes(2LL * nw * n, K) + tb)) return e;
+  const size_t norms = (size_t)nw * 2 * nc;
+  if (!fits(o, e, 2 * slice_bytes((long long)nc * n, K) + slice_bytes(2LL * nw * n, K) + tb +
+                      sizeof(double) * (norms + 4LL * nw * n)))
+    return e;
   for (int s = 0; s < 2 && e == cudaSuccess; s++) {
     e = alloc_slices(o, &o->lx[s], oz::kBM, nc * n, 1, K);
     if (e != cudaSuccess) break;
@@ -627,6 +828,13 @@ cudaError_t create_exchange(OzState* o, cudaStream_t st) {
   }
   if (e == cudaSuccess) e = alloc_slices(o, &o->gx, oz::kBN, 2 * nw * n, 1, K);
   if (e == cudaSuccess) e = oz_alloc(o, &o->T, tb / sizeof(double));
+  if (e == cudaSuccess) e = oz_alloc(o, &o->norms, norms);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->ex_gate, nw);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->sb, 4LL * nw * n);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->sa2, 2);
+  if (e == cudaSuccess) e = cudaMemsetAsync(o->sa2, 0, 2 * sizeof(double), st);
+  if (e == cudaSuccess)
+    e = pdl_launch(scale_norm_kernel, 2, 1024, 0, st, o->lx[0].scale, o->lx[1].scale, nc * n, o->sa2);
   o->exchange = e == cudaSuccess;
   return e;
 }
@@ -660,12 +868,13 @@ cudaError_t create_gsites(OzState* o, cudaStream_t st) {
     pmax = std::max(pmax, (size_t)(g.splits * rows[i] * o->part_ld));
   }
   if (!pmax || !fits(o, e, need + slice_bytes(2 * nw, K) + 8 * pmax)) return e;
-  if (e == cudaSuccess) e = alloc_slices(o, &o->gb, oz::kBN, 2 * nw, 1, K);
+  const Checked ck{st};
+  if (e == cudaSuccess) e = alloc_slices(o, &o->gb, oz::kBN, 2 * nw, 1, K, &ck);
   if (e == cudaSuccess) e = oz_alloc(o, &o->part, pmax);
   for (int i = 0; i < OZ_NG && e == cudaSuccess; i++) {
     if (!src[i]) continue;
     OzState::GSite& g = o->gs[i];
-    e = alloc_slices(o, &g.a, oz::kBM, g.rows, 1, K);
+    e = alloc_slices(o, &g.a, oz::kBM, g.rows, 1, K, &ck);
     const RowSrc rs{src[i], 1, NAK, 0};
     if (e == cudaSuccess)
       e = o->greal ? slice_rows<kReal>(rs, g.rows, (int)NAK, g.a, st)
@@ -694,8 +903,9 @@ cudaError_t create_vhs(OzState* o, cudaStream_t st) {
                                    (2e-6 + 1.0e-6 * ((K + oz::kSlab - 1) / oz::kSlab));
   if (dense >= csr) return e;
   if (!fits(o, e, slice_bytes(N2, K) + slice_bytes(2LL * in.nw, K))) return e;
-  e = alloc_slices(o, &o->sp, oz::kBM, (int)N2, 1, K);
-  if (e == cudaSuccess) e = alloc_slices(o, &o->xb, oz::kBN, 2 * in.nw, 1, K);
+  const Checked ck{st};
+  e = alloc_slices(o, &o->sp, oz::kBM, (int)N2, 1, K, &ck);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->xb, oz::kBN, 2 * in.nw, 1, K, &ck);
   if (e == cudaSuccess)
     e = o->sreal ? slice_rows<kDouble>(
                        RowSrc{reinterpret_cast<const z_t*>(in.Spvn_r), 1, in.nchol, 0}, (int)N2,
@@ -716,10 +926,12 @@ cudaError_t create_propagate(OzState* o, cudaStream_t st) {
   if (!fits(o, e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
                                                   slice_bytes(2 * n2, 2 * N))))
     return e;
-  if (e == cudaSuccess) e = alloc_slices(o, &o->pa, oz::kBM, N, 1, Kp);
-  if (e == cudaSuccess) e = alloc_slices(o, &o->va, oz::kBM, N, nw, 2 * N);
-  if (e == cudaSuccess) e = alloc_slices(o, &o->pb, oz::kBN, 2 * n2, nw, Kp);
+  const Checked ck{st};
+  if (e == cudaSuccess) e = alloc_slices(o, &o->pa, oz::kBM, N, 1, Kp, &ck);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->va, oz::kBM, N, nw, 2 * N, &ck);
+  if (e == cudaSuccess) e = alloc_slices(o, &o->pb, oz::kBN, 2 * n2, nw, Kp, &ck);
   if (e == cudaSuccess) e = alloc_slices(o, &o->tb, oz::kBN, 2 * n2, nw, 2 * N);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->prop_bad, nw);
   if (e == cudaSuccess)
     e = o->preal ? slice_rows<kReal>(RowSrc{in.P, 1, N, 0}, N, N, o->pa, st)
                  : slice_rows<kPairs>(RowSrc{in.P, 1, N, 0}, N, N, o->pa, st);
@@ -741,10 +953,12 @@ cudaError_t trace_attr(int n, size_t* smem) {
   });
 }
 
-// ek[w] = 1/2 sum of the walker's partial sums in a fixed order (NaN when a kernel timed out).
+// ek[w] = 1/2 sum of the walker's partial sums in a fixed order; gate[w]: the digits do not
+// hold it or a wait timed out.
 __global__ void __launch_bounds__(128)
-ek_sum_kernel(const z_t* __restrict__ part, int count, const int* __restrict__ err,
-              z_t* __restrict__ ek) {
+ek_sum_kernel(const z_t* __restrict__ part, const double* __restrict__ norms, int count,
+              const double* sa2, const double* __restrict__ sb, long long stride, int n,
+              const int* __restrict__ err, int* __restrict__ gate, z_t* __restrict__ ek) {
   pdl_trigger();
   pdl_wait();
   __shared__ z_t red[4];
@@ -752,8 +966,12 @@ ek_sum_kernel(const z_t* __restrict__ part, int count, const int* __restrict__ e
   z_t s = zmk(0, 0);
   for (int q = threadIdx.x; q < count; q += 128) s = zadd(s, part[(long long)w * count + q]);
   s = block_zsum(s, red);
-  const double bad = __longlong_as_double(0x7ff8000000000000LL);
-  if (threadIdx.x == 0) ek[w] = *err ? zmk(bad, bad) : zscale(s, 0.5);
+  const bool ok = exchange_holds(norms + (long long)w * count, count, sa2, sb + 2LL * w * n, stride,
+                                 n, red) && *err == 0;
+  if (threadIdx.x == 0) {
+    ek[w] = zscale(s, 0.5);
+    gate[w] = !ok;
+  }
 }
 
 // Chunks of oz_exchange_buffers: w walkers and c Cholesky vectors at a time; false when even
@@ -805,6 +1023,7 @@ cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc
   size_t smem = 0;
   cudaError_t e = trace_attr(n, &smem);
   if (e == cudaSuccess) e = cudaMemsetAsync(b.flags, 0, 2 * sizeof(int), st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.sa2, 0, 2 * sizeof(double), st);
   if (e != cudaSuccess) return e;
   int *err = b.flags, *cplx = b.flags + 1;
   oz_check_imag_kernel<<<148 * 8, 256, 0, st>>>(Lh, nc * NAK, cplx);
@@ -824,6 +1043,7 @@ cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc
     g.rows = 2 * w * n;
     const long long ld = (2LL * w * n + 3) / 4 * 4;
     for (int s = 0; s < 2; s++) {
+      g.scale = b.g_scale + (long long)s * b.g_rows;
       const RowSrc gs{Gc + w0 * NAK + (long long)s * n * N, n, NAK, N};
       pdl_launch(slice_found_kernel<true>, (w * n + 7) / 8, 256, 0, st, gs, w * n, N, g, cplx, nslab_real);
       for (int c0 = 0; c0 < nc; c0 += cc) {
@@ -832,15 +1052,18 @@ cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc
         const RowSrc as{Lh + c0 * NAK + (long long)s * n * N, n, NAK, N};
         pdl_launch(slice_found_kernel<false>, (c * n + 7) / 8, 256, 0, st, as, c * n, N, a, cplx,
                                                                   nslab_real);
+        if (w0 == 0)
+          pdl_launch(scale_norm_kernel, 1, 1024, 0, st, a.scale, nullptr, c * n, b.sa2 + s);
         oz::Gemm gm{&a, &g, c * n, 2 * w * n, 1};
         gm.cplx = cplx;
         gm.nslab_real = nslab_real;
         if ((e = oz::launch<7>(gm, EpiRows{b.T, ld, c * n}, err, st)) != cudaSuccess) return e;
         pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st, 
-            reinterpret_cast<const z_t*>(b.T), n, ld / 2, 0, c0, b.part, nc, 0, s);
+            reinterpret_cast<const z_t*>(b.T), n, ld / 2, 0, c0, b.part, nc, 0, s, b.norms);
       }
     }
-    pdl_launch(ek_sum_kernel, w, 128, 0, st, b.part, 2 * nc, err, ek + w0);
+    pdl_launch(ek_sum_kernel, w, 128, 0, st, b.part, b.norms, 2 * nc, b.sa2, b.g_scale,
+               b.g_rows, n, err, b.gate + w0, ek + w0);
   }
   return cudaGetLastError();
 }
@@ -853,6 +1076,9 @@ cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
   cudaError_t e = cudaMemGetInfo(&o->free_left, &total_b);
   if (e == cudaSuccess) e = oz_alloc(o, &o->err, 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
+  if (e == cudaSuccess) e = oz_alloc(o, &o->redone, OZ_NPRODUCTS);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(o->redone, 0, OZ_NPRODUCTS * sizeof(unsigned long long), st);
   const long long NAK = 2LL * in.n * in.N;
   RealCheck rc[4] = {{in.Lh, in.nchol * NAK, true},
                      {in.SpvnT, in.nchol * NAK, true},
@@ -886,8 +1112,25 @@ void oz_destroy(OzState* o) {
   delete o;
 }
 
+OzGate oz_gate(const OzState* o, int product) {
+  const Slices& b = product == OZ_VHS ? o->xb : o->gb;
+  OzGate g;
+  g.ok = reinterpret_cast<const uint4*>(b.ok);
+  g.n16 = (int)(ok_bytes(b.rows) / 16);
+  g.err = o->err;
+  g.redone = o->redone + product;
+  g.walkers = o->in.nw;
+  return g;
+}
+const int* oz_exchange_gate(const OzState* o) { return o->ex_gate; }
+
+cudaError_t oz_redone(const OzState* o, unsigned long long* redone) {
+  return cudaMemcpy(redone, o->redone, OZ_NPRODUCTS * sizeof(unsigned long long),
+                    cudaMemcpyDeviceToHost);
+}
+
 bool oz_has_gsite(const OzState* o, int site) { return o && o->gs[site].on; }
-int oz_gsite_launches(const OzState*, int) { return 3; }
+int oz_gsite_launches() { return 3; }
 
 cudaError_t oz_gsite(OzState* o, int site, const z_t* Gc, z_t* out, cudaStream_t st) {
   const OzState::GSite& g = o->gs[site];
@@ -900,10 +1143,12 @@ cudaError_t oz_gsite(OzState* o, int site, const z_t* Gc, z_t* out, cudaStream_t
   oz::Gemm gm{&g.a, &o->gb, g.rows, 2 * nw, g.splits, 0, 0, g.slab_split};
   e = oz::launch<7>(gm, EpiPart{o->part, o->part_ld, sz, g.rows}, o->err, st);
   if (e != cudaSuccess) return e;
-  const long long tot = (long long)g.rows * nw;
-  pdl_launch(part_sum_kernel, (unsigned)std::min<long long>((tot + 255) / 256, 148 * 16), 256, 0, st, 
-      o->part, o->part_ld, sz, g.splits, g.rows, nw, out);
-  return cudaGetLastError();
+  int lanes = 1;
+  while (lanes < 32 && lanes < nw) lanes *= 2;
+  const int ny = (nw + lanes - 1) / lanes, rpb = 256 / lanes;
+  const int nx = std::min((g.rows + rpb - 1) / rpb, std::max(1, tc::sm_count() * 16 / ny));
+  return pdl_launch(part_sum_kernel, dim3(nx, ny), 256, 0, st, o->part, o->part_ld, sz, g.splits,
+                    g.rows, nw, lanes, out, g.a.top, o->gb);
 }
 
 bool oz_has_vhs(const OzState* o) { return o && o->vhs; }
@@ -924,31 +1169,49 @@ cudaError_t oz_vhs(OzState* o, const z_t* X, z_t* vHS, cudaStream_t st) {
 }
 
 bool oz_has_propagate(const OzState* o) { return o && o->prop; }
-int oz_propagate_launches(const OzState* o) { return 1 + 1 + 2 * (2 + o->in.order); }
+int oz_propagate_launches(const OzState* o) { return 3 + 2 * (2 + o->in.order); }
 
-cudaError_t oz_propagate(OzState* o, z_t* W, const z_t* vHS, z_t* S, z_t* T, cudaStream_t st) {
+cudaError_t oz_propagate(OzState* o, const z_t* P, z_t* W, const z_t* vHS, z_t* S, z_t* T,
+                         z_t* Wt, cudaStream_t st) {
   const int N = o->in.N, n2 = 2 * o->in.n, nw = o->in.nw, order = o->in.order;
-  pdl_launch(transpose_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), 256, 0, st, W, N, n2, T);
+  pdl_launch(transpose_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), 256, 0, st, W, N, n2, Wt,
+             o->va.top, o->prop_bad);
   cudaError_t e = cudaGetLastError();
-  auto pslice = [&](const z_t* src) {   // walker columns as the B operand of Propg1
+  auto pslice = [&](const z_t* src, const RowCheck& chk) {   // walker columns as Propg1's B operand
     const RowSrc rs{src, 1, N, 0};
-    return o->preal ? slice_rows<kSplitRe>(rs, nw * n2, N, o->pb, st)
-                    : slice_rows<kSplitCx>(rs, nw * n2, N, o->pb, st);
+    return o->preal ? slice_rows<kSplitRe>(rs, nw * n2, N, o->pb, st, chk)
+                    : slice_rows<kSplitCx>(rs, nw * n2, N, o->pb, st, chk);
   };
-  if (e == cudaSuccess) e = pslice(T);
+  // each product is checked where its result is sliced (the last term with the sum it went
+  // into, the last product by its marks)
+  RowCheck chk;
+  chk.per = n2;
+  chk.bad = o->prop_bad;
+  if (e == cudaSuccess) e = pslice(Wt, RowCheck());
   oz::Gemm g{&o->pa, &o->pb, N, 2 * n2, nw};
+  g.mark = false;
   if (e == cudaSuccess) e = oz::launch<8>(g, EpiChain{S, T, N, n2, 0, 0}, o->err, st);
+  chk.top = o->pa.top;
+  chk.old = o->pb.scale;
   if (e == cudaSuccess && order > 0)
     e = slice_rows<kPairs>(RowSrc{vHS, 1, N, 0}, nw * N, N, o->va, st);
   oz::Gemm gv{&o->va, &o->tb, N, 2 * n2, nw};
   for (int k = 1; k <= order && e == cudaSuccess; k++) {
-    e = slice_rows<kSplitCx>(RowSrc{k == 1 ? S : T, 1, N, 0}, nw * n2, N, o->tb, st);
+    e = slice_rows<kSplitCx>(RowSrc{k == 1 ? S : T, 1, N, 0}, nw * n2, N, o->tb, st, chk);
     if (e == cudaSuccess)
       e = oz::launch<8>(gv, EpiChain{S, T, N, n2, k, k == order}, o->err, st);
+    chk.top = o->va.top;
+    chk.batched = 1;
+    chk.old = o->tb.scale;
+    chk.factor = k;   // T_k = (i / k) V T_{k-1}
   }
-  if (e == cudaSuccess) e = pslice(S);
+  if (e == cudaSuccess) e = pslice(S, chk);
+  g.mark = true;
   if (e == cudaSuccess) e = oz::launch<8>(g, EpiW{W, N, n2}, o->err, st);
-  return e;
+  if (e != cudaSuccess) return e;
+  return pdl_launch(prop_redo_kernel, dim3((n2 + kRedoCols - 1) / kRedoCols, nw), 256, 0, st, P, vHS,
+                    Wt, S, T, W, N, n2, order, o->pb.ok, o->prop_bad, o->err,
+                    o->redone + OZ_PROPAGATE);
 }
 
 bool oz_has_exchange(const OzState* o, int nwalk) { return o && o->exchange && nwalk <= o->in.nw; }
@@ -956,7 +1219,7 @@ bool oz_has_exchange(const OzState* o, int nwalk) { return o && o->exchange && n
 int oz_exchange_launches(const OzState* o, int nwalk) {
   const int cw = (nwalk + o->ex_w - 1) / o->ex_w;
   const int cc = (o->in.nchol + o->ex_c - 1) / o->ex_c;
-  return 2 + 4 * cw * cc;
+  return 3 + 4 * cw * cc;
 }
 
 cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nblk,
@@ -967,25 +1230,29 @@ cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nb
   cudaError_t e = trace_attr(n, &smem);
   for (int s = 0; s < 2 && e == cudaSuccess; s++) {
     const RowSrc src{Gc + (long long)s * n * N, n, NAK, N};
-    e = o->lreal ? slice_rows<kSplitRe>(src, nwalk * n, N, o->gx, st)
-                 : slice_rows<kSplitCx>(src, nwalk * n, N, o->gx, st);
+    Slices gx = o->gx;
+    gx.scale = o->sb + 2LL * s * o->in.nw * n;
+    e = o->lreal ? slice_rows<kSplitRe>(src, nwalk * n, N, gx, st)
+                 : slice_rows<kSplitCx>(src, nwalk * n, N, gx, st);
     for (int w0 = 0; w0 < nwalk && e == cudaSuccess; w0 += o->ex_w) {
       const int w = std::min(o->ex_w, nwalk - w0);
       for (int c0 = 0; c0 < nc && e == cudaSuccess; c0 += o->ex_c) {
         const int c = std::min(o->ex_c, nc - c0);
         // the row tiles that hold the chunk's rows [c0 n, (c0 + c) n)
         const int t0 = c0 * n / oz::kBM, row0 = c0 * n - t0 * oz::kBM;
-        oz::Gemm g{&o->lx[s], &o->gx, row0 + c * n, 2 * w * n, 1, t0, 2 * w0 * n / oz::kBN};
+        oz::Gemm g{&o->lx[s], &gx, row0 + c * n, 2 * w * n, 1, t0, 2 * w0 * n / oz::kBN};
         const long long ld = (2LL * w * n + 3) / 4 * 4;
         EpiRows epi{o->T, ld, row0 + c * n};
         if ((e = oz::launch<7>(g, epi, o->err, st)) != cudaSuccess) break;
         pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st, 
-            reinterpret_cast<const z_t*>(o->T), n, ld / 2, row0, c0, Kpart, nblk, w0, s);
+            reinterpret_cast<const z_t*>(o->T), n, ld / 2, row0, c0, Kpart, nblk, w0, s, o->norms);
         e = cudaGetLastError();
       }
     }
   }
-  return e;
+  if (e != cudaSuccess) return e;
+  return pdl_launch(exchange_verdict_kernel, nwalk, 128, 0, st, o->norms, 2 * nblk, o->sa2, o->sb,
+                    2LL * o->in.nw * n, n, o->err, o->ex_gate, o->redone + OZ_EXCHANGE);
 }
 
 cudaError_t oz_error(OzState* o, int* flags, cudaStream_t st) {

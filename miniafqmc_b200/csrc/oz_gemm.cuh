@@ -58,10 +58,23 @@ static_assert((kS + 1) * kBN <= 512 && kSmem <= 227 * 1024, "TMEM / shared memor
 // (piece index ^ (row / 2) mod 4).  A ring stage of an operand is then one contiguous bulk
 // copy.  K is zero padded to whole slabs; rows past the last one hold any digits (their
 // products are never stored).  scale [batch][rows] = 2^e of each row (0 for a zero row, NaN
-// for a row with a non-finite entry, which makes every output of the row NaN).
+// for a row with a non-finite entry or a maximum outside [2^-900, 2^900), which makes every
+// output of the row NaN).
+//
+// What the digits hold is relative to a row's largest entry: an output's error is about
+// 2^-56 sqrt(K) (A row's scale) (B row's scale), however small the output is.  So each B row
+// (a column of results) is marked ok once one of its outputs reaches kFloor x (largest A
+// scale) x (its own scale); the error is then below 2^-50 sqrt(K) of the column's largest
+// entry, as FP64 sums of K terms are to a few bits.  A column that no output marks (entries
+// of its operands spread so far apart that the large ones meet only zeros, or not finite)
+// leaves the call to the FP64 pipe.  top [batch] and ok [batch][rows] where the operand's
+// product is checked here.
+constexpr double kFloor = 0x1p-6;
 struct Slices {
   int8_t* d = nullptr;
   double* scale = nullptr;
+  double* top = nullptr;          // A operand: largest scale of the batch
+  unsigned char* ok = nullptr;    // B operand
   int rows = 0, batch = 0, tile = 0, nslab = 0;
   // source rows per batch, each giving one or two operand rows
   AFQ_HD int per_batch(bool two) const { return two ? rows / 2 : rows; }
@@ -80,6 +93,8 @@ AFQ_HD long long slice_offset(const Slices& s, int batch, int r, int k) {
 struct Job {
   const int8_t *a, *b;
   const double *sa, *sb;            // row scales [batch][rows]
+  const double* top;                // largest A scale per A batch (0 batches: one)
+  unsigned char* ok;                // marks of the B rows, or null
   int a_rows, b_rows, a_tiles, b_tiles;   // rows and row tiles per batch (0: not batched)
   tc::TileSched sched;
   int M, N;                         // output rows and columns per batch
@@ -318,6 +333,7 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
     const int row = wq * 32 + lane;
     const uint32_t trow = tmem + ((uint32_t)(wq * 32) << 16) + wg * 32;
     int li = 0;
+    long long marked = -1;
     for (int t = blockIdx.x; t < total; t += gridDim.x, li++) {
       int z, mt, nt;
       job.sched.decode(t, z, mt, nt);
@@ -339,9 +355,30 @@ oz_gemm_kernel(const __grid_constant__ Job job, const __grid_constant__ Epi epi,
         drain<ND, false>(trow, v);
       tc::tc_fence_before();
       tc::mbar_arrive(acce);
-      const double sa30 = sa * 0x1p-30;
+      const double sa30 = sa * 0x1p-30;   // (v sa) sb: no product of scales leaves the range
+      // the columns this warp marked last need no second look (all CTAs share their line)
+      const long long col = rb + n0 + lane;
+      if (job.ok && !__all_sync(0xffffffffu, col == marked || n0 + lane >= job.N)) {
+        // magnitudes by their high words (a bound rounded up); a NaN limit (a NaN scale of A,
+        // the only source of NaN here) lets none pass
+        const double lim = kFloor * job.top[job.a_rows ? z : 0];
+        const unsigned lw = lim == lim ? (unsigned)__double2hiint(lim) + (lim > 0.0) : 0xffffffffu;
+        unsigned any = 0;
 #pragma unroll
-      for (int c = 0; c < 32; c++) v[c] *= sa30 * __shfl_sync(0xffffffffu, sb, c);
+        for (int c = 0; c < 32; c++) {
+          v[c] *= sa30;
+          any |= (((unsigned)__double2hiint(v[c]) & 0x7fffffffu) >= lw ? 1u : 0u) << c;
+          v[c] *= __shfl_sync(0xffffffffu, sb, c);
+        }
+        any = __reduce_or_sync(0xffffffffu, any);
+        if ((any >> lane & 1) && n0 + lane < job.N && sb == sb && col != marked) {
+          job.ok[col] = 1;
+          marked = col;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 32; c++) v[c] = v[c] * sa30 * __shfl_sync(0xffffffffu, sb, c);
+      }
       epi(z, m, n0, v);
     }
   }
@@ -360,6 +397,7 @@ struct Gemm {
   int m_tile = 0, n_tile = 0;
   int slab_split = 0;
   bool m_fast = true;
+  bool mark = true;            // marks of B rows, where the operands carry them
   const int* cplx = nullptr;   // as Job::cplx, Job::nslab_real
   int nslab_real = 0;
 };
@@ -380,6 +418,8 @@ cudaError_t launch(const Gemm& g, const Epi& epi, int* err, cudaStream_t st) {
   j.b = g.b->d;
   j.sa = g.a->scale;
   j.sb = g.b->scale;
+  j.top = g.a->top;
+  j.ok = g.slab_split || !g.mark || !g.a->top ? nullptr : g.b->ok;   // K splits: checked summed
   const bool ab = !g.slab_split && g.a->batch > 1, bb = !g.slab_split && g.b->batch > 1;
   j.a_rows = ab ? g.a->rows : 0;
   j.b_rows = bb ? g.b->rows : 0;

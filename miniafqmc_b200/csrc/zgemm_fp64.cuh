@@ -24,6 +24,7 @@ struct ZGemmDesc {
   long long ldb, sB;
   z_t alpha;
   const double* Br = nullptr;   // real B operand (B_REAL launches; B unused)
+  OzGate gate;                  // set: runs only where the product's digit form does not hold
 };
 
 // ---------------------------------------------------------------- epilogues
@@ -77,6 +78,9 @@ zgemm_kernel(ZGemmDesc d, Epi epi) {
   using Cfg = ZTileCfg<BM, BN, BK, TM, TN>;
   constexpr int NTX = Cfg::NTX, NTY = Cfg::NTY, NT = Cfg::NT;
   constexpr int LDA_S = Cfg::LDA_S, LDB_S = Cfg::LDB_S;
+  pdl_trigger();
+  pdl_wait();
+  if (!oz_gate_open(d.gate)) return;
   extern __shared__ __align__(16) unsigned char zg_smem[];
   z_t* As = reinterpret_cast<z_t*>(zg_smem);
   z_t* Bs = As + 2 * BK * LDA_S;
@@ -204,8 +208,7 @@ cudaError_t zgemm_launch(const ZGemmDesc& d, int batch, const Epi& epi, cudaStre
     });                                                                                    \
     if (e != cudaSuccess) return e;                                                        \
     dim3 grid((d.N + BN_ - 1) / BN_, (d.M + BM_ - 1) / BM_, batch);                        \
-    kern<<<grid, Cfg::NT, Cfg::SMEM, st>>>(d, epi);                                        \
-    return cudaGetLastError();                                                             \
+    return pdl_launch(kern, grid, Cfg::NT, Cfg::SMEM, st, d, epi);                          \
   }
   switch (cfg) {
     case 1: AFQ_ZG_CASE(64, 32, 4, 2)
