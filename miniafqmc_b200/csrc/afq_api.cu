@@ -1057,7 +1057,9 @@ afq_status afq_set_hamiltonian(afq_handle* h, const afq_csr_z* Spvn, const afq_c
   }
   if (!h->mixed) {
     afq::OzInit oi{N, n, nc, h->nw, h->d.taylor_order, h->Lh, h->spT_dense, h->vk_dense,
-                   h->sp_dense, h->sp_dense_r, (long long)Spvn->rowIndex[N * N], h->P};
+                   h->sp_dense, h->sp_dense_r, (long long)Spvn->rowIndex[N * N],
+                   (long long)SpvnT->rowIndex[nc], Vakbl ? (long long)Vakbl->rowIndex[NAK] : 0,
+                   h->P};
     const char* digits = getenv("AFQ_FP64_DIGITS");
     if (!digits || atoi(digits) != 0) AFQ_CUDA(h, afq::oz_create(oi, &h->oz, h->st));
     if (afq::oz_has_exchange(h->oz, h->nw)) {   // one partial sum per Cholesky vector

@@ -20,7 +20,7 @@ struct OzInit {
   const z_t* Vakbl;      // dense [2nN][2nN] or null
   const z_t* Spvn;       // dense [N^2][nchol] of complex values, or null
   const double* Spvn_r;  // dense [N^2][nchol] of real values, or null
-  long long spvn_nnz;
+  long long spvn_nnz, SpvnT_nnz, Vakbl_nnz;
   const z_t* P;          // Propg1 [N][N]
 };
 

@@ -404,8 +404,12 @@ csr_gather_kernel(const int* __restrict__ rowIndex, const int* __restrict__ cols
 cudaError_t launch_csr_gather(const int* rowIndex, const int* cols, const z_t* vals, const z_t* G,
                               long long ldg, int nrows, int nw, z_t* out, cudaStream_t st,
                               const OzGate& gate) {
-  return pdl_launch(csr_gather_kernel, (nrows + 7) / 8, 256, 0, st, rowIndex, cols, vals, G, ldg,
-                    nrows, nw, out, gate);
+  if (gate.ok)
+    return pdl_launch(csr_gather_kernel, (nrows + 7) / 8, 256, 0, st, rowIndex, cols, vals, G, ldg,
+                      nrows, nw, out, gate);
+  csr_gather_kernel<<<(nrows + 7) / 8, 256, 0, st>>>(rowIndex, cols, vals, G, ldg, nrows, nw, out,
+                                                     gate);
+  return cudaGetLastError();
 }
 
 // ============================================================ weights
@@ -1247,8 +1251,12 @@ cudaError_t launch_exchange(const z_t* Lh, const z_t* Gc, int N, int n, int ncho
   if (e != cudaSuccess) return e;
   // a gated launch mostly does nothing: few CTAs, each looping over the walker groups
   dim3 grid(nblk, std::min((nw + Gw - 1) / Gw, gate ? 4 : 65535), 2);
-  return pdl_launch(exchange_kernel, grid, EX_THREADS, smem, st, Lh, Gc, N, n, nchol, nw, Gn, Gw,
-                    Kpart, stride ? stride : nblk, gate);
+  if (gate)
+    return pdl_launch(exchange_kernel, grid, EX_THREADS, smem, st, Lh, Gc, N, n, nchol, nw, Gn, Gw,
+                      Kpart, stride ? stride : nblk, gate);
+  exchange_kernel<<<grid, EX_THREADS, smem, st>>>(Lh, Gc, N, n, nchol, nw, Gn, Gw, Kpart,
+                                                  stride ? stride : nblk, gate);
+  return cudaGetLastError();
 }
 
 // ============================================================ energy reductions

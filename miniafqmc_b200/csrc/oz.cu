@@ -798,12 +798,23 @@ bool fits(OzState* o, cudaError_t e, size_t need) {
 }
 size_t slice_bytes(long long rows, long long K) { return (size_t)kS * (rows + 128) * (K + 64); }
 
+// Which exchange products take the digits: blocks of n^2 N >= 3100, where a block's
+// multiply-adds on the FP64 pipe take longer than its trace, at 32 orbitals and more (a shorter
+// K leaves the drain and T's way through memory); few smaller blocks from 64 orbitals as well,
+// where the FP64 kernel is one serial chain over K.  Energies of 256 walkers without and with,
+// us: 10 electrons at 32 orbitals, 128 vectors 238 > 183; 16 at 48, 192 vectors 661 > 412; 8 at 64,
+// 256 vectors 357 > 264; 6 at 128, 512 vectors 664 > 444; 4 at 128 411 > 380; 8 at 32, 128 vectors
+// 142 < 160; 4 at 64, 256 vectors 151 < 206 (16 walkers 97 > 64).
+bool exchange_pays(int N, int n, int nc, int nw) {
+  return (N >= 32 && (double)n * n * N >= 3100.0) || (N >= 64 && 2.0 * nc * nw <= 10000.0);
+}
 cudaError_t create_exchange(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;
   const int N = in.N, n = in.n, nc = in.nchol, nw = in.nw;
   const long long NAK = 2LL * n * N;
   cudaError_t e = cudaSuccess;
   const int K = o->lreal ? N : 2 * N;
+  if (K > oz::kMaxK || !exchange_pays(N, n, nc, nw)) return e;
   // chunk of T: walkers first (in whole 64-column tiles, up to 32 MB per 128 rows), then
   // Cholesky vectors, up to 64 MB (half of L2)
   const long long cap = 64LL << 20;
@@ -840,13 +851,20 @@ cudaError_t create_exchange(OzState* o, cudaStream_t st) {
 }
 
 // Products with G.  K splits fill the SMs when the output tiles do not (and bound a split's
-// K for the int32 accumulators), at least two slabs each.
+// K for the int32 accumulators), at least two slabs each.  From a K of 2nN = 256 on, where the
+// FP64 pipe's serial sums take longer than four launches (vbias of 256 vectors, 16 walkers: K =
+// 128 14.8 < 18.2 us, 192 19.0 < 20.3, 256 24.6 > 19.9, 512 41.5 > 22.1, 2048 150 > 22), and from
+// 96 nonzeros a row and 64 walkers, where the CSR product does (K = 2048: 43 nonzeros, 16 walkers
+// 18.9 < 22.2; 102 nonzeros 30.9 > 22.1, 64 walkers 66 > 26).
 cudaError_t create_gsites(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;
   const int nw = in.nw;
   const long long NAK = 2LL * in.n * in.N;
-  const z_t* src[OZ_NG] = {in.SpvnT, in.Lh, in.Vakbl};
   const long long rows[OZ_NG] = {in.nchol, in.nchol, NAK};
+  const long long nnz[OZ_NG] = {in.SpvnT_nnz, in.nchol * NAK, in.Vakbl_nnz};
+  const z_t* src[OZ_NG] = {in.SpvnT, in.Lh, in.Vakbl};
+  for (int i = 0; i < OZ_NG; i++)
+    if (NAK < 256 || nnz[i] * ((nw + 63) / 64) < 96 * rows[i]) src[i] = nullptr;
   cudaError_t e = cudaSuccess;
   size_t need = 0;
   for (int i = 0; i < OZ_NG; i++)
@@ -899,7 +917,8 @@ cudaError_t create_vhs(OzState* o, cudaStream_t st) {
   if (K > oz::kMaxK) return e;
   const double csr = (double)in.spvn_nnz * in.nw / (o->sreal ? 2.9e12 : 1.45e12);
   const long long tiles = (N2 + oz::kBM - 1) / oz::kBM * ((2LL * in.nw + oz::kBN - 1) / oz::kBN);
-  const double dense = 15e-6 + (double)((tiles + 147) / 148) *
+  const int sms = tc::sm_count();
+  const double dense = 15e-6 + (double)((tiles + sms - 1) / sms) *
                                    (2e-6 + 1.0e-6 * ((K + oz::kSlab - 1) / oz::kSlab));
   if (dense >= csr) return e;
   if (!fits(o, e, slice_bytes(N2, K) + slice_bytes(2LL * in.nw, K))) return e;
@@ -915,13 +934,19 @@ cudaError_t create_vhs(OzState* o, cudaStream_t st) {
   return e;
 }
 
-// Propagation: from 3e8 real operations per product (14 us of the FP64 pipe at the measured
-// 22 TFLOP/s, above the launches of the splitting kernels).
+// Propagation: from 116 orbitals and 5e8 real operations per product; 1e9 and 3e9 where more of
+// the row tiles is padding (fewer than 0.66 and 0.6 of their rows in use).  Whole chains on the
+// FP64 pipe and as digits, us: 64 orbitals 1.5e9 operations 626 < 1439, 96 638 < 815, 112 of 16+16
+// electrons 709 < 752, 116 of 20+20 5e8 453 > 311, 128 of 32+32 5e8 255 > 212; 136 of 30+30 1e9 558 <
+// 617, 3e9 1551 and 1525; 160 of 48+48 5e8 261 < 311, 1e9 461 > 451; 200 of 40+40 5e8 312 > 277; 384 of
+// 48+48 4.5e8 248 < 264, 6.8e8 389 > 267.
 cudaError_t create_propagate(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;
   const int N = in.N, n2 = 2 * in.n, nw = in.nw;
   cudaError_t e = cudaSuccess;
-  if (8.0 * N * (double)N * n2 * nw < 3e8 || 2 * N > oz::kMaxK || nw > 65535) return e;
+  const double padded = (double)((N + oz::kBM - 1) / oz::kBM * oz::kBM);
+  const double least = N < 0.6 * padded ? 3e9 : N < 0.66 * padded ? 1e9 : 5e8;
+  if (N < 116 || 8.0 * N * (double)N * n2 * nw < least || 2 * N > oz::kMaxK || nw > 65535) return e;
   const int Kp = o->preal ? N : 2 * N;
   if (!fits(o, e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
                                                   slice_bytes(2 * n2, 2 * N))))
@@ -1008,11 +1033,13 @@ bool buffers_plan(const OzBuffers& b, int N, int n, int nc, int nw, int* w, int*
 
 }  // namespace
 
-// From 8e8 real operations (about 60 us of the FP64 pipe's exchange kernel, which runs at 14
-// TFLOP/s) the digit products' launches pay.
+// As exchange_pays, and n walkers times electrons >= 200 for the splitting of Lh, which every
+// call repeats (16 electrons at 200 orbitals: 8 walkers 336 < 378 us, 33 walkers 984 > 475; at 384,
+// 2 walkers 588 < 1228), from 1.5e9 real operations (two waves of tiles).
 bool oz_exchange_buffers_fit(const OzBuffers& b, int N, int n, int nc, int nw) {
   int w, c;
-  return 16.0 * nc * n * (double)n * N * nw >= 8e8 && buffers_plan(b, N, n, nc, nw, &w, &c);
+  return n >= 4 && N >= 40 && (double)n * n * N >= 5000.0 && (double)n * nw >= 200.0 &&
+         16.0 * nc * n * (double)n * N * nw >= 1.5e9 && buffers_plan(b, N, n, nc, nw, &w, &c);
 }
 
 cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc, int N, int n,

@@ -188,7 +188,7 @@ def exchange_reference(L, G):
     return ek, size
 
 
-def buffers(cplx, nmo=41, nel=20, nchol=60, nw=60):
+def buffers(cplx, nmo=41, nel=20, nchol=120, nw=60):
     import torch
     g = torch.Generator("cuda").manual_seed(nmo)
     rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda", dtype=torch.float64)  # noqa: E731
