@@ -18,7 +18,7 @@ struct OzState {
   std::vector<void*> allocs;
   char* block = nullptr;    // rest of the last shared block
   size_t block_left = 0;
-  size_t free_left = 0;     // device memory not yet planned for
+  size_t budget = 0;        // device memory that further groups of products may take
   int* err = nullptr;
   // per product (OzProduct) the walkers whose result the digits did not hold; per walker
   // whether the last exchange's did not, and whether the propagation's did not on the way
@@ -790,10 +790,13 @@ scale_norm_kernel(const double* __restrict__ s0, const double* __restrict__ s1, 
 
 namespace {
 
-// Whether the next group of allocations takes less than a third of the device memory left.
+// Whether the next group of allocations fits what is left of the budget: a sixth of the device
+// memory free at set-up for all digits and workspaces together, so that other handles find
+// nearly the room they did without them (C4 with 128 walkers takes 3.6 GB).
+constexpr size_t kMemoryShare = 6;
 bool fits(OzState* o, cudaError_t e, size_t need) {
-  if (e != cudaSuccess || need >= o->free_left / 3) return false;
-  o->free_left -= need;
+  if (e != cudaSuccess || need > o->budget) return false;
+  o->budget -= need;
   return true;
 }
 size_t slice_bytes(long long rows, long long K) { return (size_t)kS * (rows + 128) * (K + 64); }
@@ -1100,7 +1103,8 @@ cudaError_t oz_create(const OzInit& in, OzState** out, cudaStream_t st) {
   OzState* o = new OzState();
   o->in = in;
   size_t total_b = 0;
-  cudaError_t e = cudaMemGetInfo(&o->free_left, &total_b);
+  cudaError_t e = cudaMemGetInfo(&o->budget, &total_b);
+  o->budget /= kMemoryShare;
   if (e == cudaSuccess) e = oz_alloc(o, &o->err, 1);
   if (e == cudaSuccess) e = cudaMemsetAsync(o->err, 0, sizeof(int), st);
   if (e == cudaSuccess) e = oz_alloc(o, &o->redone, OZ_NPRODUCTS);
