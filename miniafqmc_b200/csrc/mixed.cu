@@ -1685,13 +1685,30 @@ cudaError_t mixed_create(const MixedInit* init, MixedState** out, std::string* m
   {
     // Tile width.  The product is bound by shared memory: per 128-byte K slab a 128-column
     // tile's MMAs read 96 KB and its fills write 64 KB for 768 tensor clocks (1280 clocks at
-    // 128 bytes a clock), a 256-column tile 144 + 96 KB for 1536 (1920).  1536 vectors x 1024
-    // walkers of 48+48 electrons 0.68 -> 0.47 ms, 1024 x 512 of 64+64 0.23 -> 0.185, 800 x 256
-    // of 40+40 (14 tiles) vbias stage 31 -> 28 us.  With fewer tiles the slices run out (384
-    // vectors x 128 walkers 6.6 -> 8.0 us), and with 262 columns half of the second tile is
-    // padding (54 -> 77 us).
-    const int mt = (nc + 127) / 128, w128 = (2 * nw + 127) / 128, w256 = (2 * nw + 255) / 256;
-    m->part_bn = mt * w256 >= 13 && 16 * w256 <= 9 * w128 ? 256 : 128;
+    // 128 bytes a clock), a 256-column tile 144 + 96 KB for 1536 (1920).  But half as many
+    // tiles fill the last wave of SMs worse or take more slices, whose partial sums cross
+    // memory.  So both widths are estimated for the slice counts the tuner tries: waves x slabs
+    // of a slice x 0.76 or 1.18 us (128-byte slabs under load), and 5 us per million partial
+    // sums; within 5% of the measured ratio of vbias stages over 150 shapes (16 to 48 electrons at
+    // 64 to 256 orbitals, 128 to 1536 vectors, 96 to 1024 walkers).  48+48 electrons at 256
+    // orbitals: 1536 vectors x 1024 walkers 608 > 499 us, 1024 x 256 135 > 117, 640 x 512 (20 tiles,
+    // 2.2 waves) 180 < 198; 16+16 at 64 orbitals, 1024 x 512 36 < 48.
+    // Below a K of 4096 the start of the longer tiles shows: 128 columns (16+16 electrons at 64
+    // orbitals, 640 x 320 28 < 30).
+    const long long slabs = ((m->greal ? NAK : 2 * NAK) + 63) / 64;
+    auto estimate = [&](int bn, double slab_us) {
+      const int t = ((nc + 127) / 128) * ((2 * nw + bn - 1) / bn);
+      const int s0 = std::max(1, std::min(16, (4 * 148 + t - 1) / t));
+      double best = 1e30;
+      for (int s : {s0, std::max(1, s0 / 2), std::min(32, 2 * s0)}) {
+        const long long per = (slabs + s - 1) / s, used = (slabs + per - 1) / per;
+        const long long waves = (t * used + tc::sm_count() - 1) / tc::sm_count();
+        best = std::min(best, waves * per * slab_us + 5e-6 * used * nc * nw);
+      }
+      return best;
+    };
+    m->part_bn = slabs >= 64 && estimate(256, 1.18) < 0.93 * estimate(128, 0.76) ? 256 : 128;
+    const int mt = (nc + 127) / 128;
     const int tiles = mt * ((2 * nw + m->part_bn - 1) / m->part_bn);
     set_splits(m, std::max(1, std::min(16, (int)((4 * 148 + tiles - 1) / tiles))));
     m->splits0 = m->splits;
