@@ -2,6 +2,7 @@
 // oz_gemm.cuh and the kernels around them.
 #include <cooperative_groups.h>
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "afq_kernels.h"
@@ -801,15 +802,23 @@ bool fits(OzState* o, cudaError_t e, size_t need) {
 }
 size_t slice_bytes(long long rows, long long K) { return (size_t)kS * (rows + 128) * (K + 64); }
 
-// Which exchange products take the digits: blocks of n^2 N >= 3100, where a block's
-// multiply-adds on the FP64 pipe take longer than its trace, at 32 orbitals and more (a shorter
-// K leaves the drain and T's way through memory); few smaller blocks from 64 orbitals as well,
-// where the FP64 kernel is one serial chain over K.  Energies of 256 walkers without and with,
-// us: 10 electrons at 32 orbitals, 128 vectors 238 > 183; 16 at 48, 192 vectors 661 > 412; 8 at 64,
-// 256 vectors 357 > 264; 6 at 128, 512 vectors 664 > 444; 4 at 128 411 > 380; 8 at 32, 128 vectors
-// 142 < 160; 4 at 64, 256 vectors 151 < 206 (16 walkers 97 > 64).
+// Which exchange products take the digits: blocks of n^2 N >= 3100 at 32 orbitals and more (a
+// shorter K leaves the drain and T's way through memory), where a block's multiply-adds on the
+// FP64 pipe take longer than its trace.  Energies of 256 walkers without and with, us: 10
+// electrons at 32 orbitals, 128 vectors 238 > 183; 16 at 48, 192 vectors 661 > 412; 8 at 64, 256
+// vectors 357 > 264; 6 at 128, 512 vectors 664 > 444; 8 at 32, 128 vectors 142 < 160.
+// Smaller blocks: the digits take about 32 us and 1.2 ns a block, the FP64 kernel's waves 0.4 us
+// an orbital and 0.3 us for each of a warp's turns at the traces of its 96 / n by 96 / n blocks
+// (1 electron at 55 orbitals, 120 vectors, 213 walkers 339 > 123; 2 at 64, 128 vectors 256 / 512
+// walkers 131 > 125 / 134 < 197; 4 at 64, 256 vectors 16 / 256 walkers 97 > 64 / 151 < 206).
 bool exchange_pays(int N, int n, int nc, int nw) {
-  return (N >= 32 && (double)n * n * N >= 3100.0) || (N >= 64 && 2.0 * nc * nw <= 10000.0);
+  if (N >= 32 && (double)n * n * N >= 3100.0) return true;
+  const int g = 96 / n;
+  const double blocks = 2.0 * nc * nw;
+  const double ctas = 2.0 * ((nc + g - 1) / g) * ((nw + g - 1) / g);
+  const double wave = 0.3 * g * ((g + 7) / 8) * ((n * n + 31) / 32) + 0.4 * N + 4.0;
+  return (double)n * n * N < 3100.0 &&
+         32.0 + 1.2e-3 * blocks < wave * std::ceil(ctas / (2.0 * tc::sm_count()));
 }
 cudaError_t create_exchange(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;

@@ -34,12 +34,14 @@ def run(s, nw, monkeypatch, digits, taylor=6):
 
 
 @pytest.mark.parametrize("nmo,nel,nchol,nw,on", [
-    (32, 3, 24, 5, {"vbias": False, "exchange": False}),             # K = 192
-    (32, 4, 24, 5, {"vbias": True, "exchange": False}),              # K = 256, short blocks
+    (32, 3, 24, 5, {"vbias": False, "exchange": True}),              # K = 192; 32 x 32 blocks
+    (32, 4, 24, 5, {"vbias": True, "exchange": True}),               # K = 256
+    (32, 8, 24, 40, {"vbias": True, "exchange": False}),             # short blocks
     (32, 10, 24, 40, {"vbias": True, "exchange": True}),             # n^2 N = 3200
     (31, 31, 8, 40, {"vbias": True, "exchange": False}),             # K below 32
     (64, 4, 40, 60, {"exchange": True}),                             # small blocks, few of them
-    (64, 4, 80, 80, {"exchange": False}),                            # and many
+    (64, 4, 80, 160, {"exchange": False}),                           # and many
+    (17, 1, 40, 30, {"vbias": False, "exchange": True}),             # blocks of one
     (115, 32, 8, 128, {"propagate": False}),
     (116, 32, 8, 80, {"propagate": True}),
     (130, 30, 8, 60, {"propagate": False}),                          # half of the tiles padding
