@@ -50,12 +50,20 @@ struct DeviceAttr {
 AFQ_D void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 AFQ_D void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// cluster > 1: CTAs in clusters of that many along x.
 template <class... P, class... A>
-inline cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              A&&... args) {
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+inline cudaError_t pdl_launch_cluster(void (*kern)(P...), unsigned cluster, dim3 grid, dim3 block,
+                                      size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (cluster > 1) {
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster;
+    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+    n++;
+  }
+  at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[n].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -65,8 +73,13 @@ inline cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t 
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   const cudaError_t e = cudaStreamIsCapturing(st, &capture);
   if (e != cudaSuccess) return e;
-  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? n + 1 : n;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              A&&... args) {
+  return pdl_launch_cluster(kern, 1, grid, block, smem, st, static_cast<A&&>(args)...);
 }
 
 // Launch of the FP64 pipe's form of a product after its digit form (oz_gemm.cuh): the kernel

@@ -187,12 +187,15 @@ cudaError_t launch_dm(const z_t* W, const z_t* tw, int N, int n, int nw, z_t* Gc
 
 // ============================================================ sigma
 // X = x + i vbias, hybridW[w] = -sum_c i vb (x + i/2 vb)  (miniafqmc_base.cpp:281-289).
-// A cluster of 8 CTAs per 32 walkers (lanes), a CTA's 32 warps and the cluster's CTAs on
+// A cluster of up to 8 CTAs per 32 walkers (lanes), a CTA's 32 warps and the cluster's CTAs on
 // Cholesky rows; the groups' sums meet in the first CTA in a fixed order.  The field's normals
 // cost two FP64 logarithm / sine evaluations' latency per row and warp: one CTA per 32
-// walkers took 20 us at 256 rows and 90 us at 1536.
+// walkers took 20 us at 256 rows and 90 us at 1536.  A CTA per 32 rows, per 64 where the clusters
+// would fill half the SMs: two turns of a warp cost less than many clusters' start (256 rows, 32
+// / 512 walkers 10.0 / 14.1 us with 8 CTAs, 12.0 / 12.1 with 4; 16 rows, 1024 walkers 7.5 with
+// one, 14.5 with 8).
 constexpr int kSigmaCluster = 8;
-__global__ void __cluster_dims__(kSigmaCluster, 1, 1) __launch_bounds__(1024)
+__global__ void __launch_bounds__(1024)
 sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restrict__ xraw,
              z_t* __restrict__ hybridW, int nchol, int nw, const DevScalars* __restrict__ sc,
              int use_xraw) {
@@ -202,14 +205,15 @@ sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restr
   cg::cluster_group cl = cg::this_cluster();
   __shared__ z_t red[32][33];
   __shared__ z_t part[32];
-  const int lane = threadIdx.x, g = threadIdx.y, rank = blockIdx.x % kSigmaCluster;
-  const int w = blockIdx.x / kSigmaCluster * 32 + lane;
+  const int ctas = cl.num_blocks();
+  const int lane = threadIdx.x, g = threadIdx.y, rank = blockIdx.x % ctas;
+  const int w = blockIdx.x / ctas * 32 + lane;
   const unsigned long long seed = sc->seed, step = sc->step;
   const long long nwg = sc->nwalk_global > 0 ? sc->nwalk_global : nw;
   const long long woff = sc->walker_offset;
   z_t hw = zmk(0, 0);
   if (w < nw) {
-    for (int c = rank * 32 + g; c < nchol; c += 32 * kSigmaCluster) {
+    for (int c = rank * 32 + g; c < nchol; c += 32 * ctas) {
       long long e = (long long)c * nw + w;
       double x;
       if (use_xraw) {
@@ -234,12 +238,16 @@ sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restr
   if (g == 0) {
     z_t s = zmk(0, 0);
     for (int q = 0; q < 32; q++) s = zadd(s, red[q][lane]);
+    if (ctas == 1) {   // uniform
+      if (w < nw) hybridW[w] = s;
+    }
     part[lane] = s;
   }
+  if (ctas == 1) return;
   cl.sync();
   if (rank == 0 && g == 0 && w < nw) {
     z_t s = zmk(0, 0);
-    for (int q = 0; q < kSigmaCluster; q++) s = zadd(s, cl.map_shared_rank(part, q)[lane]);
+    for (int q = 0; q < ctas; q++) s = zadd(s, cl.map_shared_rank(part, q)[lane]);
     hybridW[w] = s;
   }
   cl.sync();   // every CTA's sums stay until the first has read them
@@ -247,9 +255,12 @@ sigma_kernel(const z_t* __restrict__ vbias, z_t* __restrict__ X, double* __restr
 
 cudaError_t launch_sigma(const z_t* vbias, z_t* X, double* xraw, z_t* hybridW, int nchol,
                          int nw, const DevScalars* sc, int use_xraw, cudaStream_t st) {
-  pdl_launch(sigma_kernel, (nw + 31) / 32 * kSigmaCluster, dim3(32, 32), 0, st, vbias, X, xraw, hybridW,
-                                                                       nchol, nw, sc, use_xraw);
-  return cudaGetLastError();
+  const unsigned groups = (nw + 31) / 32;
+  unsigned ctas = 1;
+  while (ctas < kSigmaCluster && 32 * (int)ctas < nchol) ctas *= 2;
+  while (ctas > 1 && groups * ctas > 74 && nchol < 64 * (int)ctas) ctas /= 2;
+  return pdl_launch_cluster(sigma_kernel, ctas, groups * ctas, dim3(32, 32), 0, st, vbias, X,
+                            xraw, hybridW, nchol, nw, sc, use_xraw);
 }
 
 // ============================================================ CSR x dense (walker-fast B)
