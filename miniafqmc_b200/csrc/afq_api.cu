@@ -1098,10 +1098,9 @@ afq_status afq_get_walkers(afq_handle* h, double* W, double* W_data) {
     AFQ_CUDA(h, afq::launch_walker_layout(h->W, h->T2, h->N, h->n, h->nw, 1, h->st));
     AFQ_CUDA(h, afq::copy_to_host(&h->ring, W, h->T2, sizeof(z_t) * count, h->st));
   }
-  if (W_data) {
+  if (W_data)
     AFQ_CUDA(h, cudaMemcpyAsync(W_data, h->Wd, sizeof(z_t) * nw * 8, cudaMemcpyDeviceToHost, h->st));
-    AFQ_CUDA(h, cudaStreamSynchronize(h->st));
-  }
+  AFQ_CUDA(h, cudaStreamSynchronize(h->st));
   return AFQ_OK;
 }
 

@@ -105,22 +105,20 @@ void share(char* dst, const char* src, size_t bytes, int i, int n) {
 
 cudaError_t copy_to_host(HostRing** ring, void* dst, const void* src, size_t bytes,
                          cudaStream_t st) {
+  if (bytes < kLeast) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
   Crew crew;
   const long chunks = (long)((bytes + kChunk - 1) / kChunk);
   auto len = [=](long c) { return c + 1 < chunks ? kChunk : bytes - (size_t)c * kChunk; };
   char* d = static_cast<char*>(dst);
   const char* s = static_cast<const char*>(src);
-  bool crewed = bytes >= kLeast && ring_ready(ring);
+  bool crewed = ring_ready(ring);
   if (crewed) {
     HostRing* r = *ring;
     crewed = crew.start(chunks, [=](long c, int i, int n) {
       share(d + (size_t)c * kChunk, r->slot[c % kSlots], len(c), i, n);
     });
   }
-  if (!crewed) {
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
-    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-  }
+  if (!crewed) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
   HostRing* r = *ring;
   cudaError_t e = cudaSuccess;
   auto issue = [&](long c) {
@@ -147,22 +145,20 @@ cudaError_t copy_to_host(HostRing** ring, void* dst, const void* src, size_t byt
 
 cudaError_t copy_to_device(HostRing** ring, void* dst, const void* src, size_t bytes,
                            cudaStream_t st) {
+  if (bytes < kLeast) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   Crew crew;
   const long chunks = (long)((bytes + kChunk - 1) / kChunk);
   auto len = [=](long c) { return c + 1 < chunks ? kChunk : bytes - (size_t)c * kChunk; };
   char* d = static_cast<char*>(dst);
   const char* s = static_cast<const char*>(src);
-  bool crewed = bytes >= kLeast && ring_ready(ring);
+  bool crewed = ring_ready(ring);
   if (crewed) {
     HostRing* r = *ring;
     crewed = crew.start(chunks, [=](long c, int i, int n) {
       share(r->slot[c % kSlots], s + (size_t)c * kChunk, len(c), i, n);
     });
   }
-  if (!crewed) {
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-  }
+  if (!crewed) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
   HostRing* r = *ring;
   cudaError_t e = cudaSuccess;
   crew.ready.store(chunks < kSlots ? chunks : kSlots, std::memory_order_release);

@@ -9,8 +9,9 @@ namespace afq {
 struct HostRing;   // allocated by the first large copy of a handle
 void host_ring_destroy(HostRing* r);
 
-// dst (host) <- src (device) or dst (device) <- src (host), in order on `st`; returns with
-// the copy done.
+// dst (host) <- src (device) or dst (device) <- src (host), in order on `st`.  Pageable host
+// memory is free for use on return; the caller synchronises `st` before it reads dst or frees
+// pinned memory.
 cudaError_t copy_to_host(HostRing** ring, void* dst, const void* src, size_t bytes, cudaStream_t st);
 cudaError_t copy_to_device(HostRing** ring, void* dst, const void* src, size_t bytes,
                            cudaStream_t st);
