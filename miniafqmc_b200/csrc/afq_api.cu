@@ -398,7 +398,7 @@ cudaError_t body_propagate(afq_handle* h) {
   if (afq::oz_has_propagate(h->oz))
     return afq::oz_propagate(h->oz, h->P, h->W, h->vHS, h->S, h->T1, h->T2, h->st);
   const int N = h->N, n2 = 2 * h->n, nw = h->nw;
-  if (afq::prop_small_fits(N, n2, nw))
+  if (afq::prop_small_fits(N, n2, nw, h->d.taylor_order))
     return afq::launch_prop_small(h->P, h->vHS, h->W, N, n2, nw, h->d.taylor_order, h->st);
   const long long sWN = (long long)N * n2, sV = (long long)N * N;
   const int zc = h->f64cfg[afq_handle::F64_PROP];
@@ -528,7 +528,7 @@ cudaError_t st_vhs(afq_handle* h) {
 cudaError_t st_propagate(afq_handle* h) {
   int nl = h->mixed ? afq::mixed_launches(h->mixed, AFQ_STAGE_PROPAGATE)
            : afq::oz_has_propagate(h->oz) ? afq::oz_propagate_launches(h->oz)
-           : afq::prop_small_fits(h->N, 2 * h->n, h->nw) ? 1 : h->d.taylor_order + 2;
+           : afq::prop_small_fits(h->N, 2 * h->n, h->nw, h->d.taylor_order) ? 1 : h->d.taylor_order + 2;
   return staged(h, AFQ_STAGE_PROPAGATE, nl, [&] { return body_propagate(h); });
 }
 cudaError_t st_weights(afq_handle* h, int update_eshift) {

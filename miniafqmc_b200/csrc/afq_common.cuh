@@ -36,6 +36,18 @@ struct DeviceAttr {
   }
 };
 
+// SMs of the device (every device is a B200).
+inline int device_sms() {
+  static const int n = [] {   // initialised once, thread-safe
+    int dev = 0, c = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0)
+      c = 148;
+    return c;
+  }();
+  return n;
+}
+
 // Programmatic dependent launch.  A kernel launched with pdl_launch may start while the kernel
 // before it on the stream still runs: its CTAs take SM slots as they come free and do their set-up
 // (barriers, TMEM), then pdl_wait() holds them until every earlier grid has completed and its

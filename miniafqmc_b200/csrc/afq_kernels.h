@@ -30,8 +30,10 @@ cudaError_t launch_set_scalars(DevScalars* sc, unsigned long long seed, unsigned
 cudaError_t launch_ortho(z_t* W, int N, int n, int nw, cudaStream_t st);
 cudaError_t launch_ortho_cholqr(z_t* W, int N, int n, int nw, int* info, cudaStream_t st);
 // The FP64 propagation of small systems in one launch (W in place; the walkers equal the
-// eight products' bit for bit); prop_small_fits: the shapes it takes.
-bool prop_small_fits(int N, int n2, int nw);
+// eight products' bit for bit); prop_small_fits: the shapes it takes; prop_zgemm_us: estimate
+// of the separate products.
+bool prop_small_fits(int N, int n2, int nw, int order);
+double prop_zgemm_us(int N, int n2, int nw, int order);
 cudaError_t launch_prop_small(const z_t* P, const z_t* V, z_t* W, int N, int n2, int nw, int order,
                               cudaStream_t st);
 // Walkers between the reference's layout [nw][2][N][n] and the device's [nw][N][2n]

@@ -6,6 +6,7 @@
 //   Gc  [nw][2][n][N] per-walker compact density matrices (linear index s*n*N + a*N + k)
 //   vHS [nw][N][N], vbias / X / xraw [nchol][nw] (reference layout)
 #include <cooperative_groups.h>
+#include <cmath>
 #include <cstdlib>
 
 #include "afq_kernels.h"
@@ -345,7 +346,7 @@ cudaError_t csr_walker_launch(const int* rowIndex, const int* cols, const z_t* z
                               long long out_ld, cudaStream_t st, const OzGate& gate) {
   dim3 grid((nrows + ROWS - 1) / ROWS, (nw + 32 * WPL - 1) / (32 * WPL));
   if (gate.ok) {
-    grid.x = std::min(grid.x, 8u * 148u);
+    grid.x = std::min(grid.x, 8u * device_sms());
     return rvals ? pdl_launch(csr_walker_kernel<true, ROWS, WPL, true>, grid, ROWS * 32, 0, st,
                               rowIndex, cols, nullptr, rvals, B, nrows, nw, out, out_ld, gate)
                  : pdl_launch(csr_walker_kernel<false, ROWS, WPL, true>, grid, ROWS * 32, 0, st,
@@ -1079,12 +1080,39 @@ prop_small_kernel(const z_t* __restrict__ P, const z_t* __restrict__ V, z_t* __r
   }
 }
 
-// Up to 1.2e8 real operations per product, where the separate products are latency bound:
-// 64 orbitals, 16 walkers (1.7e7) 70 -> 36 us, 100 orbitals, 20 walkers of 30+30 electrons
-// (9.6e7) 150 -> 127 us; past it the tiled products win (64 orbitals, 250 walkers, 2.6e8: 165
-// against 207 us).
-bool prop_small_fits(int N, int n2, int nw) {
-  return N <= kPropSmallMaxN && nw <= 65535 && 8.0 * N * N * (double)n2 * nw <= 1.2e8;
+// The chain of order + 2 separate products (ZGEMM), us: per product 4.5 for the launch, then the
+// longer of a serial sum over k (0.076 an orbital) and the tiles of the busiest SM (0.3 each and
+// 21 TFLOP/s of the whole chip, padding included), for the best of zgemm's tile shapes.  Within
+// 8% (rms) of 330 measured chains of 6 to 330 orbitals, 1e5 to 2e10 operations a product.
+double prop_zgemm_us(int N, int n2, int nw, int order) {
+  static const int shape[][2] = {{64, 32}, {64, 64}, {64, 96}, {32, 64}, {32, 96}, {128, 64}, {32, 32}};
+  const int sms = device_sms();
+  double best = 1e30;
+  for (const auto& s : shape) {
+    const double tiles = (double)((N + s[0] - 1) / s[0]) * ((n2 + s[1] - 1) / s[1]) * nw;
+    const double busiest = std::ceil(tiles / sms);
+    best = std::min(best, std::max(0.076 * N, busiest * (0.3 + N * 8.0 * s[0] * s[1] * sms / 21e6)));
+  }
+  return (order + 2) * (4.5 + best);
+}
+// Up to 1.2e8 real operations per product and where its own estimate is below 0.8 of the separate
+// products': per wave of CTAs one start a product, then a multiply-add chain (0.052 us an orbital)
+// or the multiply-adds of the CTAs that share an SM (0.038 us an orbital, CTA and row pass); within
+// 11% of 110 chains.  Separate and in one launch, us: 64 orbitals, 16 walkers of 16+16 electrons
+// 70 > 36, 100 orbitals, 20 walkers of 30+30 150 > 127; 30 orbitals, 332 walkers of 14+14 85 < 125,
+// 16 orbitals, 875 walkers of 7+7 84 < 95, 11 orbitals, 721 walkers of 5+5 66 > 52.
+bool prop_small_fits(int N, int n2, int nw, int order) {
+  if (N > kPropSmallMaxN || nw > 65535 || 8.0 * N * N * (double)n2 * nw > 1.2e8) return false;
+  const int sms = device_sms();
+  const int occ = std::max(1, std::min(4, (int)((227 << 10) / (prop_small_smem(N) + 1024))));
+  const double ctas = std::ceil((double)((n2 + PS_COLS - 1) / PS_COLS) * nw / sms);
+  const double waves = std::floor(ctas / occ), rest = ctas - waves * occ;
+  auto wave = [&](double share) {
+    const int passes = N <= PS_ROWS ? 1 : 2;
+    return (order + 2) * (1.0 + std::max(0.052 * N, 0.038 * share * N * passes));
+  };
+  const double us = waves * wave(occ) + (rest > 0 ? wave(rest) : 0.0);
+  return us < 0.8 * prop_zgemm_us(N, n2, nw, order);
 }
 
 cudaError_t launch_prop_small(const z_t* P, const z_t* V, z_t* W, int N, int n2, int nw, int order,

@@ -946,19 +946,32 @@ cudaError_t create_vhs(OzState* o, cudaStream_t st) {
   return e;
 }
 
-// Propagation: from 116 orbitals and 5e8 real operations per product; 1e9 and 3e9 where more of
-// the row tiles is padding (fewer than 0.66 and 0.6 of their rows in use).  Whole chains on the
-// FP64 pipe and as digits, us: 64 orbitals 1.5e9 operations 626 < 1439, 96 638 < 815, 112 of 16+16
-// electrons 709 < 752, 116 of 20+20 5e8 453 > 311, 128 of 32+32 5e8 255 > 212; 136 of 30+30 1e9 558 <
-// 617, 3e9 1551 and 1525; 160 of 48+48 5e8 261 < 311, 1e9 461 > 451; 200 of 40+40 5e8 312 > 277; 384 of
-// 48+48 4.5e8 248 < 264, 6.8e8 389 > 267.
+// Propagation: where the chain's estimate is below 0.97 of the FP64 pipe's (prop_zgemm_us), us:
+// 110 for the launches of splitting, products and checks, the busiest SM's tiles (2.74 and 1.42 a
+// slab each), 2.6e-6 a digit split and 1.5e-3 a row; within 8% (rms) of 190 measured chains of 50 to
+// 330 orbitals, 3e8 to 2e10 operations a product.  Not for chains that run in one launch.  FP64
+// pipe and digits, us: 64 orbitals, 1431 walkers of 16+16 electrons 626 < 1439; 96, 318 of 32+32 638
+// < 815; 105, 3000 of 24+24 8825 > 6140; 121, 986 of 2+2 1521 > 745; 128, 119 of 32+32 492 > 365; 136, 113
+// of 30+30 558 < 617; 160, 25 of 48+48 261 < 311, 76 662 > 630; 200, 20 of 40+40 312 > 277; 384, 4 of 48+48
+// 248 < 264, 9 548 > 344.
+double prop_digits_us(int N, int n2, int nw, int order, bool preal) {
+  auto slabs = [](int K) { return (K + oz::kSlab - 1) / oz::kSlab; };
+  const int sms = tc::sm_count();
+  const double tiles = (double)((N + oz::kBM - 1) / oz::kBM) *
+                       ((2 * n2 + oz::kBN - 1) / oz::kBN) * nw;
+  const double busiest = std::ceil(tiles / sms), kp = oz::kSlab * slabs(2 * N);
+  const double rows = (double)nw * (N + (order + 1.0) * n2);
+  return 110.0 + busiest * (order * (2.74 + 1.42 * slabs(2 * N)) +
+                            2.0 * (2.74 + 1.42 * slabs(preal ? N : 2 * N))) +
+         2.6e-6 * kp * nw * (N + (order + 1.0) * 2 * n2) + 1.5e-3 * rows;
+}
 cudaError_t create_propagate(OzState* o, cudaStream_t st) {
   const OzInit& in = o->in;
   const int N = in.N, n2 = 2 * in.n, nw = in.nw;
   cudaError_t e = cudaSuccess;
-  const double padded = (double)((N + oz::kBM - 1) / oz::kBM * oz::kBM);
-  const double least = N < 0.6 * padded ? 3e9 : N < 0.66 * padded ? 1e9 : 5e8;
-  if (N < 116 || 8.0 * N * (double)N * n2 * nw < least || 2 * N > oz::kMaxK || nw > 65535) return e;
+  if (2 * N > oz::kMaxK || nw > 65535 || prop_small_fits(N, n2, nw, in.order) ||
+      prop_digits_us(N, n2, nw, in.order, o->preal) >= 0.97 * prop_zgemm_us(N, n2, nw, in.order))
+    return e;
   const int Kp = o->preal ? N : 2 * N;
   if (!fits(o, e, slice_bytes(N, Kp) + (size_t)nw * (slice_bytes(N, 2 * N) + slice_bytes(2 * n2, Kp) +
                                                   slice_bytes(2 * n2, 2 * N))))

@@ -1087,16 +1087,7 @@ cudaError_t launch_multi(const MultiJob<Epi, NP>& job, int* err, cudaStream_t st
   return cudaGetLastError();
 }
 
-inline int sm_count() {
-  static const int n = [] {   // initialised once, thread-safe (every device is a B200)
-    int dev = 0, c = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || c <= 0)
-      c = 148;
-    return c;
-  }();
-  return n;
-}
+inline int sm_count() { return device_sms(); }
 
 template <int BN, int STAGES, int FMT, bool SPLIT, class Epi, int EPI_WG = 1, int SLAB = 128>
 cudaError_t launch_persistent(const Maps& maps, const GemmShape& g, const Epi& epi, int* err,

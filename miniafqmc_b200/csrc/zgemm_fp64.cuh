@@ -14,6 +14,8 @@
 // shared memory with cp.async.  A and B slabs are stored [k][m] / [k][n] so the inner
 // loop reads one A broadcast and TN consecutive B values per k.
 #pragma once
+#include <type_traits>
+
 #include "afq_common.cuh"
 
 struct ZGemmDesc {
@@ -71,16 +73,20 @@ struct ZTileCfg {
   static constexpr size_t SMEM = sizeof(z_t) * 2 * BK * (LDA_S + LDB_S);
 };
 
+// GATED: the form after a digit product.  An instance of its own: four registers more leave one
+// CTA of the 64 x 64 shapes on an SM instead of two.
 template <int BM, int BN, int BK, int TM, int TN, bool A_KMAJ, bool B_KMAJ, class Epi,
-          bool B_REAL = false>
+          bool B_REAL = false, bool GATED = false>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 zgemm_kernel(ZGemmDesc d, Epi epi) {
   using Cfg = ZTileCfg<BM, BN, BK, TM, TN>;
   constexpr int NTX = Cfg::NTX, NTY = Cfg::NTY, NT = Cfg::NT;
   constexpr int LDA_S = Cfg::LDA_S, LDB_S = Cfg::LDB_S;
-  pdl_trigger();
-  pdl_wait();
-  if (!oz_gate_open(d.gate)) return;
+  if constexpr (GATED) {
+    pdl_trigger();
+    pdl_wait();
+    if (!oz_gate_open(d.gate)) return;
+  }
   extern __shared__ __align__(16) unsigned char zg_smem[];
   z_t* As = reinterpret_cast<z_t*>(zg_smem);
   z_t* Bs = As + 2 * BK * LDA_S;
@@ -201,17 +207,25 @@ cudaError_t zgemm_launch(const ZGemmDesc& d, int batch, const Epi& epi, cudaStre
 #define AFQ_ZG_CASE(BM_, BN_, TM_, TN_)                                                     \
   {                                                                                        \
     using Cfg = ZTileCfg<BM_, BN_, 16, TM_, TN_>;                                          \
+    dim3 grid((d.N + BN_ - 1) / BN_, (d.M + BM_ - 1) / BM_, batch);                        \
+    if constexpr (std::is_same<Epi, EpiStore>::value) {                                    \
+      if (d.gate.ok) {                                                                     \
+        auto gated = zgemm_kernel<BM_, BN_, 16, TM_, TN_, A_KMAJ, B_KMAJ, Epi, B_REAL, true>; \
+        static DeviceAttr gattr;                                                           \
+        const cudaError_t ge = gattr.ensure(Cfg::SMEM, [gated](size_t b) {                 \
+          return cudaFuncSetAttribute(gated, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b); \
+        });                                                                                \
+        return ge == cudaSuccess ? pdl_launch(gated, grid, Cfg::NT, Cfg::SMEM, st, d, epi) : ge; \
+      }                                                                                    \
+    }                                                                                      \
     auto kern = zgemm_kernel<BM_, BN_, 16, TM_, TN_, A_KMAJ, B_KMAJ, Epi, B_REAL>;         \
     static DeviceAttr attr;                                                                \
     const cudaError_t e = attr.ensure(Cfg::SMEM, [kern](size_t b) {                        \
       return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b); \
     });                                                                                    \
     if (e != cudaSuccess) return e;                                                        \
-    dim3 grid((d.N + BN_ - 1) / BN_, (d.M + BM_ - 1) / BM_, batch);                        \
-    /* dependent CTAs that start early sit on the SMs the running product leaves free, and \
-       then share them (propagation of 9 walkers at 384 orbitals 548 -> 911 us): only the   \
-       gated form, which mostly returns at once, is launched so */                          \
-    if (d.gate.ok) return pdl_launch(kern, grid, Cfg::NT, Cfg::SMEM, st, d, epi);            \
+    /* a plain launch: dependent CTAs that start early sit on the SMs the running product  \
+       leaves free, and then share them (9 walkers at 384 orbitals 548 -> 911 us) */       \
     kern<<<grid, Cfg::NT, Cfg::SMEM, st>>>(d, epi);                                        \
     return cudaGetLastError();                                                             \
   }

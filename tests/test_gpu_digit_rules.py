@@ -42,11 +42,13 @@ def run(s, nw, monkeypatch, digits, taylor=6):
     (64, 4, 40, 60, {"exchange": True}),                             # small blocks, few of them
     (64, 4, 80, 160, {"exchange": False}),                           # and many
     (17, 1, 40, 30, {"vbias": False, "exchange": True}),             # blocks of one
-    (115, 32, 8, 128, {"propagate": False}),
-    (116, 32, 8, 80, {"propagate": True}),
-    (130, 30, 8, 60, {"propagate": False}),                          # half of the tiles padding
+    (64, 16, 8, 700, {"propagate": False}),                          # two slabs of padding
+    (121, 2, 8, 986, {"propagate": True}),
+    (130, 30, 8, 30, {"propagate": False}),                          # half of the tiles padding
     (130, 64, 8, 175, {"propagate": True}),
     (192, 32, 8, 30, {"propagate": True}),
+    (30, 14, 8, 332, {"propagate": False}),                          # one launch or eight
+    (11, 5, 8, 721, {"propagate": False}),
 ])
 def test_rules_of_size(nmo, nel, nchol, nw, on, monkeypatch):
     s = tiny_system(complex_trial=False, complex_chol=False, nmo=nmo, nel=nel, nchol=nchol)

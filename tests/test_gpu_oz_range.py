@@ -131,7 +131,7 @@ def test_vhs_of_graded_rows():
 def test_propagation_past_a_large_entry_of_vhs():
     """vHS couples orbital p to orbital q by 1e12; no walker reaches q."""
     from miniafqmc_b200.afqmc import AfqmcSys
-    nmo, nel, nchol, nw, p, q = 128, 16, 64, 160, 9, 40
+    nmo, nel, nchol, nw, p, q = 128, 20, 64, 160, 9, 40
     s = dataclasses.replace(tiny_system(complex_trial=False, complex_chol=False, nmo=nmo, nel=nel,
                                         nchol=nchol))
     A = s.Spvn.todense().reshape(nmo, nmo, nchol)
@@ -237,7 +237,7 @@ def test_infinity_is_the_fp64_pipes(monkeypatch):
 def test_waits_that_run_out_are_reported_and_the_fp64_pipe_computes():
     from miniafqmc_b200.afqmc import AfqmcError, AfqmcSys, load_library
     lib = load_library()
-    s = tiny_system(complex_trial=False, complex_chol=False, nmo=128, nel=16, nchol=64)
+    s = tiny_system(complex_trial=False, complex_chol=False, nmo=128, nel=20, nchol=64)
     nw = 160
     e = AfqmcSys(s, nw, use_vakbl=False, walkers=walkers(s, nw))
     on = e.digit_products()
