@@ -1128,8 +1128,8 @@ cudaError_t launch_prop_small(const z_t* P, const z_t* V, z_t* W, int N, int n2,
     return r;
   });
   if (e != cudaSuccess) return e;
-  pdl_launch(prop_small_kernel, dim3((n2 + PS_COLS - 1) / PS_COLS, nw), PS_THREADS, smem, st, P, V, W, N, n2,
-                                                                                      order);
+  pdl_launch(prop_small_kernel, dim3((n2 + PS_COLS - 1) / PS_COLS, nw), PS_THREADS, smem, st, P, V,
+             W, N, n2, order);
   return cudaGetLastError();
 }
 
@@ -1350,8 +1350,8 @@ energy_reduce_kernel(const z_t* __restrict__ Gc, const z_t* __restrict__ haj, in
 cudaError_t launch_energy_reduce(const z_t* Gc, const z_t* haj, int nak, const z_t* Gcloc,
                                  const z_t* cv, int nchol, const z_t* Kpart, int nblk, int nw,
                                  int mode, z_t* Wd, double* parts, cudaStream_t st) {
-  pdl_launch(energy_reduce_kernel, nw, 256, 0, st, Gc, haj, nak, Gcloc, cv, nchol, Kpart, nblk, nw, mode,
-                                           Wd, parts);
+  pdl_launch(energy_reduce_kernel, nw, 256, 0, st, Gc, haj, nak, Gcloc, cv, nchol, Kpart, nblk, nw,
+             mode, Wd, parts);
   return cudaGetLastError();
 }
 

@@ -1922,8 +1922,8 @@ static cudaError_t vhs_product(MixedState* m, cudaStream_t st) {
 
 cudaError_t mixed_vhs_pack(MixedState* m, const z_t* X, cudaStream_t st) {
   const int nc = m->nc, nw = m->nw;
-  pdl_launch(pack_x_kernel, dim3((nc + 31) / 32, (nw + 31) / 32), dim3(32, 8), 0, st, X, nc, nw, m->Kv,
-                                                                             m->s_real, m->Xf);
+  pdl_launch(pack_x_kernel, dim3((nc + 31) / 32, (nw + 31) / 32), dim3(32, 8), 0, st, X, nc, nw,
+             m->Kv, m->s_real, m->Xf);
   return cudaGetLastError();
 }
 
@@ -1961,8 +1961,8 @@ static cudaError_t propagate_chain(MixedState* m, z_t* W, int wave, bool timing,
   if (!timing) m->packed = false;
   cudaError_t e;
   if (!from_f2 && !timing) {
-    pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, 
-        W, N, n2, m->F[0], pr ? 2 : 1);
+    pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, W, N,
+               n2, m->F[0], pr ? 2 : 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   ChainJob job{};
@@ -2030,8 +2030,8 @@ cudaError_t mixed_propagate(MixedState* m, z_t* W, const z_t*, cudaStream_t st) 
   m->packed = false;
   cudaError_t e;
   if (!from_f2) {
-    pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, 
-        W, N, n2, m->F[0], pr ? 2 : 1);
+    pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, W, N,
+               n2, m->F[0], pr ? 2 : 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   const int mt = (N + 127) / 128;
@@ -2202,8 +2202,8 @@ cudaError_t mixed_vhs_multi(MixedState* const* ms, int n, cudaStream_t st) {
 cudaError_t mixed_prop_pack(MixedState* m, const z_t* W, cudaStream_t st) {
   if (m->packed) return cudaSuccess;   // the P W operand is in F2
   const bool pr = m->preal && m->in.order >= 1;
-  pdl_launch(pack_w_kernel, dim3((m->N + 31) / 32, (2 * m->n + 31) / 32, m->nw), dim3(32, 8), 0, st, 
-      W, m->N, 2 * m->n, m->F[0], pr ? 2 : 1);
+  pdl_launch(pack_w_kernel, dim3((m->N + 31) / 32, (2 * m->n + 31) / 32, m->nw), dim3(32, 8), 0,
+             st, W, m->N, 2 * m->n, m->F[0], pr ? 2 : 1);
   return cudaGetLastError();
 }
 
@@ -2310,16 +2310,16 @@ static cudaError_t splitk_product(MixedState* m, const tc::Maps& mp, int prec, f
   }
   if (e != cudaSuccess) return e;
   const bool f16 = prec == PREC_SPLIT16;
-  pdl_launch(reduce_part_kernel, grid_for((long long)nc * nw), 256, 0, st, 
-      m->part, m->splits, nc, nw, out, f16 ? ascale : 1.0f, f16 ? m->wscale : nullptr);
+  pdl_launch(reduce_part_kernel, grid_for((long long)nc * nw), 256, 0, st, m->part, m->splits, nc,
+             nw, out, f16 ? ascale : 1.0f, f16 ? m->wscale : nullptr);
   return cudaGetLastError();
 }
 
 // Gb of every walker (per-walker scales first when the G products run fp16 split)
 static cudaError_t pack_gb(MixedState* m, const z_t* Gc, cudaStream_t st) {
   if (m->Gb.f16) gc_scale_kernel<<<m->nw, 256, 0, st>>>(Gc, m->NAK, m->wscale);
-  pdl_launch(pack_gc_kernel, grid_for((long long)m->nw * m->NAK), 256, 0, st, 
-      Gc, m->nw, m->n, m->N, m->Gb, Op{}, 0, m->greal, m->Gb.f16 ? m->wscale : nullptr);
+  pdl_launch(pack_gc_kernel, grid_for((long long)m->nw * m->NAK), 256, 0, st, Gc, m->nw, m->n,
+             m->N, m->Gb, Op{}, 0, m->greal, m->Gb.f16 ? m->wscale : nullptr);
   return cudaGetLastError();
 }
 
@@ -2419,8 +2419,8 @@ cudaError_t mixed_exchange(MixedState* m, const z_t* Gc, int nsub, z_t* Kpart, i
   if (!m->in.Lh || nsub > m->nw) return cudaErrorInvalidValue;
   const bool f16 = m->Gx.f16;
   if (f16) gc_scale_kernel<<<nsub, 256, 0, st>>>(Gc, m->NAK, m->wscale);
-  pdl_launch(pack_gc_kernel, grid_for((long long)nsub * m->NAK), 256, 0, st, 
-      Gc, nsub, m->n, m->N, Op{}, m->Gx, m->nw, m->greal, f16 ? m->wscale : nullptr);
+  pdl_launch(pack_gc_kernel, grid_for((long long)nsub * m->NAK), 256, 0, st, Gc, nsub, m->n, m->N,
+             Op{}, m->Gx, m->nw, m->greal, f16 ? m->wscale : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return exchange_product(m, nsub, Kpart, nblk, st);
@@ -2453,8 +2453,8 @@ cudaError_t mixed_exchange_lowp(MixedState* m, const z_t* Gc, int nsub, z_t* Kpa
                                 cudaStream_t st) {
   if (!m->in.Lh || nsub > m->nw) return cudaErrorInvalidValue;
   if (m->Gx.f16 || m->prec_ek != PREC_SPLIT) return cudaErrorNotSupported;
-  pdl_launch(pack_gc_kernel, grid_for((long long)nsub * m->NAK), 256, 0, st, 
-      Gc, nsub, m->n, m->N, Op{}, m->Gx, m->nw, m->greal, nullptr);
+  pdl_launch(pack_gc_kernel, grid_for((long long)nsub * m->NAK), 256, 0, st, Gc, nsub, m->n, m->N,
+             Op{}, m->Gx, m->nw, m->greal, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // the base's fp32 sums over K need no promotion next to its bf16 operand rounding; the
@@ -2491,8 +2491,8 @@ cudaError_t mixed_dm(MixedState* m, const z_t* W, z_t* Gc, z_t* Wd, int* info, i
     // T1 (conjugated) of both spins: one 128-row tile per walker; its A operand is packed
     // unless the walkers' packed forms are current
     if (!m->packed) {
-      pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, W, N, n2,
-                                                                                   m->F[0], 0);
+      pdl_launch(pack_w_kernel, dim3((N + 31) / 32, (n2 + 31) / 32, nw), dim3(32, 8), 0, st, W, N,
+                 n2, m->F[0], 0);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     const tc::Maps& mt1 = (m->packed && m->fa_buf == 1) ? m->m_t1_1 : m->m_t1;

@@ -681,7 +681,10 @@ prop_redo_kernel(const z_t* __restrict__ P, const z_t* __restrict__ V, const z_t
 // by asynchronous copies: few registers and 16 n (n + 1) bytes a CTA keep several CTAs per
 // SM, whose copies overlap the others' sums (the block is fresh in L2).
 // norms[w][s][c] = half of |T|^2: the real parts of even columns and the imaginary parts of odd
-// ones (one multiply-add an entry beside the trace's four; FP64 sets the kernel's pace).
+// ones (one multiply-add an entry beside the trace's four; all of it and the scales' norms in
+// this kernel took 4% of the exchange of 32 electrons at 128 orbitals).  What bounds the kernel:
+// the blocks' latency at five CTAs an SM for n = 48 (counters: issue slots 41%, L1 40%, waiting
+// for loads first).
 constexpr int kTraceThreads = 128;
 __global__ void __launch_bounds__(kTraceThreads)
 trace_kernel(const z_t* __restrict__ T, int n, long long ld, int row0, int c_first,
@@ -1097,25 +1100,26 @@ cudaError_t oz_exchange_buffers(const OzBuffers& b, const z_t* Lh, const z_t* Gc
     for (int s = 0; s < 2; s++) {
       g.scale = b.g_scale + (long long)s * b.g_rows;
       const RowSrc gs{Gc + w0 * NAK + (long long)s * n * N, n, NAK, N};
-      pdl_launch(slice_found_kernel<true>, (w * n + 7) / 8, 256, 0, st, gs, w * n, N, g, cplx, nslab_real);
+      pdl_launch(slice_found_kernel<true>, (w * n + 7) / 8, 256, 0, st, gs, w * n, N, g, cplx,
+                 nslab_real);
       for (int c0 = 0; c0 < nc; c0 += cc) {
         const int c = std::min(cc, nc - c0);
         a.rows = c * n;
         const RowSrc as{Lh + c0 * NAK + (long long)s * n * N, n, NAK, N};
         pdl_launch(slice_found_kernel<false>, (c * n + 7) / 8, 256, 0, st, as, c * n, N, a, cplx,
-                                                                  nslab_real);
+                   nslab_real);
         if (w0 == 0)
           pdl_launch(scale_norm_kernel, 1, 1024, 0, st, a.scale, nullptr, c * n, b.sa2 + s);
         oz::Gemm gm{&a, &g, c * n, 2 * w * n, 1};
         gm.cplx = cplx;
         gm.nslab_real = nslab_real;
         if ((e = oz::launch<7>(gm, EpiRows{b.T, ld, c * n}, err, st)) != cudaSuccess) return e;
-        pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st, 
-            reinterpret_cast<const z_t*>(b.T), n, ld / 2, 0, c0, b.part, nc, 0, s, b.norms);
+        pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st,
+                   reinterpret_cast<const z_t*>(b.T), n, ld / 2, 0, c0, b.part, nc, 0, s, b.norms);
       }
     }
-    pdl_launch(ek_sum_kernel, w, 128, 0, st, b.part, b.norms, 2 * nc, b.sa2, b.g_scale,
-               b.g_rows, n, err, b.gate + w0, ek + w0);
+    pdl_launch(ek_sum_kernel, w, 128, 0, st, b.part, b.norms, 2 * nc, b.sa2, b.g_scale, b.g_rows,
+               n, err, b.gate + w0, ek + w0);
   }
   return cudaGetLastError();
 }
@@ -1262,8 +1266,8 @@ cudaError_t oz_propagate(OzState* o, const z_t* P, z_t* W, const z_t* vHS, z_t* 
   g.mark = true;
   if (e == cudaSuccess) e = oz::launch<8>(g, EpiW{W, N, n2}, o->err, st);
   if (e != cudaSuccess) return e;
-  return pdl_launch(prop_redo_kernel, dim3((n2 + kRedoCols - 1) / kRedoCols, nw), 256, 0, st, P, vHS,
-                    Wt, S, T, W, N, n2, order, o->pb.ok, o->prop_bad, o->err,
+  return pdl_launch(prop_redo_kernel, dim3((n2 + kRedoCols - 1) / kRedoCols, nw), 256, 0, st, P,
+                    vHS, Wt, S, T, W, N, n2, order, o->pb.ok, o->prop_bad, o->err,
                     o->redone + OZ_PROPAGATE);
 }
 
@@ -1297,9 +1301,9 @@ cudaError_t oz_exchange(OzState* o, const z_t* Gc, int nwalk, z_t* Kpart, int nb
         const long long ld = (2LL * w * n + 3) / 4 * 4;
         EpiRows epi{o->T, ld, row0 + c * n};
         if ((e = oz::launch<7>(g, epi, o->err, st)) != cudaSuccess) break;
-        pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st, 
-            reinterpret_cast<const z_t*>(o->T), n, ld / 2, row0, c0, Kpart, nblk, w0, s, o->norms);
-        e = cudaGetLastError();
+        e = pdl_launch(trace_kernel, dim3(c, w), kTraceThreads, smem, st,
+                       reinterpret_cast<const z_t*>(o->T), n, ld / 2, row0, c0, Kpart, nblk, w0, s,
+                       o->norms);
       }
     }
   }

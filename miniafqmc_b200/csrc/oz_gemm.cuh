@@ -21,11 +21,14 @@
 // 1 .. S + 1 - i are ONE matrix product of N = 64 (S + 1 - i) columns whose accumulators
 // are consecutive in TMEM, starting at accumulator i: ten tcgen05.mma per 32 bytes of K
 // instead of 28 (ND = 7), and each A slice is read from shared memory once or twice.
-// What bounds it: shared memory.  Per 32 bytes of K the ten MMAs read 97 KB of operands and
-// the ring is filled with 43 KB, 1093 clocks at 128 bytes a clock against 896 of the tensor
-// pipe; the rest is the drain of the last tile and the power limit.  768 x 12288 x 384 real,
-// row-major FP64 results: 78 us, 2.6e15 digit operations a second (the
-// FP64 pipe's 37e12 a second would take 196 us for the same 7.2 GFLOP).
+// What bounds it: per tile, the MMAs and then the drain, since one tile's accumulators fill
+// TMEM and no MMA runs while they are read.  Counters (chunks of the exchange at 384 orbitals, 32
+// vectors x 64 walkers of 48 electrons, 17.2K clocks a tile of six slabs): tensor pipe active 55%
+// of the elapsed clocks, its shared-memory reads 47% of the peak (per 32 bytes of K the ten MMAs
+// read 97 KB and the ring is filled with 43 KB, 1093 clocks at 128 bytes a clock against 896 of
+// the tensor pipe), issue slots 16%; the chain's products at 384 orbitals (12 slabs, 34 pairs) 57%
+// and 47%.  768 x 12288 x 384 real, row-major FP64 results: 78 us, 2.6e15 digit operations a second
+// (the FP64 pipe's 37e12 a second would take 196 us for the same 7.2 GFLOP).
 //
 // One persistent CTA per SM: warp 8 copies slabs (bulk copies) into a two-stage ring, one thread of
 // warp 9 issues the MMAs, and warps 0-7 turn the accumulators into FP64 results in

@@ -829,7 +829,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
             for (int part = 0; part < nparts; part++) {
               const uint64_t ad = sdesc_k<SLAB>(smem_u32(stA(s, part)));
               const uint64_t bd = sdesc_k<SLAB>(smem_u32(stB(s, part)));
-  #pragma unroll
+#pragma unroll
               for (int k = 0; k < C::BK / C::UK; k++)
                 umma<FMT>(d, ad + 2 * k, bd + 2 * k, ID, (f != 0 || part != 0 || k != 0) ? 1u : 0u);
             }
@@ -860,13 +860,13 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
             tc_fence_after();
             const uint64_t ad = sdesc_k<SLAB>(smem_u32(stA(s, 0)));
             const uint64_t bd = sdesc_k<SLAB>(smem_u32(stB(s, 0)));
-  #pragma unroll
+#pragma unroll
             for (int k = 0; k < C::BK / C::UK; k++)
               umma<FMT>(d, ad + 2 * k, bd + 2 * k, ID, (kb != kb0 || k != 0) ? 1u : 0u);
             if (SPLIT) {
               const uint64_t al = sdesc_k<SLAB>(smem_u32(stA(s, 1)));
               const uint64_t bl = sdesc_k<SLAB>(smem_u32(stB(s, 1)));
-  #pragma unroll
+#pragma unroll
               for (int k = 0; k < C::BK / C::UK; k++) {
                 umma<FMT>(d, ad + 2 * k, bl + 2 * k, ID, 1u);
                 umma<FMT>(d, al + 2 * k, bd + 2 * k, ID, 1u);
@@ -911,10 +911,10 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
             const uint32_t trow =
                 tmem + b * C::TMEM_COLS + ((uint32_t)(wq * 32) << 16) + (uint32_t)(wg * CPW);
             if (ch == 0) {
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < CPW / 32; j++) tmem_ld32(trow + j * 32, acc + j * 32);
             } else {
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < CPW / 32; j++) tmem_ld32_add(trow + j * 32, acc + j * 32);
             }
             tc_fence_before();
@@ -925,7 +925,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
             epi.regs(z, mt, nt, row, acc, scr, wg);
           } else {
             const int m0 = mt * job.m_step[p], n0 = nt * job.n_step[p];
-  #pragma unroll
+#pragma unroll
             for (int j = 0; j < CPW / 32; j++) epi(z, row, m0 + row, n0 + wg * CPW + j * 32, acc + j * 32);
           }
         }
@@ -958,7 +958,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
         if constexpr (Epi::kPair) {
           const int Pw = epi.pair_stride();
           float u[32];
-  #pragma unroll 1
+#pragma unroll 1
           for (int c0 = wg * 32; c0 < Pw && c0 + Pw < bn + 1; c0 += 32 * EPI_WG) {
             tmem_ld32(trow + c0, v);
             tmem_ld32(trow + c0 + Pw, u);
@@ -969,7 +969,7 @@ tc_gemm_persistent_kernel(const __grid_constant__ PJob<Epi, NP> job, int* err) {
           auto ld = [&](int col, float* out) { tmem_ld32(trow + col, out); };
           epi.staged(z, mt, nt, row, ld, scr, wg);
         } else {
-  #pragma unroll 1
+#pragma unroll 1
           for (int c0 = wg * 32; c0 < bn; c0 += 32 * EPI_WG) {
             tmem_ld32(trow + c0, v);
             epi(z, row, m0 + row, n0 + c0, v);
