@@ -269,7 +269,8 @@ afq_status afq_stage_times(afq_handle* h, double* ms, long long* launches, int r
  *   [6]     mixed form: split-K slice count;
  *   [7..11] FP64 form: CTA shape of the vHS CSR product, ZGEMM tile shape of the
  *           propagation chain, dense vbias, Coulomb and dense Vakbl products
- *           (0 built-in rule, k > 0 the k-th listed shape).
+ *           (0 built-in rule, k > 0 the k-th listed shape); the FP64 pipe's, whether or
+ *           not the product runs as a digit product.
  * ms[24]: for mixed sites the timed milliseconds of candidates 1 and 2, for FP64 sites
  * those of the chosen shape and of the rule (0 when not timed).  Sites of the other form
  * read 0.  AFQ_TUNE=0 in the environment skips the timing, AFQ_TUNE=1 or 2 forces one
@@ -283,7 +284,9 @@ afq_status afq_get_tuning(afq_handle* h, int* choice, double* ms);
  * slower operand is freed (Spvn keeps its CSR for the full-G path).  path[3], for Spvn
  * (vHS), SpvnT (vbias) and Vakbl (energy): 1 dense-tile GEMM, 0 CSR, -1 operand absent or
  * mixed form.  ms[6]: the best milliseconds of the CSR product and of the dense product
- * per operand (0 when not timed).  With AFQ_TUNE=0 the rule is dense at >= 25% density. */
+ * per operand (0 when not timed).  With AFQ_TUNE=0 the rule is dense at >= 25% density.
+ * A product that runs as a digit product (afq_get_digit_products) uses this choice for the
+ * results its digits do not hold. */
 afq_status afq_get_sparse_paths(afq_handle* h, int* path, double* ms);
 /* FP64 form: which products run as digit products on the int8 tensor cores (operands
  * written as signed 8-bit digits; AFQ_PREC_FP64 above), 0s for the mixed form.  on[6]:
@@ -414,7 +417,8 @@ afq_status afq_selftest_tc_gemm(int M, int N, int K, int batch, int tf32, int bn
  * producer, MMA issuer and epilogue gives up after this many clocks, sets a timeout flag
  * (reported, then cleared, by afq_synchronize) and ends the kernel's work; the kernel still
  * waits, with the default bound, for the copies and MMAs it has issued before it frees its
- * tensor memory.  clocks <= 0 restores the default (2e9 clocks, about one second).  Meant
+ * tensor memory.  A digit product of the FP64 form, or of afq_exchange_energy_noalloc, that
+ * timed out is computed by the FP64 pipe in the same call.  clocks <= 0 restores the default (2e9 clocks, about one second).  Meant
  * for tests of the timeout path and for watchdogs; it applies to every handle on the
  * device, so set it while no other work of this library runs there. */
 afq_status afq_set_tc_wait_limit(int device, long long clocks);

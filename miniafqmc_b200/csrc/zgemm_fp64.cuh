@@ -7,7 +7,8 @@
 //
 // Products large enough for the digit splitting of oz.cu run on the int8 tensor cores; this
 // kernel keeps the smaller ones, those whose digits do not fit the device memory, sites
-// without a digit form and the K beyond its int32 sums.  sm_100a has no FP64 tensor-core kind
+// without a digit form and the K beyond its int32 sums, and behind a gate (GATED instances)
+// computes the results that the digits do not hold.  sm_100a has no FP64 tensor-core kind
 // for tcgen05 and its FP64 FMA rate equals its FP64 MMA rate, so it is a register-tiled
 // CUDA-core GEMM: a BM x BN tile per
 // CTA, TM x TN complex accumulators per thread, BK-deep k slabs double-buffered in
