@@ -418,9 +418,10 @@ afq_status afq_selftest_tc_gemm(int M, int N, int K, int batch, int tf32, int bn
  * (reported, then cleared, by afq_synchronize) and ends the kernel's work; the kernel still
  * waits, with the default bound, for the copies and MMAs it has issued before it frees its
  * tensor memory.  A digit product of the FP64 form, or of afq_exchange_energy_noalloc, that
- * timed out is computed by the FP64 pipe in the same call.  clocks <= 0 restores the default (2e9 clocks, about one second).  Meant
- * for tests of the timeout path and for watchdogs; it applies to every handle on the
- * device, so set it while no other work of this library runs there. */
+ * timed out is computed by the FP64 pipe in the same call.  clocks <= 0 restores the
+ * default (2e9 clocks, about one second).  Meant for tests of the timeout path and for
+ * watchdogs; it applies to every handle on the device, so set it while no other work of
+ * this library runs there. */
 afq_status afq_set_tc_wait_limit(int device, long long clocks);
 
 #ifdef __cplusplus
